@@ -42,6 +42,16 @@
 #define COLREC_NNEW 148 // [6] count of further neighbours
 #define COLREC_WORDS 160
 
+// Edge records of a W column (7 per column, EDGE_W words each): neighbour,
+// V face (bit 31: the column is side 2, itab_v%iw(2), of the face), the
+// face's lowest device level (mza past npoly, so that no level uses it),
+// dirv; order-2 gradient weights x, y; the column's own face offsets dxps,
+// dyps.  Third-order records (EDGE3_W floats per edge): the five quadratic
+// gradient weights, the five face offsets (dxps, dyps, xx0, xy0, yy0 of the
+// column's side), pad.
+#define EDGE_W 8
+#define EDGE3_W 12
+
 namespace olamgpu {
 
 // ---- error handling ---------------------------------------------------------
@@ -169,6 +179,8 @@ struct DevGrid {
   DevBuf<float> xx0_v, xy0_v, yy0_v, xx0_vu, xy0_vu, yy0_vu;  // (mva, 2)
   DevBuf<float> a_w, a_wu;       // Fortran (mza, 2, 2)
   DevBuf<float> volti;           // (mwa, mza)
+  DevBuf<int> edge;              // (mwa, 7, EDGE_W)
+  DevBuf<float> edge3_b, edge3_u;  // (mwa, 7, EDGE3_W), order 3: bounded and unbounded
   // fused-kernel stencil weights: for V face iv and side s the value
   // reconstructed from cell c = iw(s) is
   //   S(c) + sum_n ew[iv][s][n] * (S(w_nb[c][n]) - S(c))
@@ -480,6 +492,7 @@ Context& ctx();
 // set-up helpers (setup.cu)
 int upload_grid(const olamgpu_grid* g, DevGrid& d, cudaStream_t s);
 int build_fused_weights(const olamgpu_grid* g, DevGrid& d, int order, cudaStream_t s);
+int build_edges(const olamgpu_grid* g, DevGrid& d, int order, cudaStream_t s);
 // host tile tables (layouts above); T == 0 when the grid is left to the column kernel
 struct TileHost {
   int T = 0, ntiles = 0, nu_max = 0, order = 0;

@@ -195,6 +195,53 @@ int upload_grid(const olamgpu_grid* g, DevGrid& d, cudaStream_t s) {
   return OLAMGPU_OK;
 }
 
+// edge records of every W column (layout in internal.h)
+int build_edges(const olamgpu_grid* g, DevGrid& d, int order, cudaStream_t s) {
+  const int mwa = g->mwa, mza = g->mza;
+  std::vector<int> e((size_t)mwa * 7 * EDGE_W, 0);
+  std::vector<float> b, u;
+  if (order == 3) {
+    b.assign((size_t)mwa * 7 * EDGE3_W, 0.f);
+    u.assign((size_t)mwa * 7 * EDGE3_W, 0.f);
+  }
+  auto bits = [](float f) { int i; std::memcpy(&i, &f, 4); return i; };
+  for (int iw = 0; iw < mwa; ++iw) {
+    const int np = iw > 0 ? g->npoly[iw] : 0;
+    for (int n = 0; n < 7; ++n) {
+      const size_t x = (size_t)iw * 7 + n;
+      int* r = &e[x * EDGE_W];
+      r[0] = iw;
+      r[2] = mza;
+      if (n >= np) continue;
+      const int iv = g->itab_w_iv[x] - 1;
+      r[0] = g->itab_w_iw[x] - 1;
+      if (iv < 1) continue;   // a face outside this grid (the rim of a halo)
+      const int side = g->itab_v_iw[(size_t)iv * 2] - 1 == iw ? 0 : 1;
+      const size_t f = (size_t)iv * 2 + side;
+      r[1] = side ? (iv | (int)0x80000000) : iv;
+      r[2] = g->lpv[iv] - 1;
+      r[3] = bits(g->itab_w_dirv[x]);
+      r[4] = bits(g->gxps_coef[x]);
+      r[5] = bits(g->gyps_coef[x]);
+      r[6] = bits(g->dxps[f]);
+      r[7] = bits(g->dyps[f]);
+      if (order != 3) continue;
+      float* pb = &b[x * EDGE3_W];
+      float* pu = &u[x * EDGE3_W];
+      for (int m = 0; m < 5; ++m) { pb[m] = g->xy_h[x * 5 + m]; pu[m] = g->xy_hu[x * 5 + m]; }
+      pb[5] = pu[5] = g->dxps[f];
+      pb[6] = pu[6] = g->dyps[f];
+      pb[7] = g->xx0_v[f]; pb[8] = g->xy0_v[f]; pb[9] = g->yy0_v[f];
+      pu[7] = g->xx0_vu[f]; pu[8] = g->xy0_vu[f]; pu[9] = g->yy0_vu[f];
+    }
+  }
+  OG_CHECK(upload(d.edge, e.data(), e.size(), s));
+  OG_CHECK(upload(d.edge3_b, b.data(), b.size(), s));
+  OG_CHECK(upload(d.edge3_u, u.data(), u.size(), s));
+  OG_CUDA(cudaStreamSynchronize(s));
+  return OLAMGPU_OK;
+}
+
 // Per V face and side, the reconstruction folded into one weight per
 // neighbour of the upwind cell: value = S(c) + sum_n w_n (S(nb_n) - S(c)).
 // Restates scalar_v_column (scalar_transport_rk.F90:497-525) composed with

@@ -125,13 +125,23 @@ int tracers_to_host(cudaStream_t s) {
   return OLAMGPU_OK;
 }
 
+static int grow(DevBuf<float>& b, size_t n) { return b.n >= n ? OLAMGPU_OK : b.alloc(n); }
+
+// Tracers (padded) up to which a stage runs as passes over cells: the tiled
+// kernel gives 8 lanes or more to a column whatever the count, and needs the
+// step's weight records (128 B a cell).  Measured per stage at NXP=100, 60
+// levels, order 2 (tiles + half of the records against cells): 4 tracers 1.26
+// / 0.52 ms, 8: 1.26 / 0.99, 12: 1.27 / 1.43.
+#ifndef CELL_NTP_MAX
+#define CELL_NTP_MAX 8
+#endif
+
 // scratch of the reference-mirroring passes for a group of nt tracers
 static int ensure_pass_scratch(Context& C, int nt, int order) {
   const DevGrid& d = C.g;
   Transport& tp = C.tp;
   const size_t wz = (size_t)d.mwa * d.mza * nt, vz = (size_t)d.mva * d.mza * nt;
   const int i2d = order == 3 ? 5 : 2;
-  auto grow = [](DevBuf<float>& b, size_t n) { return b.n >= n ? OLAMGPU_OK : b.alloc(n); };
   OG_CHECK(grow(tp.gx, wz * i2d));
   OG_CHECK(grow(tp.upv, vz));
   OG_CHECK(grow(tp.hiv, vz));
@@ -365,6 +375,8 @@ int transport_run(const float* rho_old_host, olamgpu_cfl_diag* diag) {
     set_error("the fused transport form needs mwa * mza * ntp / 2 < 2^32; use the plain form");
     return OLAMGPU_E_UNSUPPORTED;
   }
+  // few tracers in the tiled form run as passes over cells
+  bool cells = tiled && tr.ntp <= CELL_NTP_MAX && tp.autotune && !C.halo.on && cell_stage_available(d, order);
   if (batched && !tiled && d.ew_order != order)
     OG_CHECK(build_fused_weights(&C.hgrid, C.g, order, s));
 
@@ -395,7 +407,15 @@ int transport_run(const float* rho_old_host, olamgpu_cfl_diag* diag) {
     if (tp.have_turb)
       for (int n = 0; n < tr.n; ++n)
         if (tr.sgsmix[n]) launch_diffusion(d, tp, CTView{A, ntp, n}, TView{T, ntp, n}, 1, s);
-    if (tiled) {
+    if (cells && grow(tp.upv, (size_t)mva * mza * ntp) != OLAMGPU_OK) {
+      cudaGetLastError();   // no room for the face values: the tiles need none
+      cells = false;
+    }
+    CellStage cs{};
+    cs.ld = ntp;
+    cs.vmasc = tp.vmasc.p; cs.wmasc = tp.wmasc.p; cs.rhos = rhos_nrk; cs.ff = tp.ff.p;
+    cs.nrk = nrk;
+    if (tiled && !cells) {
       OG_PROF("tile_weights", s);
       OG_CHECK(launch_tile_weights(d, tp, rhos_nrk, s));
       // the stage kernel's shape for this grid and tracer count, chosen on
@@ -409,19 +429,31 @@ int transport_run(const float* rho_old_host, olamgpu_cfl_diag* diag) {
       float* IN = tr.q[in_b].p;
       float* OUT = tr.q[out_b].p;
       const bool last = istage == nrk;
-      if (last && any_pdm)
-        launch_scp0_pd_update(d, tp, TView{A, ntp, 0}, CTView{T, ntp, 0}, tp.d_mode.p + tr.n, tr.n, dtr, s);
+      cs.istage = istage; cs.dtr = dtr;
+      if (last && any_pdm) launch_cell_preupdate(d, tp, A, T, ntp, tr.n, tp.d_mode.p + tr.n, dtr, s);
       if (last && anylim) {
-        // limited last stage: the reference's passes over tracer groups sized
-        // to a scratch budget
-        const size_t per = (size_t)4 * mza * ((size_t)7 * mwa + (size_t)3 * mva) + 1;
-        int grp = (int)std::max<size_t>(1, std::min<size_t>((size_t)tr.n, (size_t)(8ull << 30) / per));
-        OG_CHECK(ensure_pass_scratch(C, grp, order));
+        // limited last stage: passes over cells for tracer groups (multiples
+        // of 4) sized to a scratch budget
+        const bool monot = C.opts.iscal_monot == 1;
+        const size_t vz = (size_t)mva * mza, per = 4 * ((monot ? 2 : 1) * wz + vz);
+        const int grp = (int)std::max<size_t>(4, std::min<size_t>((size_t)ntp, (size_t)(8ull << 30) / per / 4 * 4));
+        OG_CHECK(grow(tp.upv, vz * grp));
+        OG_CHECK(grow(tp.scale, wz * grp * (monot ? 2 : 1)));
+        cs.limited = C.opts.iscal_monot;
+        cs.face = tp.upv.p; cs.scale = tp.scale.p;
         for (int g0 = 0; g0 < tr.n; g0 += grp) {
-          int nt = std::min(grp, tr.n - g0);
-          passes_stage(C, CTView{IN, ntp, g0}, CTView{A, ntp, g0}, CTView{T, ntp, g0},
-                       TView{OUT, ntp, g0}, nt, istage, nrk, dtr, rhos_nrk, tp.d_mode.p + g0, true, s);
+          cs.S = IN + g0; cs.S0 = A + g0; cs.SCT = T + g0; cs.out = OUT + g0;
+          cs.nt = std::min(grp, tr.n - g0);
+          cs.mode = tp.d_mode.p + g0;
+          OG_CHECK(launch_cell_stage(d, order, cs, s));
         }
+      } else if (cells) {
+        // the profile's name of a stage of the fused form, whichever kernels run it
+        OG_PROF(istage == 1 ? "tile_stage1" : "tile_stage", s);
+        cs.limited = 0;
+        cs.face = tp.upv.p;
+        cs.S = IN; cs.S0 = A; cs.SCT = T; cs.out = OUT; cs.nt = ntp;
+        OG_CHECK(launch_cell_stage(d, order, cs, s));
       } else {
         OG_PROF(tiled ? (istage == 1 ? "tile_stage1" : "tile_stage") : (istage == 1 ? "fused_stage1" : "fused_stage"), s);
         if (tiled) OG_CHECK(launch_tile_stage(d, tp, IN, A, T, OUT, ntp, istage, nrk, dtr, C.status.p, s));

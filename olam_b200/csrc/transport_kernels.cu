@@ -1232,30 +1232,15 @@ static int update_scalar_noalloc(const float* scp, const float* scp0, const floa
   }
   float* scr = nullptr;
   OG_CHECK(noalloc_scratch(dev, &scr));
-  float* gx = scr;
-  float* upv = scr + n_gx;
-  float* ff = upv + n_upv;
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : C.stream;
-  // every column explicit: the implicit fraction must read zero
-  OG_CUDA(cudaMemsetAsync(ff, 0, n_ff * sizeof(float), s));
-  const CTView in{scp, 1, 0}, in0{scp0, 1, 0}, tend{sct, 1, 0};
-  const GridK g = gridk(d);
-  const size_t ng = (size_t)d.nw_prog * d.mza;
-  k_grad<<<cdiv(ng, 256), 256, 0, s>>>(g, d.jtw_prog.p, d.nw_prog, in, gx, 1, order, d.gxc.p, d.gyc.p, d.xy_h.p);
-  const VCoef vc{d.dxps.p, d.dyps.p, d.xx0_v.p, d.xy0_v.p, d.yy0_v.p};
-  const size_t nv = (size_t)d.nv_wadj * d.mza;
-  k_vflux<<<cdiv(nv, 256), 256, 0, s>>>(g, d.jtv_wadj.p, d.nv_wadj, in, in0, gx, vmasc, 1, order, vc, nullptr,
-                                        upv, nullptr, nullptr);
-  WcolArgs A;
-  A.g = g;
-  A.prog = d.jtw_prog.p; A.nprog = d.nw_prog;
-  A.scp = in; A.scp0 = in0; A.sct = tend; A.rhos = rhos;
-  A.vmasc = vmasc; A.wmasc = wmasc; A.ff = ff;
-  A.upv = upv; A.sfv = nullptr; A.scale = nullptr; A.upw = nullptr;
-  A.out = TView{out, 1, 0}; A.nt = 1; A.istage = 1; A.nrk = 1; A.dtr = dtr;
-  A.mode = nullptr;
-  k_wcol<<<cdiv((size_t)d.nw_prog, 128), 128, 0, s>>>(A);
-  OG_LAUNCHED(); OG_LAUNCHED(); OG_LAUNCHED();
+  CellStage c{};
+  c.S = scp; c.S0 = scp0; c.SCT = sct; c.out = out;
+  c.ld = 1; c.nt = 1;
+  c.vmasc = vmasc; c.wmasc = wmasc; c.rhos = rhos;
+  c.ff = nullptr;                       // every column explicit
+  c.face = scr;
+  c.istage = 1; c.nrk = 1; c.dtr = dtr;
+  OG_CHECK(launch_cell_stage(d, order, c, s));
   OG_CUDA(cudaGetLastError());
   return OLAMGPU_OK;
 }

@@ -115,6 +115,26 @@ bool tile_shape_fits(const DevGrid& d, int G);
 // scratch); rebuilds the tile tables when the width changes
 int tile_autotune(Context& C, const float* S, const float* S0, const float* SCT, float* OUT, float dtr);
 
+// a stage as passes over cells (transport_cell.cu): nt tracers of rows of ld
+// floats (ld 1: one tracer in OLAM's layout, unlimited only; else ld and the
+// first tracer's offset are multiples of 4), limited as iscal_monot
+struct CellStage {
+  const float *S, *S0, *SCT;
+  float* out;
+  int ld, nt, limited;
+  const int* mode;                         // limited: each tracer's last-stage mode
+  const float *vmasc, *wmasc, *rhos, *ff;  // ff (mwa, nrk); NULL: every column explicit
+  float* face;                             // scratch: (mva, mza, cell_width(nt)), ld 1: (mva, mza)
+  float* scale;                            // limited: (mwa, mza, cell_width(nt)), twice with the monotonic limiter
+  int istage, nrk;
+  float dtr;
+};
+inline int cell_width(int nt) { return (nt + 3) / 4 * 4; }
+bool cell_stage_available(const DevGrid& d, int order);
+int launch_cell_stage(const DevGrid& d, int order, const CellStage& c, cudaStream_t s);
+void launch_cell_preupdate(const DevGrid& d, const Transport& tp, float* S0, const float* SCT, int ld, int nt,
+                           const int* mode, float dtr, cudaStream_t s);
+
 // copy the columns outside jtw_prog (colsize floats each) from src to dst
 void launch_copy_cols(const int* cols, int ncol, const float* src, float* dst, size_t colsize,
                       cudaStream_t s);
