@@ -222,17 +222,15 @@ int transport_prepare(Context& C, const float* rho_old_host, bool upload_tracers
   OG_CHECK(tp.rhos.alloc((size_t)nrk * wz));
   OG_CHECK(tp.ff.alloc((size_t)nrk * mwa));
   OG_CHECK(tp.imp_list.alloc((size_t)nrk * mwa));
-  OG_CHECK(tp.imp_count.alloc(3));
   OG_CHECK(tp.imp_b.alloc((size_t)nrk * mwa * 3 * mza));
-  OG_CHECK(tp.cfl_loc.alloc(6));
+  OG_CHECK(tp.cfl_loc.alloc(8));   // six maxima, then the counts of implicit columns
+  tp.imp_count.borrow(reinterpret_cast<int*>(tp.cfl_loc.p + 6), 4);
 
   const float dtl = (float)C.opts.dtlm;
   const float one3 = 1.f / 3.f;
   for (int n = 0; n < nrk; ++n) dtlr[n] = dtl * (nrk == 3 ? (n == 0 ? one3 : (n == 1 ? 0.5f : 1.0f))
                                                           : (n == 0 ? 0.5f : 1.0f));
-  { OG_PROF("check_cfls", s); launch_check_cfls(d, tp, nrk, dtl, tp.cfl_loc.p, s); }
-  { OG_PROF("rhos", s); launch_rhos(d, tp, nrk, s); }
-  { OG_PROF("implicit_prep", s); launch_implicit_prep(d, tp, nrk, dtlr, s); }
+  if (d.nw_prog > 0) { OG_PROF("prepare", s); launch_prepare(d, tp, nrk, dtl, dtlr, s); }
   return OLAMGPU_OK;
 }
 

@@ -51,180 +51,168 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
   return v;
 }
 
-// one warp per prognostic column, lanes over levels (coalesced in k)
-__global__ void k_check_cfls(GridK g, const int* __restrict__ prog, int nprog,
-                             const float* __restrict__ vmasc, const float* __restrict__ wmasc,
-                             const float* __restrict__ rho, const float* __restrict__ wc, int nrk,
-                             float dt, float* __restrict__ ff, unsigned long long* red) {
-  const int j = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (j >= nprog) return;
-  const int mza = g.mza;
-  const int iw = prog[j];
-  const int np = g.npoly[iw];
-  int ev[7];
-  float dv[7];
-#pragma unroll
-  for (int n = 0; n < 7; ++n) {
-    ev[n] = g.w_ev[iw * 8 + n];
-    dv[n] = g.w_dirv[iw * 8 + n];
-  }
-  float fimp[3] = {0.f, 0.f, 0.f};
-  unsigned long long kc = 0, kh = 0, kw = 0, nc = 0, nh = 0, nwn = 0;
-  for (int kd = g.lpw[iw] + lane; kd < mza; kd += 32) {
-    float cflh = 0.f;
-#pragma unroll
-    for (int n = 0; n < 7; ++n)
-      if (n < np && kd >= g.lpv[ev[n]])
-        cflh = cflh - fminf(dv[n] * __ldg(vmasc + (size_t)ev[n] * mza + kd), 0.0f);
-    const float dovr = dt * g.volti[(size_t)iw * mza + kd] / rho[(size_t)iw * mza + kd];
-    cflh = cflh * dovr;
-    float cflw = (fmaxf(wmasc[(size_t)iw * mza + kd], 0.f) - fminf(wmasc[(size_t)iw * mza + kd - 1], 0.f)) * dovr;
-    const float cfl = cflh + cflw;
-    cflw = fmaxf(cflw, .1f);
-    fimp[nrk - 1] = fmaxf(fimp[nrk - 1], (cfl - 0.98f) / cflw);
-    fimp[nrk - 2] = fmaxf(fimp[nrk - 2], (cfl - 1.98f) / cflw);
-    if (nrk == 3) fimp[0] = fmaxf(fimp[0], (cfl - 2.98f) / cflw);
-    const unsigned int order = (unsigned int)j * (unsigned int)mza + (unsigned int)kd;
-    const unsigned long long low = 0xffffffffull - order;
-    if (cfl != cfl) nc = max(nc, order + 1ull);
-    else if (cfl > 0.f) kc = max(kc, ((unsigned long long)__float_as_uint(cfl) << 32) | low);
-    if (cflh != cflh) nh = max(nh, order + 1ull);
-    else if (cflh > 0.f) kh = max(kh, ((unsigned long long)__float_as_uint(cflh) << 32) | low);
-    if (wc) {
-      const float w = wc[(size_t)iw * mza + kd];
-      if (w != w) nwn = max(nwn, order + 1ull);
-      else if (fabsf(w) > 0.f) kw = max(kw, ((unsigned long long)__float_as_uint(fabsf(w)) << 32) | low);
-    }
-  }
-#pragma unroll
-  for (int n = 0; n < 3; ++n)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) fimp[n] = fmaxf(fimp[n], __shfl_xor_sync(0xffffffffu, fimp[n], o));
-  kc = warp_max_u64(kc); nc = warp_max_u64(nc);
-  kh = warp_max_u64(kh); nh = warp_max_u64(nh);
-  kw = warp_max_u64(kw); nwn = warp_max_u64(nwn);
-  if (lane == 0) {
-    for (int n = 0; n < nrk; ++n) {
-      float f = fminf(1.0f, fimp[n]);
-      if (f < .02f) f = 0.f;
-      ff[(size_t)iw * nrk + n] = f;
-    }
-    if (red) {
-      if (kc) atomicMax(&red[0], kc);
-      if (nc) atomicMax(&red[1], nc);
-      if (kh) atomicMax(&red[2], kh);
-      if (nh) atomicMax(&red[3], nh);
-      if (kw) atomicMax(&red[4], kw);
-      if (nwn) atomicMax(&red[5], nwn);
-    }
-  }
-}
-
-void launch_check_cfls(const DevGrid& d, const Transport& tp, int nrk, float dtl,
-                       unsigned long long* red, cudaStream_t s) {
-  if (red) cudaMemsetAsync(red, 0, 6 * sizeof(unsigned long long), s);
-  const int nb = 256;  // 8 columns per block
-  k_check_cfls<<<cdiv((size_t)d.nw_prog * 32, nb), nb, 0, s>>>(gridk(d), d.jtw_prog.p, d.nw_prog,
-                                                              tp.vmasc.p, tp.wmasc.p, tp.rho_old.p,
-                                                              tp.wc.p, nrk, dtl, tp.ff.p, red);
-  OG_LAUNCHED();
-}
-
-// ---------------------------------------------------------------------------
-// rhos (scalar_transport_rk.F90:117-152), nudging off
-// ---------------------------------------------------------------------------
-__global__ void k_rhos(GridK g, const int* __restrict__ prog, int nprog, const double* __restrict__ rho,
-                       const float* __restrict__ rho_old, float* __restrict__ rhos, int nrk) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int mza = g.mza;
-  if (i >= (size_t)nprog * mza) return;
-  int j = (int)(i / mza), kd = (int)(i % mza);
-  int iw = prog[j];
-  if (kd < g.lpw[iw]) return;
-  size_t ix = (size_t)iw * mza + kd;
-  size_t plane = (size_t)g.mwa * mza;
-  float rhof = (float)rho[ix];
-  float ro = rho_old[ix];
-  if (nrk == 3) {
-    rhos[ix] = (2.f / 3.f) * ro + (1.f / 3.f) * rhof;
-    rhos[plane + ix] = 0.5f * (ro + rhof);
-    rhos[2 * plane + ix] = rhof;
-  } else {
-    rhos[ix] = 0.5f * (ro + rhof);
-    rhos[plane + ix] = rhof;
-  }
-}
-
-void launch_rhos(const DevGrid& d, Transport& tp, int nrk, cudaStream_t s) {
-  size_t n = (size_t)d.nw_prog * d.mza;
-  k_rhos<<<cdiv(n, 256), 256, 0, s>>>(gridk(d), d.jtw_prog.p, d.nw_prog, tp.rho.p, tp.rho_old.p,
-                                      tp.rhos.p, nrk);
-  OG_LAUNCHED();
-}
-
-// ---------------------------------------------------------------------------
-// implicit-column factorisation (scalar_transport_rk.F90:164-217) with
-// tridif_prep (tridiag_lib.f90:321-338).  Column slots are handed out by an
-// atomic counter; each column's result does not depend on its slot.
-// imp_b[(n*mwa + slot)*3*mza + {0,1,2}*mza + kd] = b1, scr1, cji.
-// ---------------------------------------------------------------------------
 struct Dtlr { float v[3]; };
 
-__global__ void k_implicit_prep(GridK g, const int* __restrict__ prog, int nprog,
-                                const float* __restrict__ ff, const float* __restrict__ wmasc,
-                                const float* __restrict__ rhos, int nrk, Dtlr dtlr,
-                                int* __restrict__ list, int* __restrict__ count, float* __restrict__ b) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nprog) return;
-  const int mza = g.mza;
-  int iw = prog[j];
-  int kb = g.lpw[iw];
-  size_t plane = (size_t)g.mwa * mza;
-  for (int n = 0; n < nrk; ++n) {
-    float f = ff[(size_t)iw * nrk + n];
-    if (!(f > 0.001f)) continue;
-    int slot = atomicAdd(&count[n], 1);
-    list[(size_t)n * g.mwa + slot] = iw;
-    float* b1 = b + ((size_t)n * g.mwa + slot) * 3 * mza;
-    float* scr1 = b1 + mza;
-    float* cji = b1 + 2 * mza;
-    float c1 = f * dtlr.v[n];
-    const float* wm = wmasc + (size_t)iw * mza;
-    // wup(kd) = max(wmasc,0), wdn(kd) = min(wmasc,0) for kd in [kb, mza-2];
-    // zero at kb-1 and mza-1
-    float cji_prev = 0.f, cip1_prev = 0.f;
-    for (int kd = kb; kd < mza; ++kd) {
-      float wup_m1 = (kd - 1 >= kb) ? fmaxf(wm[kd - 1], 0.f) : 0.f;
-      float wdn_m1 = (kd - 1 >= kb) ? fminf(wm[kd - 1], 0.f) : 0.f;
-      float wup = (kd <= mza - 2) ? fmaxf(wm[kd], 0.f) : 0.f;
-      float wdn = (kd <= mza - 2) ? fminf(wm[kd], 0.f) : 0.f;
-      float c2 = c1 * g.volti[(size_t)iw * mza + kd] / rhos[(size_t)n * plane + (size_t)iw * mza + kd];
-      float cim1 = -c2 * wup_m1;
-      float ci = 1.0f + c2 * (wup - wdn_m1);
-      float cip1 = c2 * wdn;
-      b1[kd] = cim1;
-      if (kd == kb) {
-        cji_prev = 1.0f / ci;
-        cji[kd] = cji_prev;
-        scr1[kd] = 0.f;
-      } else {
-        float sc = cji_prev * cip1_prev;
-        scr1[kd] = sc;
-        cji_prev = 1.0f / (ci - cim1 * sc);
-        cji[kd] = cji_prev;
+struct PrepArgs {
+  GridK g;
+  const int4* edge;                // edge records (EDGE_W words)
+  const int* prog; int nprog;
+  const float* vmasc; const float* wmasc; const float* rho_old; const float* wc;
+  const double* rho;
+  int nrk; float dt; Dtlr dtlr;
+  float* ff;                       // (mwa, nrk)
+  float* rhos;                     // (nrk, mwa, mza)
+  unsigned long long* red;
+  int* list; int* count; float* b; // implicit columns
+};
+
+// The per-step coefficients of a column, one warp per prognosed column, lanes
+// over levels:
+//   check_cfls (scalar_transport_rk.F90:1476-1712): CFL maxima and ff_implic
+//   rhos       (117-152), nudging off
+//   the factorisation of an implicit column (164-217) with tridif_prep
+//   (tridiag_lib.f90:321-338), by the warp's first lane.  Slots are handed
+//   out by an atomic counter; a column's result does not depend on its slot.
+//   imp_b[(n*mwa + slot)*3*mza + {0,1,2}*mza + kd] = b1, scr1, cji.
+// Bound: HBM (48 B per cell).  As three kernels with an atomic per column and
+// maximum it took 263 + 46 + 10 us at NXP=100, 60 levels: the atomics on three
+// addresses were serial (2.5 ns a column).  A block now reduces its columns
+// first and only tries an atomic that can raise the maximum.
+__global__ void __launch_bounds__(256) k_prepare(PrepArgs A) {
+  __shared__ unsigned long long part[6][8];
+  const GridK& g = A.g;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j = blockIdx.x * 8 + warp;
+  const int mza = g.mza, nrk = A.nrk;
+  unsigned long long kc = 0, kh = 0, kw = 0, nc = 0, nh = 0, nwn = 0;
+  if (j < A.nprog) {
+    const int iw = A.prog[j], np = g.npoly[iw], kb = g.lpw[iw];
+    const size_t cb = (size_t)iw * mza, plane = (size_t)g.mwa * mza;
+    int4 e[7];
+#pragma unroll
+    for (int n = 0; n < 7; ++n) e[n] = __ldg(A.edge + ((size_t)iw * 7 + n) * (EDGE_W / 4));
+    float fimp[3] = {0.f, 0.f, 0.f};
+    for (int kd = kb + lane; kd < mza; kd += 32) {
+      float vm[7];
+#pragma unroll
+      for (int n = 0; n < 7; ++n) {
+        vm[n] = 0.f;
+        if (n < np && kd >= e[n].z) vm[n] = __ldg(A.vmasc + (size_t)(e[n].y & 0x7fffffff) * mza + kd);
       }
-      cip1_prev = cip1;
+      const float ro = __ldg(A.rho_old + cb + kd), vt = __ldg(g.volti + cb + kd);
+      const float wp = __ldg(A.wmasc + cb + kd), wm = __ldg(A.wmasc + cb + kd - 1);
+      const float rhof = (float)__ldg(A.rho + cb + kd);
+      float cflh = 0.f;
+#pragma unroll
+      for (int n = 0; n < 7; ++n)
+        if (n < np && kd >= e[n].z) cflh = cflh - fminf(__int_as_float(e[n].w) * vm[n], 0.0f);
+      const float dovr = A.dt * vt / ro;
+      cflh = cflh * dovr;
+      float cflw = (fmaxf(wp, 0.f) - fminf(wm, 0.f)) * dovr;
+      const float cfl = cflh + cflw;
+      cflw = fmaxf(cflw, .1f);
+      fimp[nrk - 1] = fmaxf(fimp[nrk - 1], (cfl - 0.98f) / cflw);
+      fimp[nrk - 2] = fmaxf(fimp[nrk - 2], (cfl - 1.98f) / cflw);
+      if (nrk == 3) fimp[0] = fmaxf(fimp[0], (cfl - 2.98f) / cflw);
+      const unsigned int order = (unsigned int)j * (unsigned int)mza + (unsigned int)kd;
+      const unsigned long long low = 0xffffffffull - order;
+      if (cfl != cfl) nc = max(nc, order + 1ull);
+      else if (cfl > 0.f) kc = max(kc, ((unsigned long long)__float_as_uint(cfl) << 32) | low);
+      if (cflh != cflh) nh = max(nh, order + 1ull);
+      else if (cflh > 0.f) kh = max(kh, ((unsigned long long)__float_as_uint(cflh) << 32) | low);
+      if (A.wc) {
+        const float w = __ldg(A.wc + cb + kd);
+        if (w != w) nwn = max(nwn, order + 1ull);
+        else if (fabsf(w) > 0.f) kw = max(kw, ((unsigned long long)__float_as_uint(fabsf(w)) << 32) | low);
+      }
+      float* r = A.rhos + cb + kd;
+      if (nrk == 3) {
+        r[0] = (2.f / 3.f) * ro + (1.f / 3.f) * rhof;
+        r[plane] = 0.5f * (ro + rhof);
+        r[2 * plane] = rhof;
+      } else {
+        r[0] = 0.5f * (ro + rhof);
+        r[plane] = rhof;
+      }
     }
+#pragma unroll
+    for (int n = 0; n < 3; ++n)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) fimp[n] = fmaxf(fimp[n], __shfl_xor_sync(0xffffffffu, fimp[n], o));
+    __syncwarp();   // the warp's rhos, before its first lane reads them
+    if (lane == 0) {
+      for (int n = 0; n < nrk; ++n) {
+        float f = fminf(1.0f, fimp[n]);
+        if (f < .02f) f = 0.f;
+        A.ff[(size_t)iw * nrk + n] = f;
+        if (!(f > 0.001f)) continue;
+        const int slot = atomicAdd(&A.count[n], 1);
+        A.list[(size_t)n * g.mwa + slot] = iw;
+        float* b1 = A.b + ((size_t)n * g.mwa + slot) * 3 * mza;
+        float* scr1 = b1 + mza;
+        float* cji = b1 + 2 * mza;
+        const float c1 = f * A.dtlr.v[n];
+        const float* w = A.wmasc + cb;
+        const float* rs = A.rhos + (size_t)n * plane + cb;
+        // wup(kd) = max(wmasc,0), wdn(kd) = min(wmasc,0) for kd in [kb, mza-2];
+        // zero at kb-1 and mza-1
+        float cji_prev = 0.f, cip1_prev = 0.f;
+        for (int kd = kb; kd < mza; ++kd) {
+          const float wup_m1 = (kd - 1 >= kb) ? fmaxf(w[kd - 1], 0.f) : 0.f;
+          const float wdn_m1 = (kd - 1 >= kb) ? fminf(w[kd - 1], 0.f) : 0.f;
+          const float wup = (kd <= mza - 2) ? fmaxf(w[kd], 0.f) : 0.f;
+          const float wdn = (kd <= mza - 2) ? fminf(w[kd], 0.f) : 0.f;
+          const float c2 = c1 * g.volti[cb + kd] / rs[kd];
+          const float cim1 = -c2 * wup_m1;
+          const float ci = 1.0f + c2 * (wup - wdn_m1);
+          const float cip1 = c2 * wdn;
+          b1[kd] = cim1;
+          if (kd == kb) {
+            cji_prev = 1.0f / ci;
+            cji[kd] = cji_prev;
+            scr1[kd] = 0.f;
+          } else {
+            const float sc = cji_prev * cip1_prev;
+            scr1[kd] = sc;
+            cji_prev = 1.0f / (ci - cim1 * sc);
+            cji[kd] = cji_prev;
+          }
+          cip1_prev = cip1;
+        }
+      }
+    }
+    kc = warp_max_u64(kc); nc = warp_max_u64(nc);
+    kh = warp_max_u64(kh); nh = warp_max_u64(nh);
+    kw = warp_max_u64(kw); nwn = warp_max_u64(nwn);
+  }
+  if (lane == 0) {
+    part[0][warp] = kc; part[1][warp] = nc; part[2][warp] = kh;
+    part[3][warp] = nh; part[4][warp] = kw; part[5][warp] = nwn;
+  }
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    unsigned long long v = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v = max(v, part[threadIdx.x][w]);
+    unsigned long long* p = A.red + threadIdx.x;
+    // a stale read only costs an atomic that changes nothing
+    if (v > *reinterpret_cast<volatile unsigned long long*>(p)) atomicMax(p, v);
   }
 }
 
-void launch_implicit_prep(const DevGrid& d, Transport& tp, int nrk, const float* dtlr, cudaStream_t s) {
-  cudaMemsetAsync(tp.imp_count.p, 0, sizeof(int) * 3, s);
-  Dtlr v{{dtlr[0], dtlr[1], nrk > 2 ? dtlr[2] : 0.f}};
-  k_implicit_prep<<<cdiv(d.nw_prog, 128), 128, 0, s>>>(gridk(d), d.jtw_prog.p, d.nw_prog, tp.ff.p,
-                                                       tp.wmasc.p, tp.rhos.p, nrk, v, tp.imp_list.p,
-                                                       tp.imp_count.p, tp.imp_b.p);
+void launch_prepare(const DevGrid& d, Transport& tp, int nrk, float dtl, const float* dtlr, cudaStream_t s) {
+  // the maxima and the counts of implicit columns, one allocation
+  cudaMemsetAsync(tp.cfl_loc.p, 0, tp.cfl_loc.bytes(), s);
+  PrepArgs A;
+  A.g = gridk(d);
+  A.edge = reinterpret_cast<const int4*>(d.edge.p);
+  A.prog = d.jtw_prog.p; A.nprog = d.nw_prog;
+  A.vmasc = tp.vmasc.p; A.wmasc = tp.wmasc.p; A.rho_old = tp.rho_old.p; A.wc = tp.wc.p; A.rho = tp.rho.p;
+  A.nrk = nrk; A.dt = dtl;
+  A.dtlr = Dtlr{{dtlr[0], dtlr[1], nrk > 2 ? dtlr[2] : 0.f}};
+  A.ff = tp.ff.p; A.rhos = tp.rhos.p; A.red = tp.cfl_loc.p;
+  A.list = tp.imp_list.p; A.count = tp.imp_count.p; A.b = tp.imp_b.p;
+  k_prepare<<<cdiv(d.nw_prog, 8), 256, 0, s>>>(A);
   OG_LAUNCHED();
 }
 
@@ -234,13 +222,12 @@ __global__ void k_implicit_solve(GridK g, const int* __restrict__ list, const in
                                  const float* __restrict__ b, const float* __restrict__ ff,
                                  const float* __restrict__ wmasc, const float* __restrict__ rhos_st,
                                  int nrk, int istage, float dtr, CTView scp0, TView scp, int nt) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int n = *count;
-  if (i >= (size_t)n * nt) return;
-  int slot = (int)(i / nt), t = (int)(i % nt);
+  const size_t all = (size_t)*count * nt;
   const int mza = g.mza;
-  int iw = list[slot];
-  int kb = g.lpw[iw];
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < all; i += (size_t)gridDim.x * blockDim.x) {
+  const int slot = (int)(i / nt), t = (int)(i % nt);
+  const int iw = list[slot];
+  const int kb = g.lpw[iw];
   const float* b1 = b + (size_t)slot * 3 * mza;
   const float* scr1 = b1 + mza;
   const float* cji = b1 + 2 * mza;
@@ -267,12 +254,15 @@ __global__ void k_implicit_solve(GridK g, const int* __restrict__ list, const in
   }
   for (int kd = kb; kd < mza; ++kd) sp[(size_t)kd * scp.ld] = S0(kd) + sp[(size_t)kd * scp.ld];
   for (int kd = 1; kd < kb; ++kd) sp[(size_t)kd * scp.ld] = sp[(size_t)kb * scp.ld];
+  }
 }
 
 void launch_implicit_solve(const DevGrid& d, const Transport& tp, int nrk, int istage, float dtr,
                            CTView scp0, TView scp, int nt, cudaStream_t s) {
-  // an upper bound on the launch size; threads past the device count exit
-  size_t n = (size_t)d.nw_prog * nt;
+  // The count is on the device and mostly zero: blocks for every column and
+  // tracer took 57 us at NXP=100 with 128 tracers to find nothing to do.  At
+  // most four waves of blocks walk the implicit columns.
+  const size_t n = std::min<size_t>((size_t)d.nw_prog * nt, (size_t)128 * 16 * 148 * 4);
   size_t plane = (size_t)d.mwa * d.mza;
   const float* b = tp.imp_b.p + (size_t)(istage - 1) * d.mwa * 3 * d.mza;
   k_implicit_solve<<<cdiv(n, 128), 128, 0, s>>>(gridk(d), tp.imp_list.p + (size_t)(istage - 1) * d.mwa,

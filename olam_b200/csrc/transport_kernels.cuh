@@ -67,11 +67,8 @@ __device__ __forceinline__ void zrec(const float* a, int mza, int kd, int kb, fl
 enum { MODE_PLAIN = 0, MODE_MONOT = 1, MODE_PD = 2 };
 
 // ---- launchers (transport_kernels.cu) ------------------------------------
-void launch_check_cfls(const DevGrid& d, const Transport& tp, int nrk, float dtl,
-                       unsigned long long* red, cudaStream_t s);
-void launch_rhos(const DevGrid& d, Transport& tp, int nrk, cudaStream_t s);
-void launch_implicit_prep(const DevGrid& d, Transport& tp, int nrk, const float* dtlr,
-                          cudaStream_t s);
+// check_cfls, rhos and the implicit columns' factors, one launch
+void launch_prepare(const DevGrid& d, Transport& tp, int nrk, float dtl, const float* dtlr, cudaStream_t s);
 void launch_implicit_solve(const DevGrid& d, const Transport& tp, int nrk, int istage, float dtr,
                            CTView scp0, TView scp, int nt, cudaStream_t s);
 void launch_diffusion(const DevGrid& d, const Transport& tp, CTView scp, TView sct, int nt,
