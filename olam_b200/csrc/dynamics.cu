@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "transport_kernels.cuh"
 
@@ -47,6 +48,7 @@ struct DynK {
   const int* __restrict__ lpm;
   const float* __restrict__ volti;
   const float* __restrict__ a_w;
+  const int4* __restrict__ edge;    // EDGE_W words per edge, 7 edges per W column
   // flat: lpw = lpv = 2 everywhere (device level 1), no table read needed;
   // off_*: the loop table is the contiguous run off, off + 1, ... (a
   // global domain), no table read needed; -1 otherwise
@@ -66,6 +68,7 @@ static DynK dynk(const DevGrid& d) {
   k.npoly = d.npoly.p; k.w_nb = d.w_nb.p; k.w_ev = d.w_ev.p; k.w_dirv = d.w_dirv.p;
   k.v_iw = d.v_iw.p; k.v_im = d.v_im.p; k.m_iv = d.m_iv.p; k.m_im = d.m_im.p;
   k.lpw = d.lpw.p; k.lpv = d.lpv.p; k.lpm = d.lpm.p; k.volti = d.volti.p; k.a_w = d.a_w.p;
+  k.edge = reinterpret_cast<const int4*>(d.edge.p);
   k.flat = ctx().tp.flat ? 1 : 0;
   k.off_w = d.off_wprog; k.off_vp = d.off_vprog; k.off_va = d.off_vwadj;
   return k;
@@ -105,24 +108,6 @@ __global__ void k_setup_w(DynK g, const int* __restrict__ prog, int nprog, Setup
   a.sh_vz[x] = a.vmzet[x] * v4;
 }
 
-__global__ void k_setup_v(DynK g, const int* __restrict__ vprog, int nv, const float* __restrict__ vmc,
-                          const float* __restrict__ vmt, float* __restrict__ vmc0, float* __restrict__ sh_vmt,
-                          const float* __restrict__ rayf_cof, const float* __restrict__ vc03d,
-                          const float* __restrict__ vc, const double* __restrict__ rho, int krayf_bot) {
-  PK(j, kd, nv);
-  const int iv = VPTAB(j);
-  const size_t x = (size_t)iv * g.mza + kd;
-  vmc0[x] = vmc[x];
-  float v = vmt[x];
-  if (rayf_cof && kd >= krayf_bot - 1) {
-    const int iw1 = g.v_iw[iv * 2], iw2 = g.v_iw[iv * 2 + 1];
-    const double t = (double)(rayf_cof[kd] * 0.5f) * (rho[(size_t)iw1 * g.mza + kd] + rho[(size_t)iw2 * g.mza + kd]) *
-                     (double)(vc03d[x] - vc[x]);
-    v = (float)((double)v + t);
-  }
-  sh_vmt[x] = v;
-}
-
 // ---- divh_damp ----------------------------------------------------------------
 __global__ void k_div_fdivh(DynK g, const int* __restrict__ vprog, int nv, const float* __restrict__ arw0,
                             const float* __restrict__ dniv, const float* __restrict__ zfacit,
@@ -144,49 +129,6 @@ __global__ void k_div_fdivh(DynK g, const int* __restrict__ vprog, int nv, const
     v = (double)fact2 * (double)dniv[iv] * (double)zfacit[kd] * (double)dzit[kd] * vmin;
   }
   fdivh[(size_t)iv * g.mza + kd] = (float)v;
-}
-
-// The saved div2d is not cleared: plane 1 accumulates onto what the previous
-// call left there, as the Fortran does (vort_div_damp.f90:136-148).
-__global__ void k_div_accum(DynK g, const int* __restrict__ prog, int nprog, const float* __restrict__ arv,
-                            const float* __restrict__ vmc, float* __restrict__ div1) {
-  PK(j, kd, nprog);
-  const int iw = WTAB(j);
-  const size_t x = (size_t)iw * g.mza + kd;
-  float d = div1[x];
-  const int np = g.npoly[iw];
-  for (int n = 0; n < np; ++n) {
-    const int iv = g.w_ev[iw * 8 + n];
-    if (kd >= LPV(iv))
-      d = d - arv[(size_t)iv * g.mza + kd] * g.w_dirv[iw * 8 + n] * vmc[(size_t)iv * g.mza + kd];
-  }
-  if (kd >= LPW(iw)) d = d * g.volti[x];
-  div1[x] = d;
-}
-
-// laplacian2d (grad_lib.f90:494-524)
-__global__ void k_lap_w(DynK g, const int* __restrict__ prog, int nprog, const float* __restrict__ xx_yy,
-                        const float* __restrict__ src, float* __restrict__ dst) {
-  PK(j, kd, nprog);
-  const int iw = WTAB(j);
-  const size_t x = (size_t)iw * g.mza + kd;
-  float d = 0.f;
-  const int np = g.npoly[iw];
-  for (int n = 0; n < np; ++n) {
-    const int iv = g.w_ev[iw * 8 + n], iwn = g.w_nb[iw * 8 + n];
-    if (kd >= LPV(iv)) d = d + (src[(size_t)iwn * g.mza + kd] - src[x]) * xx_yy[iw * 7 + n];
-  }
-  dst[x] = d;
-}
-
-__global__ void k_div_apply(DynK g, const int* __restrict__ vprog, int nv, const float* __restrict__ fdivh,
-                            const float* __restrict__ dh, float* __restrict__ vmt) {
-  PK(j, kd, nv);
-  const int iv = VPTAB(j);
-  if (kd < LPV(iv)) return;
-  const int iw1 = g.v_iw[iv * 2], iw2 = g.v_iw[iv * 2 + 1];
-  const size_t x = (size_t)iv * g.mza + kd;
-  vmt[x] = vmt[x] + fdivh[x] * (dh[(size_t)iw2 * g.mza + kd] - dh[(size_t)iw1 * g.mza + kd]);
 }
 
 // ---- vort_damp ----------------------------------------------------------------
@@ -221,52 +163,233 @@ __global__ void k_vort_first_v(DynK g, const int* __restrict__ vprog, int nv, co
   fvortl[iv] = (level > 2) ? 0.50f * dniu[iv] / dtm_f * pl : 0.f;
 }
 
-__global__ void k_vort(DynK g, const int* __restrict__ mprog, int nm, const float* __restrict__ vfact,
-                       const float* __restrict__ vc, float* __restrict__ v1) {
-  PK(j, kd, nm);
-  const int im = mprog[j];
-  float v = 0.f;
-  for (int jv = 0; jv < 3; ++jv) {
-    const int iv = g.m_iv[im * 3 + jv];
-    if (kd >= LPV(iv)) v = v + vc[(size_t)iv * g.mza + kd] * vfact[im * 3 + jv];
+// The per-point kernels below give a warp to a point and R = 1, 2 or 4 levels
+// (mza up to 32, 64, 128) to a lane: the point's table entries are one uniform
+// read a warp, and every load of the R levels is issued before any is used.
+// A thread per (point, level) over the flat range, its neighbours read in
+// turn, left each warp waiting on one or two loads at a time; with one level
+// a lane the table reads weigh as much as the data (NXP=100, 60 levels, one
+// level against two: first planes 174 / 135 us, a Laplacian step 124 / 87,
+// velocities 123 / 78).
+#define WARP_POINT(n, first)                                                  \
+  const int lane = threadIdx.x & 31;                                          \
+  const unsigned w_ = (blockIdx.x - (first)) * 8u + (threadIdx.x >> 5);       \
+  if (w_ >= (unsigned)(n)) return;
+
+struct DampArgs {
+  const int* wprog; int nw;           // divergence of the W columns
+  const int* mprog; int nm;           // vorticity at the M points
+  unsigned mblock;                    // first block of the M part
+  const float* arv; const float* vmc; const float* vc;
+  const float* xx_yy; const float* xx_yy_m; const float* vfact;
+  const float* wsrc; float* wdst;     // planes of the Laplacian step
+  const float* msrc; float* mdst;
+};
+
+// First planes of divh_damp and vort_damp (vort_div_damp.f90:126-148,
+// 296-330), the W columns and the M points side by side in one launch.
+// The saved div2d is not cleared: plane 1 accumulates onto what the previous
+// call left there, as the Fortran does (vort_div_damp.f90:136-148).
+template <int R>
+__global__ void __launch_bounds__(256) k_damp_first(DynK g, DampArgs A) {
+  const int mza = g.mza;
+  if (blockIdx.x < A.mblock) {
+    WARP_POINT(A.nw, 0u);
+    const int* prog = A.wprog;
+    const int iw = WTAB((int)w_), np = g.npoly[iw], kb = LPW(iw);
+    const size_t cb = (size_t)iw * mza;
+    const int4* E = g.edge + (size_t)iw * (7 * EDGE_W / 4);
+    int4 e[6];
+#pragma unroll
+    for (int n = 0; n < 6; ++n) e[n] = __ldg(E + 2 * n);
+    float d[R], vt[R], ar[R][6], vm[R][6];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int kd = lane + 32 * r;
+      d[r] = vt[r] = 0.f;
+      if (kd < mza) { d[r] = A.wdst[cb + kd]; vt[r] = g.volti[cb + kd]; }
+#pragma unroll
+      for (int n = 0; n < 6; ++n) {
+        ar[r][n] = vm[r][n] = 0.f;
+        if (kd < mza && kd >= e[n].z) {
+          const size_t xv = (size_t)(e[n].y & 0x7fffffff) * mza + kd;
+          ar[r][n] = A.arv[xv];
+          vm[r][n] = A.vmc[xv];
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int kd = lane + 32 * r;
+      if (kd >= mza) continue;
+#pragma unroll
+      for (int n = 0; n < 6; ++n) d[r] = d[r] - ar[r][n] * __int_as_float(e[n].w) * vm[r][n];
+      if (np > 6) {
+        const int4 q = __ldg(E + 12);
+        const size_t xv = (size_t)(q.y & 0x7fffffff) * mza + kd;
+        if (kd >= q.z) d[r] = d[r] - A.arv[xv] * __int_as_float(q.w) * A.vmc[xv];
+      }
+      if (kd >= kb) d[r] = d[r] * vt[r];
+      A.wdst[cb + kd] = d[r];
+    }
+  } else {
+    WARP_POINT(A.nm, A.mblock);
+    const int im = A.mprog[w_];
+    int iv[3], lv[3];
+    float f[3], x[R][3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) { iv[q] = g.m_iv[im * 3 + q]; f[q] = A.vfact[im * 3 + q]; }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) lv[q] = LPV(iv[q]);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const int kd = lane + 32 * r;
+        x[r][q] = 0.f;
+        if (kd < mza && kd >= lv[q]) x[r][q] = A.vc[(size_t)iv[q] * mza + kd];
+      }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int kd = lane + 32 * r;
+      float v = 0.f;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) v = v + x[r][q] * f[q];
+      if (kd < mza) A.mdst[(size_t)im * mza + kd] = v;
+    }
   }
-  v1[(size_t)im * g.mza + kd] = v;
 }
 
-// laplacian_m (grad_lib.f90:531-559)
-__global__ void k_lap_m(DynK g, const int* __restrict__ mprog, int nm, const float* __restrict__ xx_yy_m,
-                        const float* __restrict__ src, float* __restrict__ dst) {
-  PK(j, kd, nm);
-  const int im = mprog[j];
-  const size_t x = (size_t)im * g.mza + kd;
-  float d = 0.f;
-  for (int jj = 0; jj < 3; ++jj) {
-    const int imn = g.m_im[im * 3 + jj];
-    if (kd >= LPV(g.m_iv[im * 3 + jj])) d = d + (src[(size_t)imn * g.mza + kd] - src[x]) * xx_yy_m[im * 3 + jj];
+// laplacian2d (grad_lib.f90:494-524) of the divergence plane and laplacian_m
+// (:531-559) of the vorticity plane
+template <int R>
+__global__ void __launch_bounds__(256) k_damp_lap(DynK g, DampArgs A) {
+  const int mza = g.mza;
+  if (blockIdx.x < A.mblock) {
+    WARP_POINT(A.nw, 0u);
+    const int* prog = A.wprog;
+    const int iw = WTAB((int)w_), np = g.npoly[iw];
+    const size_t cb = (size_t)iw * mza;
+    const int4* E = g.edge + (size_t)iw * (7 * EDGE_W / 4);
+    int4 e[6];
+    float c[6];
+#pragma unroll
+    for (int n = 0; n < 6; ++n) { e[n] = __ldg(E + 2 * n); c[n] = A.xx_yy[iw * 7 + n]; }
+    float s[R], x[R][6];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int kd = lane + 32 * r;
+      s[r] = kd < mza ? A.wsrc[cb + kd] : 0.f;
+#pragma unroll
+      for (int n = 0; n < 6; ++n) {
+        x[r][n] = 0.f;
+        if (kd < mza && kd >= e[n].z) x[r][n] = A.wsrc[(size_t)e[n].x * mza + kd];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int kd = lane + 32 * r;
+      if (kd >= mza) continue;
+      float d = 0.f;
+#pragma unroll
+      for (int n = 0; n < 6; ++n) if (kd >= e[n].z) d = d + (x[r][n] - s[r]) * c[n];
+      if (np > 6) {
+        const int4 q = __ldg(E + 12);
+        if (kd >= q.z) d = d + (A.wsrc[(size_t)q.x * mza + kd] - s[r]) * A.xx_yy[iw * 7 + 6];
+      }
+      A.wdst[cb + kd] = d;
+    }
+  } else {
+    WARP_POINT(A.nm, A.mblock);
+    const int im = A.mprog[w_];
+    const size_t cb = (size_t)im * mza;
+    int nb[3], lv[3];
+    float c[3], s[R], x[R][3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      nb[q] = g.m_im[im * 3 + q];
+      c[q] = A.xx_yy_m[im * 3 + q];
+      lv[q] = LPV(g.m_iv[im * 3 + q]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int kd = lane + 32 * r;
+      s[r] = kd < mza ? A.msrc[cb + kd] : 0.f;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        x[r][q] = 0.f;
+        if (kd < mza && kd >= lv[q]) x[r][q] = A.msrc[(size_t)nb[q] * mza + kd];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int kd = lane + 32 * r;
+      float d = 0.f;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) if (kd >= lv[q]) d = d + (x[r][q] - s[r]) * c[q];
+      if (kd < mza) A.mdst[cb + kd] = d;
+    }
   }
-  dst[x] = d;
 }
 
-__global__ void k_vort_apply(DynK g, const int* __restrict__ vprog, int nv, int level,
-                             const float* __restrict__ fvorth, const float* __restrict__ fvortl,
-                             const float* __restrict__ dl, const float* __restrict__ dh,
-                             const double* __restrict__ rho, float* __restrict__ vmt) {
-  PK(j, kd, nv);
-  const int iv = VPTAB(j);
-  if (kd < LPV(iv)) return;
-  const int iw1 = g.v_iw[iv * 2], iw2 = g.v_iw[iv * 2 + 1];
-  const int im1 = g.v_im[iv * 2], im2 = g.v_im[iv * 2 + 1];
-  const float rr = (float)(rho[(size_t)iw1 * g.mza + kd] + rho[(size_t)iw2 * g.mza + kd]);
-  const size_t x = (size_t)iv * g.mza + kd;
-  if (level == 1) {
-    vmt[x] = vmt[x] + fvorth[iv] * (dh[(size_t)im2 * g.mza + kd] - dh[(size_t)im1 * g.mza + kd]) * rr;
-    return;
+// V tendency of the step: the long-step tendency, the Rayleigh term
+// (prog_wrtv_rk.f90:289-303) and both dampings (vort_div_damp.f90:208-230,
+// 400-445), each left out where its switch is off; with vmc0 the start
+// momentum is kept too (prog_wrtv_rk.f90:289)
+struct VtendArgs {
+  const int* vprog; int nv;
+  const float* src; float* dst;       // tendency in and out (may be one array)
+  const float* vmc; float* vmc0;      // NULL vmc0: not kept
+  const float* rayf_cof; const float* vc03d; const float* vc; int krayf_bot;
+  const double* rho;
+  const float* fdivh; const float* dh;             // NULL dh: no divergence damping
+  const float* fvorth; const float* fvortl;        // NULL fvorth: no vorticity damping
+  const float* vl; const float* vh; int vlevel;
+};
+
+// A warp to 32 levels of a V point: here two levels a lane cost more in
+// registers (half the warps) than they save in table reads (203 us against
+// 160 at NXP=100, 60 levels).
+__global__ void __launch_bounds__(256) k_vtend(DynK g, VtendArgs A) {
+  const int mza = g.mza;
+  const unsigned nch = ((unsigned)mza + 31u) / 32u, q = blockIdx.x * 8u + (threadIdx.x >> 5), j = q / nch;
+  if (j >= (unsigned)A.nv) return;
+  const int kd = (int)((q - j * nch) * 32u + (threadIdx.x & 31u));
+  if (kd >= mza) return;
+  const int* vprog = A.vprog;
+  const int iv = VPTAB((int)j), kv = LPV(iv);
+  const int2 iw = *reinterpret_cast<const int2*>(g.v_iw + iv * 2), im = *reinterpret_cast<const int2*>(g.v_im + iv * 2);
+  const size_t x = (size_t)iv * mza + kd;
+  const bool open = kd >= kv, div = A.dh && open, vor = A.fvorth && open;
+  const bool ray = A.rayf_cof && kd >= A.krayf_bot - 1;
+  float t = A.src[x], v0 = 0.f, fd = 0.f, d1 = 0.f, d2 = 0.f, v1 = 0.f, v2 = 0.f, fv = 0.f;
+  double r1 = 0.0, r2 = 0.0;
+  if (A.vmc0) v0 = A.vmc[x];
+  if (div) {
+    fd = A.fdivh[x];
+    d1 = A.dh[(size_t)iw.x * mza + kd];
+    d2 = A.dh[(size_t)iw.y * mza + kd];
   }
-  const int ka = (level == 3) ? max(g.lpm[im1], g.lpm[im2]) : LPV(iv);
-  if (kd < ka)
-    vmt[x] = vmt[x] + fvortl[iv] * (dl[(size_t)im2 * g.mza + kd] - dl[(size_t)im1 * g.mza + kd]) * rr;
-  else
-    vmt[x] = vmt[x] + fvorth[iv] * (dh[(size_t)im2 * g.mza + kd] - dh[(size_t)im1 * g.mza + kd]) * rr;
+  if (vor || ray) {
+    r1 = A.rho[(size_t)iw.x * mza + kd];
+    r2 = A.rho[(size_t)iw.y * mza + kd];
+  }
+  if (vor) {
+    // below ka the level-3 damping takes the second-order plane
+    const int ka = A.vlevel != 3 || g.flat ? kv : max(g.lpm[im.x], g.lpm[im.y]);
+    const float* p = kd < ka ? A.vl : A.vh;
+    fv = kd < ka ? A.fvortl[iv] : A.fvorth[iv];
+    v1 = p[(size_t)im.x * mza + kd];
+    v2 = p[(size_t)im.y * mza + kd];
+  }
+  if (ray) {
+    const double w = (double)(A.rayf_cof[kd] * 0.5f) * (r1 + r2) * (double)(A.vc03d[x] - A.vc[x]);
+    t = (float)((double)t + w);
+  }
+  if (div) t = t + fd * (d2 - d1);
+  if (vor) t = t + fv * (v2 - v1) * (float)(r1 + r2);
+  A.dst[x] = t;
+  if (A.vmc0) A.vmc0[x] = v0;
 }
 
 // ---- stage kernels ----------------------------------------------------------------
@@ -293,22 +416,31 @@ struct VSide { const float* dxps; const float* dyps; const float* xx0_v; const f
 // face unless vmc < 0 -- each face being written by exactly one of its two
 // cells: S(k,iw) + dxps dS/dx + dyps dS/dy (+ the quadratic terms at ORD 3)
 // for the fields in gmask, S(k,iw) alone for those in pmask.  No gradient
-// planes go through memory.  Thread per (column, level); the neighbour loop
-// is outside the field loop, so each neighbour's table entries and
-// coefficients are read once for the four fields.
-template <int ORD>
-__global__ void __launch_bounds__(256, ORD == 2 ? 6 : 1)   // order 2: 40 registers, six blocks per SM
-k_grad_upv4(DynK g, const int* __restrict__ prog, int nprog, Four s, unsigned gmask,
-                            unsigned pmask, const float* __restrict__ cx, const float* __restrict__ cy,
-                            const float* __restrict__ xy_hu, VSide c, const float* __restrict__ vmc,
-                            float* __restrict__ upv) {
-  PK(j, kd, nprog);
+// planes go through memory.  The four values of a face and level are one
+// 16-byte element of upv.  With vmca the cell also writes the mass flux
+// vmc arv of its faces, and with vmasc adds it there (the last stage).
+// A warp per column and 32 levels; the neighbours' values of all four fields
+// are loaded before any is used.
+struct FaceFlux { const float* arv; float* vmca; float* vmasc; };
+
+// ALL: gmask holds the four fields.  Three edges a batch keep it at 64
+// registers, 32 warps an SM: six at a time took 85 registers and 16 warps
+// (316 us at NXP=100, 60 levels, against 208).
+template <int ORD, bool ALL>
+__global__ void __launch_bounds__(256, ORD == 2 ? 4 : 2)
+k_grad_upv4(DynK g, const int* __restrict__ prog, int nprog, int nch, Four s, unsigned gmask_,
+                            unsigned pmask, const float* __restrict__ xy_hu, VSide c, const float* __restrict__ vmc,
+                            float4* __restrict__ upv, FaceFlux ff) {
   constexpr int NPL = ORD == 2 ? 2 : 5;
-  const int iw = WTAB(j);
-  const unsigned mza = g.mza;
-  const size_t vplane = (size_t)g.mva * mza;
-  const unsigned x = (unsigned)iw * mza + kd;
-  const int np = g.npoly[iw];
+  const unsigned gmask = ALL ? 0xFu : gmask_;
+  const unsigned w_ = blockIdx.x * 8u + (threadIdx.x >> 5);
+  const unsigned j = w_ / (unsigned)nch;
+  if (j >= (unsigned)nprog) return;
+  const int mza = g.mza, kd = (int)((w_ - j * (unsigned)nch) * 32u + (threadIdx.x & 31u));
+  if (kd >= mza) return;
+  const int iw = WTAB((int)j), np = g.npoly[iw];
+  const unsigned x = (unsigned)iw * (unsigned)mza + kd;
+  const int4* E = g.edge + (size_t)iw * (7 * EDGE_W / 4);
   float c0[4], a[4][NPL];
 #pragma unroll
   for (int f = 0; f < 4; ++f) {
@@ -316,50 +448,101 @@ k_grad_upv4(DynK g, const int* __restrict__ prog, int nprog, Four s, unsigned gm
 #pragma unroll
     for (int m = 0; m < NPL; ++m) a[f][m] = 0.f;
   }
+  auto gradient = [&](auto cnt, int n0) {
+    constexpr int N = decltype(cnt)::value;
+    int4 e[N];
+    float q[N][4];
 #pragma unroll
-  for (int n = 0; n < 7; ++n) {
-    if (n >= np) break;
-    const int iv = g.w_ev[iw * 8 + n], iwn = g.w_nb[iw * 8 + n];
-    if (kd < LPV(iv)) continue;
-    float w[NPL];
-    if (ORD == 2) {
-      w[0] = cx[iw * 7 + n];
-      w[1] = cy[iw * 7 + n];
-    } else {
+    for (int i = 0; i < N; ++i) e[i] = __ldg(E + 2 * (n0 + i));
 #pragma unroll
-      for (int m = 0; m < NPL; ++m) w[m] = xy_hu[((size_t)iw * 7 + n) * 5 + m];
-    }
-    const unsigned xn = (unsigned)iwn * mza + kd;
+    for (int i = 0; i < N; ++i) {
 #pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      if (!((gmask >> f) & 1u)) continue;
-      const float d = s.f[f][xn] - c0[f];
+      for (int f = 0; f < 4; ++f) q[i][f] = c0[f];
+      if (kd >= e[i].z) {
+        const unsigned xn = (unsigned)e[i].x * (unsigned)mza + kd;
 #pragma unroll
-      for (int m = 0; m < NPL; ++m) a[f][m] = a[f][m] + w[m] * d;
-    }
-  }
-#pragma unroll
-  for (int n = 0; n < 7; ++n) {
-    if (n >= np) break;
-    const int iv = g.w_ev[iw * 8 + n];
-    if (kd < LPV(iv)) continue;
-    const unsigned xv = (unsigned)iv * mza + kd;
-    const int side = g.v_iw[iv * 2] == iw ? 0 : 1;
-    if ((vmc[xv] < 0.f) != (side == 1)) continue;   // the other cell is upwind
-    const float dx = c.dxps[iv * 2 + side], dy = c.dyps[iv * 2 + side];
-    float xx = 0.f, xy = 0.f, yy = 0.f;
-    if (ORD == 3) { xx = c.xx0_v[iv * 2 + side]; xy = c.xy0_v[iv * 2 + side]; yy = c.yy0_v[iv * 2 + side]; }
-#pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      if (!(((gmask | pmask) >> f) & 1u)) continue;
-      float v = c0[f];
-      if ((gmask >> f) & 1u) {
-        v = v + dx * a[f][0] + dy * a[f][1];
-        if (ORD == 3) v = v + xx * a[f][2] + xy * a[f][3] + yy * a[f][4];
+        for (int f = 0; f < 4; ++f) if ((gmask >> f) & 1u) q[i][f] = s.f[f][xn];
       }
-      upv[(size_t)f * vplane + xv] = v;
     }
-  }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      float w[NPL];
+      if (ORD == 2) {
+        const int4 b = __ldg(E + 2 * (n0 + i) + 1);
+        w[0] = __int_as_float(b.x);
+        w[1] = __int_as_float(b.y);
+      } else {
+#pragma unroll
+        for (int m = 0; m < NPL; ++m) w[m] = xy_hu[((size_t)iw * 7 + n0 + i) * 5 + m];
+      }
+      // a closed edge adds nothing: q = c0
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        const float d = q[i][f] - c0[f];
+#pragma unroll
+        for (int m = 0; m < NPL; ++m) a[f][m] = a[f][m] + w[m] * d;
+      }
+    }
+  };
+  gradient(std::integral_constant<int, 3>(), 0);
+  gradient(std::integral_constant<int, 3>(), 3);
+  if (np > 6) gradient(std::integral_constant<int, 1>(), 6);
+  auto faces = [&](auto cnt, int n0) {
+    constexpr int N = decltype(cnt)::value;
+    int4 e[N];
+    float vm[N], ar[N], vs[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) e[i] = __ldg(E + 2 * (n0 + i));
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      vm[i] = ar[i] = vs[i] = 0.f;
+      if (kd >= e[i].z) {
+        const unsigned xv = (unsigned)(e[i].y & 0x7fffffff) * (unsigned)mza + kd;
+        vm[i] = vmc[xv];
+        if (ff.vmca) ar[i] = ff.arv[xv];
+        if (ff.vmasc) vs[i] = ff.vmasc[xv];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int side = e[i].y < 0 ? 1 : 0;
+      if (kd < e[i].z || (vm[i] < 0.f) != (side == 1)) continue;   // closed, or the other cell is upwind
+      const int iv = e[i].y & 0x7fffffff;
+      const unsigned xv = (unsigned)iv * (unsigned)mza + kd;
+      if (ff.vmca) {
+        const float v = vm[i] * ar[i];
+        ff.vmca[xv] = v;
+        if (ff.vmasc) ff.vmasc[xv] = vs[i] + v;
+      }
+      float dx, dy, xx = 0.f, xy = 0.f, yy = 0.f;
+      if (ORD == 2) {
+        const int4 b = __ldg(E + 2 * (n0 + i) + 1);
+        dx = __int_as_float(b.z);
+        dy = __int_as_float(b.w);
+      } else {
+        dx = c.dxps[iv * 2 + side]; dy = c.dyps[iv * 2 + side];
+        xx = c.xx0_v[iv * 2 + side]; xy = c.xy0_v[iv * 2 + side]; yy = c.yy0_v[iv * 2 + side];
+      }
+      float o[4];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        float v = c0[f];
+        if ((gmask >> f) & 1u) {
+          v = v + dx * a[f][0] + dy * a[f][1];
+          if (ORD == 3) v = v + xx * a[f][2] + xy * a[f][3] + yy * a[f][4];
+        }
+        o[f] = v;
+      }
+      if (ALL || (gmask | pmask) == 0xFu) upv[xv] = make_float4(o[0], o[1], o[2], o[3]);
+      else {
+        float* p = reinterpret_cast<float*>(upv + xv);
+#pragma unroll
+        for (int f = 0; f < 4; ++f) if (((gmask | pmask) >> f) & 1u) p[f] = o[f];
+      }
+    }
+  };
+  faces(std::integral_constant<int, 6>(), 0);
+  if (np > 6) faces(std::integral_constant<int, 1>(), 6);
 }
 
 // vertical upwind face values of the four fields (scalar_w_column of
@@ -393,19 +576,20 @@ __global__ void k_upw4(DynK g, const int* __restrict__ prog, int nprog, Four s, 
   }
 }
 
-// ---- prog_wrt_begs: one warp per column ------------------------------------------
+// ---- prog_wrt_begs ------------------------------------------
 struct WrtArgs {
   int istage, nrk;
   double dt8;
   float dts, fcoriol, c8, c9, rocv;
   double pc2, pc3, fr;
   const int* prog; int nprog;
-  const float* vmc; const float* arv;                       // vmca = vmc arv
-  const float* upv; const float* upw;                       // 4-field arrays
-  const float* sh_th; const float* sh_vx; const float* sh_vy; const float* sh_vz;   // *_rk at stage start
+  const float* vmca; const float4* upv;                     // face mass flux, the four face values
+  const float* upw;                                         // 4-field array (not LEAN)
+  // *_rk at stage start: *_short, or the long-step tendencies (LEAN)
+  const float* sh_th; const float* sh_vx; const float* sh_vy; const float* sh_vz;
   float* rk_vx; float* rk_vy; float* rk_vz;
-  double* rho; double* press; const double* rho0; const double* rth0;
-  float* thil; float* wc; float* wmc; const float* wmc0; const float* vxe; const float* vye;
+  double* rho; double* press; double* rho0; double* rth0;
+  float* thil; float* wc; float* wmc; float* wmc0; const float* vxe; const float* vye; const float* vze;
   float* wmasc;
   const float* alpha_press; const float* pwfac;
   const double* volt; const float* volwi; const float* arw; const float* wn;
@@ -413,220 +597,320 @@ struct WrtArgs {
   const double* zwgt_bot8; const double* zwgt_top8; const float* b20;
 };
 
-#define WRT_WARPS 4
-// per-warp shared scratch, arrays of mza entries
-struct WrtSmem {
-  double *hflx, *rt, *b10, *b5, *drt, *pex, *rex, *rhon;
-  float *b15, *rkx, *rky, *rkz, *b31, *b32, *b33, *dwm, *wmf;
-};
+// columns per block: four one-warp columns, else one
+#define WRT_COLS(NW) ((NW) == 1 ? 4 : 1)
 
-// The W system of prog_wrt_begs, b31(k) x(k-1) + b32(k) x(k) + b33(k) x(k+1)
-// = dwm(k) for k = k0 .. k1, which the reference solves with the Thomas
-// algorithm (tridiffo, outils/tridiag_lib.f90:10-36), solved here by
-// parallel cyclic reduction over a warp: row i = k - k0 is updated by lane
-// i % 32 (R rows per lane, i = lane + 32 r); in a step of stride s every row
-// eliminates its couplings to rows i - s and i + s with those rows' current
-// equations (rows outside the system act as identity rows), so after
-// ceil(log2(n)) steps each row holds x(k) = d / b.  A lane keeps its rows'
-// equations in registers and publishes, per step, a, c, d and 1 / b of each
-// in the column's shared memory for the rows that eliminate against it (one
-// division per row and step).  The equations are FP64 (the inputs and the
-// result are the reference's real(4)): w is a small residual of large
-// terms, and FP64 keeps it nearer the exact solve than a real(4) sweep.  The
-// four FP64 arrays reuse pex and rex (not read after phase 2) and the float
-// coefficient arrays themselves (read into registers first).
-template <int R>
-__device__ __forceinline__ void warp_tridiag(WrtSmem& m, int k0, int k1, int lane) {
-  const int n = k1 - k0 + 1;
-  double* A = m.pex;
-  double* RB = m.rex;                               // 1 / b
-  double* Cc = reinterpret_cast<double*>(m.b31);   // b31 and b32: 2 mza floats
-  double* D = reinterpret_cast<double*>(m.b33);    // b33 and dwm
-  double ra[R], rb[R], rc[R], rd[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int i = lane + 32 * r;
-    ra[r] = i < n && i > 0 ? (double)m.b31[k0 + i] : 0.0;
-    rb[r] = i < n ? (double)m.b32[k0 + i] : 1.0;
-    rc[r] = i < n - 1 ? (double)m.b33[k0 + i] : 0.0;
-    rd[r] = i < n ? (double)m.dwm[k0 + i] : 0.0;
-  }
-  __syncwarp();
-  for (int s = 1; s < n; s <<= 1) {
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = lane + 32 * r;
-      if (i < n) { A[i] = ra[r]; RB[i] = 1.0 / rb[r]; Cc[i] = rc[r]; D[i] = rd[r]; }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = lane + 32 * r;
-      if (i >= n) continue;
-      const int im = i - s, ip = i + s;
-      double al = 0.0, ga = 0.0, am = 0.0, cm = 0.0, dm = 0.0, ap = 0.0, cp = 0.0, dp = 0.0;
-      if (im >= 0) { al = -ra[r] * RB[im]; am = A[im]; cm = Cc[im]; dm = D[im]; }
-      if (ip < n) { ga = -rc[r] * RB[ip]; ap = A[ip]; cp = Cc[ip]; dp = D[ip]; }
-      rb[r] = rb[r] + al * cm + ga * ap;
-      rd[r] = rd[r] + al * dm + ga * dp;
-      ra[r] = al * am;
-      rc[r] = ga * cp;
-    }
-    __syncwarp();
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int i = lane + 32 * r;
-    if (i < n) m.wmf[k0 + i] = (float)(rd[r] / rb[r]);
-  }
+// the lanes of a column meet
+template <int NW>
+__device__ __forceinline__ void column_sync() {
+  if constexpr (NW == 1) __syncwarp();
+  else __syncthreads();
 }
 
-__global__ void __launch_bounds__(WRT_WARPS * 32, 8) k_wrt_begs(DynK g, WrtArgs A) {
-  extern __shared__ double wsm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j = blockIdx.x * WRT_WARPS + warp;
-  if (j >= A.nprog) return;
-  const int mza = g.mza;
-  double* base = wsm + (size_t)warp * mza * 13;  // 8 double + 9 float arrays (9 floats <= 5 doubles)
-  WrtSmem m;
-  m.hflx = base; m.rt = base + mza; m.b10 = base + 2 * mza; m.b5 = base + 3 * mza; m.drt = base + 4 * mza;
-  m.pex = base + 5 * mza; m.rex = base + 6 * mza; m.rhon = base + 7 * mza;
-  float* fb = reinterpret_cast<float*>(base + 8 * mza);
-  m.b15 = fb; m.rkx = fb + mza; m.rky = fb + 2 * mza; m.rkz = fb + 3 * mza; m.b31 = fb + 4 * mza;
-  m.b32 = fb + 5 * mza; m.b33 = fb + 6 * mza; m.dwm = fb + 7 * mza; m.wmf = fb + 8 * mza;
+// 1 / x in FP64 from the approximate reciprocal and two Newton steps (each
+// squares the error, 2^-20 at the start); x is a normal number here
+__device__ __forceinline__ double recip(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
 
-  const int iw = A.prog[j];
+// The W system of prog_wrt_begs, b31(k) x(k-1) + b32(k) x(k) + b33(k) x(k+1)
+// = dwm(k) for n levels k, row i of which lane i of the column holds; the
+// reference solves it with the Thomas algorithm (tridiffo,
+// outils/tridiag_lib.f90:10-36).  The equations are FP64 (the inputs and the
+// result are the reference's real(4)): w is a small residual of large terms,
+// and FP64 keeps it nearer the exact solve than a real(4) sweep.
+//
+// n <= 64 (one or two warps a column): one step of cyclic reduction
+// eliminates the even rows, which leaves at most 32 odd rows to the lanes of
+// the first warp, and parallel cyclic reduction solves those: in a step of
+// stride s every row, scaled to a unit diagonal, eliminates its couplings to
+// rows m - s and m + s, whose coefficients come by shuffles (rows outside the
+// system couple with 0).  The even rows follow by substitution.  All rows in
+// parallel cyclic reduction through shared memory took 42 % of the kernel's
+// shared-memory and 30 % of its issue slots.  P: seven arrays of 32 doubles.
+// The solution goes to x[0 .. n) of shared memory.
+template <int NW>
+__device__ __forceinline__ void column_solve(double* P, int n, int i, double ra, double rb, double rc, double rd,
+                                             float* x) {
+  const int m = i >> 1;
+  if (i & 1) {
+    if (i < n) { P[96 + m] = ra; P[128 + m] = rb; P[160 + m] = rc; P[192 + m] = rd; }
+  } else if (i < n) {
+    const double r = recip(rb);
+    P[m] = ra * r; P[32 + m] = rc * r; P[64 + m] = rd * r;
+  }
+  column_sync<NW>();
+  if (i < 32) {
+    const bool even = 2 * i < n, odd = 2 * i + 1 < n, next = 2 * i + 2 < n;
+    const double ae = even ? P[i] : 0.0, ce = even ? P[32 + i] : 0.0, de = even ? P[64 + i] : 0.0;
+    double a = 0.0, c = 0.0, d = 0.0;
+    if (odd) {
+      const double oa = P[96 + i], ob = P[128 + i], oc = P[160 + i], od = P[192 + i];
+      const double an = next ? P[i + 1] : 0.0, cn = next ? P[33 + i] : 0.0, dn = next ? P[65 + i] : 0.0;
+      const double r = recip(ob - oa * ce - oc * an);
+      a = -oa * ae * r;
+      c = -oc * cn * r;
+      d = (od - oa * de - oc * dn) * r;
+    }
+    const int no = n >> 1;   // odd rows
+    for (int s = 1; s < no; s <<= 1) {
+      const double am = __shfl_up_sync(0xffffffffu, a, s), cm = __shfl_up_sync(0xffffffffu, c, s),
+                   dm = __shfl_up_sync(0xffffffffu, d, s);
+      const double ap = __shfl_down_sync(0xffffffffu, a, s), cp = __shfl_down_sync(0xffffffffu, c, s),
+                   dp = __shfl_down_sync(0xffffffffu, d, s);
+      const double r = recip(1.0 - a * cm - c * ap);
+      d = (d - a * dm - c * dp) * r;
+      a = -a * am * r;
+      c = -c * cp * r;
+    }
+    const double below = __shfl_up_sync(0xffffffffu, d, 1);   // row 2 i - 1
+    if (even) x[2 * i] = (float)(de - (i > 0 ? ae * below : 0.0) - ce * d);
+    if (odd) x[2 * i + 1] = (float)d;
+  }
+  column_sync<NW>();
+}
+
+// n up to 128 (four warps a column): parallel cyclic reduction of all rows,
+// each publishing a, c, d and 1 / b per step.  P: four arrays of mza doubles.
+template <>
+__device__ __forceinline__ void column_solve<4>(double* P, int n, int i, double ra, double rb, double rc, double rd,
+                                                float* x) {
+  double* A = P;
+  double* RB = P + 128;                             // 1 / b
+  double* Cc = P + 256;
+  double* D = P + 384;
+  for (int s = 1; s < n; s <<= 1) {
+    if (i < n) { A[i] = ra; RB[i] = recip(rb); Cc[i] = rc; D[i] = rd; }
+    column_sync<4>();
+    if (i < n) {
+      const int im = i - s, ip = i + s;
+      double al = 0.0, ga = 0.0, am = 0.0, cm = 0.0, dm = 0.0, ap = 0.0, cp = 0.0, dp = 0.0;
+      if (im >= 0) { al = -ra * RB[im]; am = A[im]; cm = Cc[im]; dm = D[im]; }
+      if (ip < n) { ga = -rc * RB[ip]; ap = A[ip]; cp = Cc[ip]; dp = D[ip]; }
+      rb = rb + al * cm + ga * ap;
+      rd = rd + al * dm + ga * dp;
+      ra = al * am;
+      rc = ga * cp;
+    }
+    column_sync<4>();
+  }
+  if (i < n) x[i] = (float)(rd * recip(rb));
+  column_sync<4>();
+}
+
+// NW = 1, 2 or 4 warps per column (mza up to 32, 64, 128), a level per lane
+// from the first phase to the last: what only the same level reads later
+// stays in registers, what the levels above and below read goes through
+// shared memory (64 B a level: the two halves of the explicit terms, then the
+// solve's rows; the four fields, then w and rho; the four fields' W-face
+// values).  Every load of a level is issued before the first is used: with a
+// warp per column and two levels a lane in turn, a warp went to memory four
+// times one after the other.
+// LEAN: no eddy, Rayleigh or flux-corrected terms -- the tendencies are
+// formed here from the long-step ones, the first stage keeps the start
+// values, and the W-face values (scalar_w_column of fluxes_wrtv,
+// prog_wrtv_rk.f90:1085-1126) are formed from the column's own rows, so that
+// the set-up pass and the W-face pass are not run.
+template <int NW, bool LEAN>
+__global__ void __launch_bounds__(32 * NW * WRT_COLS(NW), 24 / (NW * WRT_COLS(NW))) k_wrt_begs(DynK g, WrtArgs A) {
+  extern __shared__ double wsm[];
+  constexpr int LANES = 32 * NW;
+  const int grp = threadIdx.x / LANES, i = threadIdx.x - grp * LANES;   // the column of the block, the lane of the column
+  const int j = blockIdx.x * WRT_COLS(NW) + grp;
+  if (j >= A.nprog) return;                                             // whole columns
+  const int mza = g.mza;
+  // the solve's rows share the first half with the explicit terms
+  constexpr int half = NW == 1 ? 224 : 4 * LANES;   // doubles: at least 4 mza and the solve's arrays
+  double* base = wsm + (size_t)grp * (half + 4 * mza);
+  double* PEX = base;
+  double* REX = base + mza;
+  float* B15 = reinterpret_cast<float*>(base + 2 * mza);
+  float* RKX = B15 + mza;
+  float* RKY = B15 + 2 * mza;
+  float* RKZ = B15 + 3 * mza;
+  float* S = reinterpret_cast<float*>(base + half);         // thil, vxe, vye, vze
+  float* WMF = S;
+  double* RHON = base + half + mza;
+  float* U = reinterpret_cast<float*>(base + half + 2 * mza);   // their W-face values
+
+  const int* prog = A.prog;
+  const int iw = WTAB(j);
   const int kb = LPW(iw);
   const int np = g.npoly[iw];
   const size_t cb = (size_t)iw * mza;
-  const size_t wplane = (size_t)g.mwa * mza, vplane = (size_t)g.mva * mza;
-  const float* thil_upw = A.upw;
-  const float* vxe_upw = A.upw + wplane;
-  const float* vye_upw = A.upw + 2 * wplane;
-  const float* vze_upw = A.upw + 3 * wplane;
-  const float wnx = A.wn[iw * 3], wny = A.wn[iw * 3 + 1], wnz = A.wn[iw * 3 + 2];
-  // the column's edges, read once: V point, with the sign bit set where the
-  // edge's dirv is not positive; -1 past npoly
-  int ev[7];
-#pragma unroll
-  for (int n = 0; n < 7; ++n) {
-    const int iv = n < np ? g.w_ev[iw * 8 + n] : -1;
-    ev[n] = (iv >= 0 && !(g.w_dirv[iw * 8 + n] > 0.f)) ? (iv | (int)0x80000000) : iv;
-  }
+  const int4* E = g.edge + (size_t)iw * (7 * EDGE_W / 4);
+  const bool first = A.istage == 1;
+  const bool in = kb + i < mza;
+  const int kd = min(kb + i, mza - 1);   // lanes past the top repeat it and store nothing
+  const size_t x = cb + kd;
 
   // phase 1: horizontal sums, Coriolis and explicit density / rho*thil terms
-  for (int kd = kb + lane; kd < mza; kd += 32) {
-    double hf = 0.0;
-    // *_rk start each stage as *_short (prog_wrtv_rk.f90:320-330)
-    float th = A.sh_th[cb + kd], vx = A.sh_vx[cb + kd], vy = A.sh_vy[cb + kd], vz = A.sh_vz[cb + kd];
+  int4 e[6];
 #pragma unroll
-    for (int n = 0; n < 7; ++n) {
-      if (ev[n] == -1) break;
-      const int iv = ev[n] & 0x7fffffff;
-      if (kd < LPV(iv)) continue;
-      const size_t xv = (size_t)iv * mza + kd;
-      const float vm = A.vmc[xv] * A.arv[xv];
-      const float u0 = A.upv[xv], u1 = A.upv[vplane + xv], u2 = A.upv[2 * vplane + xv],
-                  u3 = A.upv[3 * vplane + xv];
-      if (ev[n] >= 0) {
-        hf = hf + (double)vm;
-        th = th + vm * u0;
-        vx = vx + vm * u1;
-        vy = vy + vm * u2;
-        vz = vz + vm * u3;
-      } else {
-        hf = hf - (double)vm;
-        th = th - vm * u0;
-        vx = vx - vm * u1;
-        vy = vy - vm * u2;
-        vz = vz - vm * u3;
-      }
+  for (int n = 0; n < 6; ++n) e[n] = __ldg(E + 2 * n);
+  float th = A.sh_th[x], vx = A.sh_vx[x], vy = A.sh_vy[x], vz = A.sh_vz[x];
+  const double rho = A.rho[x], volt = A.volt[x];
+  const float thil = A.thil[x], vye = A.vye[x], vxe = A.vxe[x], alpha = A.alpha_press[x];
+  const float vti = g.volti[x];
+  const float vze = LEAN ? A.vze[x] : 0.f, wms = LEAN ? A.wmc[x] : 0.f;
+  float wm0 = wms;
+  double rho0 = rho, t0 = 0.0;
+  if (!(LEAN && first)) { wm0 = A.wmc0[x]; rho0 = A.rho0[x]; }
+  if (!first) t0 = A.rth0[x];
+  const int up = kd < mza - 1 ? 1 : 0;
+  const float arwm = A.arw[x - 1], arw0 = A.arw[x], arwp = A.arw[x + up];
+  const float wcm = A.wc[x - 1], wcp = A.wc[x + up];
+  const float vwi = A.volwi[x], pwf = A.pwfac[x], vtp = g.volti[x + up];
+  float vm[6];
+  float4 fu[6];
+#pragma unroll
+  for (int n = 0; n < 6; ++n) {
+    vm[n] = 0.f;
+    fu[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (kd >= e[n].z) {
+      const size_t xv = (size_t)(e[n].y & 0x7fffffff) * mza + kd;
+      vm[n] = __ldg(A.vmca + xv);
+      fu[n] = __ldg(A.upv + xv);
     }
-    const double rho = A.rho[cb + kd];
-    const float mass = (float)(rho * A.volt[cb + kd]);
-    vx = vx + mass * A.fcoriol * A.vye[cb + kd];
-    vy = vy - mass * A.fcoriol * A.vxe[cb + kd];
-    const double rt = rho * (double)A.thil[cb + kd];
-    const double b10 = A.dt8 * (double)g.volti[cb + kd];
-    const double b5 = (double)(A.alpha_press[cb + kd] * powf((float)rt, A.rocv));
-    double drho = b10 * hf;
-    double drt = b10 * (double)th;
-    if (A.istage > 1) {
-      drho = drho + A.rho0[cb + kd] - rho;
-      drt = drt + A.rth0[cb + kd] - rt;
-    }
-    m.hflx[kd] = hf; m.rt[kd] = rt; m.b10[kd] = b10; m.b5[kd] = b5; m.drt[kd] = drt;
-    m.pex[kd] = b5 * (rt + A.pc2 * drt);
-    m.rex[kd] = rho + A.fr * drho;
-    m.b15[kd] = (float)(b10 * b5);
-    m.rkx[kd] = vx; m.rky[kd] = vy; m.rkz[kd] = vz;
   }
-  __syncwarp();
+  if (LEAN) {
+    const float v4 = (float)volt;
+    th = __fmul_rn(th, v4); vx = __fmul_rn(vx, v4); vy = __fmul_rn(vy, v4); vz = __fmul_rn(vz, v4);
+  }
+  double hf = 0.0;
+  auto add = [&](const int4& q, float m, const float4& v) {
+    if (__int_as_float(q.w) > 0.f) {
+      hf = hf + (double)m;
+      th = th + m * v.x;
+      vx = vx + m * v.y;
+      vy = vy + m * v.z;
+      vz = vz + m * v.w;
+    } else {
+      hf = hf - (double)m;
+      th = th - m * v.x;
+      vx = vx - m * v.y;
+      vy = vy - m * v.z;
+      vz = vz - m * v.w;
+    }
+  };
+#pragma unroll
+  for (int n = 0; n < 6; ++n) add(e[n], vm[n], fu[n]);
+  if (np > 6) {
+    const int4 q = __ldg(E + 12);
+    if (kd >= q.z) {
+      const size_t xv = (size_t)(q.y & 0x7fffffff) * mza + kd;
+      add(q, __ldg(A.vmca + xv), __ldg(A.upv + xv));
+    }
+  }
+  const float mass = (float)(rho * volt);
+  vx = vx + mass * A.fcoriol * vye;
+  vy = vy - mass * A.fcoriol * vxe;
+  const double rt = rho * (double)thil;
+  const double b10 = A.dt8 * (double)vti;
+  const double b5 = (double)(alpha * powf((float)rt, A.rocv));
+  double drho = b10 * hf;
+  double drt = b10 * (double)th;
+  if (!first) {
+    drho = drho + rho0 - rho;
+    drt = drt + t0 - rt;
+  }
+  if (in) {
+    PEX[kd] = b5 * (rt + A.pc2 * drt);
+    REX[kd] = rho + A.fr * drho;
+    B15[kd] = (float)(b10 * b5);
+    RKX[kd] = vx; RKY[kd] = vy; RKZ[kd] = vz;
+    if (LEAN) {
+      S[kd] = thil; S[mza + kd] = vxe; S[2 * mza + kd] = vye; S[3 * mza + kd] = vze;
+      if (first) { A.rho0[x] = rho; A.rth0[x] = rt; A.wmc0[x] = wms; }
+    }
+  }
+  column_sync<NW>();
+  // the W-face values of the lane's level, and below the floor
+  float u[4];
+  if (LEAN) {
+    const bool top = kd == mza - 1, down = wms < 0.f;
+    const int lev = !top && down ? kd + 1 : kd;
+    const float c1 = g.a_w[lev + (down ? 0 : 2 * mza)];
+    const float c2 = g.a_w[lev + (down ? mza : 3 * mza)];
+    const int lu = min(lev + 1, mza - 1), ld = max(lev - 1, kb);
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      const float b = S[f * mza + lev];
+      const float dsk = (lev <= mza - 2) ? S[f * mza + lu] - b : 0.f;
+      const float dskm1 = (lev >= kb + 1) ? b - S[f * mza + ld] : 0.f;
+      u[f] = top ? b : b + dsk * c1 + dskm1 * c2;
+    }
+  } else {
+#pragma unroll
+    for (int f = 0; f < 4; ++f) u[f] = A.upw[(size_t)f * g.mwa * mza + x];
+  }
+  if (in) {
+#pragma unroll
+    for (int f = 0; f < 4; ++f) U[f * mza + kd] = u[f];
+  }
+  if (i < 4) U[i * mza + kb - 1] = LEAN ? S[i * mza + kb] : A.upw[(size_t)i * g.mwa * mza + cb + kb - 1];
+  column_sync<NW>();
   // phase 2: explicit W momentum and the tridiagonal coefficients (faces kb..mza-2)
-  for (int kd = kb + lane; kd <= mza - 2; kd += 32) {
-    const size_t x = cb + kd;
-    const float a = (float)(m.pex[kd] - m.pex[kd + 1]) * A.pwfac[x];
-    const float b = (float)(A.gdz_wgtm8[kd] * m.rex[kd] + A.gdz_wgtp8[kd] * m.rex[kd + 1]);
-    const float c = (wnx * (m.rkx[kd] + m.rkx[kd + 1]) + wny * (m.rky[kd] + m.rky[kd + 1]) +
-                     wnz * (m.rkz[kd] + m.rkz[kd + 1])) * A.volwi[x];
-    m.dwm[kd] = A.wmc0[x] + A.dts * (a - b + c);
-    const float b7 = A.dts * A.volwi[x];
-    const float b8 = A.c8 * A.pwfac[x];
-    const float b21 = b7 * A.wc[x - 1];
-    const float b22 = b7 * A.wc[x + 1];
-    const float b23 = b8 * m.b15[kd];
-    const float b24 = b8 * m.b15[kd + 1];
-    const float b25 = A.c9 * g.volti[x] * A.gdz_wgtm[kd];
-    const float b26 = A.c9 * g.volti[x + 1] * A.gdz_wgtp[kd];
-    m.b31[kd] = -A.arw[x - 1] * (b21 + b25 + b23 * thil_upw[x - 1]);
-    m.b32[kd] = A.b20[kd] + A.arw[x] * (b25 - b26 + (b23 + b24) * thil_upw[x]);
-    m.b33[kd] = A.arw[x + 1] * (b22 + b26 - b24 * thil_upw[x + 1]);
+  const int n = mza - 1 - kb;
+  double ra = 0.0, rb = 1.0, rc = 0.0, rd = 0.0;
+  if (i < n) {
+    const float wnx = A.wn[iw * 3], wny = A.wn[iw * 3 + 1], wnz = A.wn[iw * 3 + 2];
+    const float a = (float)(PEX[kd] - PEX[kd + 1]) * pwf;
+    const float b = (float)(A.gdz_wgtm8[kd] * REX[kd] + A.gdz_wgtp8[kd] * REX[kd + 1]);
+    const float c = (wnx * (vx + RKX[kd + 1]) + wny * (vy + RKY[kd + 1]) + wnz * (vz + RKZ[kd + 1])) * vwi;
+    rd = (double)(wm0 + A.dts * (a - b + c));
+    const float b7 = A.dts * vwi;
+    const float b8 = A.c8 * pwf;
+    const float b21 = b7 * wcm;
+    const float b22 = b7 * wcp;
+    const float b23 = b8 * B15[kd];
+    const float b24 = b8 * B15[kd + 1];
+    const float b25 = A.c9 * vti * A.gdz_wgtm[kd];
+    const float b26 = A.c9 * vtp * A.gdz_wgtp[kd];
+    if (i > 0) ra = (double)(-arwm * (b21 + b25 + b23 * U[kd - 1]));
+    rb = (double)(A.b20[kd] + arw0 * (b25 - b26 + (b23 + b24) * u[0]));
+    if (i < n - 1) rc = (double)(arwp * (b22 + b26 - b24 * U[kd + 1]));
   }
-  __syncwarp();
-  // phase 3: tridiffo's system (faces kb..mza-2) by cyclic reduction across
-  // the warp's lanes
-  if (kb <= mza - 2) {
-    if (mza - 1 - kb <= 64) warp_tridiag<2>(m, kb, mza - 2, lane);
-    else warp_tridiag<4>(m, kb, mza - 2, lane);   // mza <= 128
-  }
-  __syncwarp();
+  column_sync<NW>();
+  // phase 3: tridiffo's system across the column's lanes
+  column_solve<NW>(base, n, i, ra, rb, rc, rd, WMF + kb);
+  const float wf = i < n ? WMF[kd] : 0.f;
   // phase 4: implicit fluxes and the updates of rho, press, thil and vm*et_rk
-  for (int kd = kb + lane; kd < mza; kd += 32) {
-    const size_t x = cb + kd;
-    const float wma = (kd <= mza - 2) ? m.wmf[kd] * A.arw[x] : 0.f;
-    const float wmam = (kd - 1 >= kb) ? m.wmf[kd - 1] * A.arw[x - 1] : 0.f;
-    const double vft = (kd <= mza - 2) ? (double)(wma * thil_upw[x]) : 0.0;
-    const double vftm = (kd - 1 >= kb) ? (double)(wmam * thil_upw[x - 1]) : 0.0;
-    const float vfx = (kd <= mza - 2) ? wma * vxe_upw[x] : 0.f;
-    const float vfxm = (kd - 1 >= kb) ? wmam * vxe_upw[x - 1] : 0.f;
-    const float vfy = (kd <= mza - 2) ? wma * vye_upw[x] : 0.f;
-    const float vfym = (kd - 1 >= kb) ? wmam * vye_upw[x - 1] : 0.f;
-    const float vfz = (kd <= mza - 2) ? wma * vze_upw[x] : 0.f;
-    const float vfzm = (kd - 1 >= kb) ? wmam * vze_upw[x - 1] : 0.f;
-    if (A.istage == A.nrk && kd <= mza - 2) A.wmasc[x] = A.wmasc[x] + wma;
-    const double rhon = A.rho0[x] + A.dt8 * (double)g.volti[x] * (m.hflx[kd] + (double)wmam - (double)wma);
+  if (in) {
+    const float wma = i < n ? wf * arw0 : 0.f;
+    const float wmam = i > 0 ? WMF[kd - 1] * arwm : 0.f;
+    const double vft = i < n ? (double)(wma * u[0]) : 0.0;
+    const double vftm = i > 0 ? (double)(wmam * U[kd - 1]) : 0.0;
+    const float vfx = i < n ? wma * u[1] : 0.f;
+    const float vfxm = i > 0 ? wmam * U[mza + kd - 1] : 0.f;
+    const float vfy = i < n ? wma * u[2] : 0.f;
+    const float vfym = i > 0 ? wmam * U[2 * mza + kd - 1] : 0.f;
+    const float vfz = i < n ? wma * u[3] : 0.f;
+    const float vfzm = i > 0 ? wmam * U[3 * mza + kd - 1] : 0.f;
+    if (A.istage == A.nrk && i < n) A.wmasc[x] = A.wmasc[x] + wma;
+    const double rhon = rho0 + b10 * (hf + (double)wmam - (double)wma);
     A.rho[x] = rhon;
-    m.rhon[kd] = rhon;
-    const double drt = m.drt[kd] + m.b10[kd] * (vftm - vft);
-    A.press[x] = m.b5[kd] * (m.rt[kd] + A.pc3 * drt);
-    A.thil[x] = (float)((m.rt[kd] + drt) / rhon);
-    A.rk_vx[x] = m.rkx[kd] + vfxm - vfx;
-    A.rk_vy[x] = m.rky[kd] + vfym - vfy;
-    A.rk_vz[x] = m.rkz[kd] + vfzm - vfz;
+    RHON[kd] = rhon;
+    drt = drt + b10 * (vftm - vft);
+    A.press[x] = b5 * (rt + A.pc3 * drt);
+    const float thn = (float)((rt + drt) * recip(rhon));
+    A.thil[x] = thn;
+    if (i == 0)
+      for (int k = 0; k < kb; ++k) A.thil[cb + k] = thn;   // bottom values
+    A.rk_vx[x] = vx + vfxm - vfx;
+    A.rk_vy[x] = vy + vfym - vfy;
+    A.rk_vz[x] = vz + vfzm - vfz;
   }
-  __syncwarp();
-  // phase 5: W momentum and velocity, bottom values
-  for (int kd = kb + lane; kd <= mza - 2; kd += 32) {
-    const size_t x = cb + kd;
-    const float wf = m.wmf[kd];
+  column_sync<NW>();
+  // phase 5: W momentum and velocity
+  if (i < n) {
     A.wmc[x] = wf;
-    A.wc[x] = wf / (float)(A.zwgt_bot8[kd] * m.rhon[kd] + A.zwgt_top8[kd] * m.rhon[kd + 1]);
-  }
-  __syncwarp();
-  if (lane == 0) {
-    A.wc[cb + kb - 1] = A.wc[cb + kb];
-    const float t = A.thil[cb + kb];
-    for (int kd = 0; kd < kb; ++kd) A.thil[cb + kd] = t;
+    const float w = wf / (float)(A.zwgt_bot8[kd] * RHON[kd] + A.zwgt_top8[kd] * RHON[kd + 1]);
+    A.wc[x] = w;
+    if (i == 0) A.wc[x - 1] = w;
   }
 }
 
@@ -693,49 +977,76 @@ static Shaved shaved_args(const Dyn& y, const Transport& tp, int prog, float dts
 // update_vxe_undrgnd (prog_wrtv_rk.f90:1558-1595) and vel_t3d_hex
 // (vel_t3d.f90:39-108): a closed face (below its lpv) contributes the normal
 // component of the cell's prognosed velocity at that level
-__global__ void k_vel_t3d(DynK g, const int* __restrict__ prog, int nprog, const float* __restrict__ wc,
+// ecv: four floats per edge (x, y, z, 0), 7 edges per column
+template <int R>
+__global__ void __launch_bounds__(256) k_vel_t3d(DynK g, const int* __restrict__ prog, int nprog, const float* __restrict__ wc,
                           const float* __restrict__ vc, const float* __restrict__ wno2,
-                          const float* __restrict__ ecv, float* __restrict__ vxe, float* __restrict__ vye,
+                          const float4* __restrict__ ecv, float* __restrict__ vxe, float* __restrict__ vye,
                           float* __restrict__ vze, Shaved sh) {
-  PK(j, kd, nprog);
-  const int iw = WTAB(j);
-  const int kb = LPW(iw);
-  if (kd < kb) return;
+  WARP_POINT(nprog, 0u);
   const int mza = g.mza;
+  const int iw = WTAB((int)w_), kb = LPW(iw), np = g.npoly[iw];
   const size_t cb = (size_t)iw * mza;
-  const int ks = kd - kb;
-  const bool shaved = sh.lve2 && ks < sh.lve2[iw];
-  float p1x = 0.f, p1y = 0.f, p1z = 0.f;
-  if (shaved) {
-    if (sh.prog) {
-      const float rsi = 1.0f / (float)sh.rho[cb + kd];
-      const float vt = g.volti[cb + kd];
-      const float* m = sh.vm0 + ((size_t)iw * sh.nve2 + ks) * 3;
-      p1x = (m[0] + sh.dts * (sh.rkx[cb + kd] * vt)) * rsi;
-      p1y = (m[1] + sh.dts * (sh.rky[cb + kd] * vt)) * rsi;
-      p1z = (m[2] + sh.dts * (sh.rkz[cb + kd] * vt)) * rsi;
-    } else {
-      p1x = vxe[cb + kd]; p1y = vye[cb + kd]; p1z = vze[cb + kd];
+  const int4* E = g.edge + (size_t)iw * (7 * EDGE_W / 4);
+  const float wx = wno2[iw * 3], wy = wno2[iw * 3 + 1], wz = wno2[iw * 3 + 2];
+  const int lve = sh.lve2 ? sh.lve2[iw] : 0;
+  int4 e[6];
+  float4 ec[6];
+#pragma unroll
+  for (int n = 0; n < 6; ++n) { e[n] = __ldg(E + 2 * n); ec[n] = __ldg(ecv + iw * 7 + n); }
+  float wl[R], wu[R], v[R][6];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int kd = lane + 32 * r;
+    wl[r] = wu[r] = 0.f;
+    if (kd >= kb && kd < mza) { wl[r] = wc[cb + kd - 1]; wu[r] = wc[cb + kd]; }
+#pragma unroll
+    for (int n = 0; n < 6; ++n) {
+      v[r][n] = 0.f;
+      if (kd >= e[n].z && kd < mza) v[r][n] = vc[(size_t)(e[n].y & 0x7fffffff) * mza + kd];
     }
   }
-  const float wst = wc[cb + kd - 1] + wc[cb + kd];
-  float x = wst * wno2[iw * 3], y = wst * wno2[iw * 3 + 1], z = wst * wno2[iw * 3 + 2];
-  const int np = g.npoly[iw];
 #pragma unroll
-  for (int n = 0; n < 7; ++n) {
-    if (n >= np) break;
-    const int iv = g.w_ev[iw * 8 + n];
-    float v;
-    if (kd >= LPV(iv)) v = vc[(size_t)iv * mza + kd];
-    else if (shaved) v = sh.vn[iv * 3] * p1x + sh.vn[iv * 3 + 1] * p1y + sh.vn[iv * 3 + 2] * p1z;
-    else continue;
-    x = x + ecv[(iw * 7 + n) * 3] * v;
-    y = y + ecv[(iw * 7 + n) * 3 + 1] * v;
-    z = z + ecv[(iw * 7 + n) * 3 + 2] * v;
+  for (int r = 0; r < R; ++r) {
+    const int kd = lane + 32 * r;
+    if (kd < kb || kd >= mza) continue;
+    const int ks = kd - kb;
+    const bool shaved = ks < lve;
+    float p1x = 0.f, p1y = 0.f, p1z = 0.f;
+    if (shaved) {
+      if (sh.prog) {
+        const float rsi = 1.0f / (float)sh.rho[cb + kd];
+        const float vt = g.volti[cb + kd];
+        const float* m = sh.vm0 + ((size_t)iw * sh.nve2 + ks) * 3;
+        p1x = (m[0] + sh.dts * (sh.rkx[cb + kd] * vt)) * rsi;
+        p1y = (m[1] + sh.dts * (sh.rky[cb + kd] * vt)) * rsi;
+        p1z = (m[2] + sh.dts * (sh.rkz[cb + kd] * vt)) * rsi;
+      } else {
+        p1x = vxe[cb + kd]; p1y = vye[cb + kd]; p1z = vze[cb + kd];
+      }
+    }
+    const float wst = wl[r] + wu[r];
+    float x = wst * wx, y = wst * wy, z = wst * wz;
+    auto add = [&](const int4& q, const float4& c, float u) {
+      if (kd < q.z) {   // a face under ground
+        if (!shaved) return;
+        const int iv = q.y & 0x7fffffff;
+        u = sh.vn[iv * 3] * p1x + sh.vn[iv * 3 + 1] * p1y + sh.vn[iv * 3 + 2] * p1z;
+      }
+      x = x + c.x * u;
+      y = y + c.y * u;
+      z = z + c.z * u;
+    };
+#pragma unroll
+    for (int n = 0; n < 6; ++n) if (n < 5 || np > 5) add(e[n], ec[n], v[r][n]);
+    if (np > 6) {
+      const int4 q = __ldg(E + 12);
+      add(q, __ldg(ecv + iw * 7 + 6), kd >= q.z ? vc[(size_t)(q.y & 0x7fffffff) * mza + kd] : 0.f);
+    }
+    vxe[cb + kd] = x; vye[cb + kd] = y; vze[cb + kd] = z;
+    if (kd == kb)
+      for (int k2 = 0; k2 < kb; ++k2) { vxe[cb + k2] = x; vye[cb + k2] = y; vze[cb + k2] = z; }
   }
-  vxe[cb + kd] = x; vye[cb + kd] = y; vze[cb + kd] = z;
-  if (kd == kb)
-    for (int k2 = 0; k2 < kb; ++k2) { vxe[cb + k2] = x; vye[cb + k2] = y; vze[cb + k2] = z; }
 }
 
 // tend0 (timestep.f90:430-496) for the hot-path arrays
@@ -834,14 +1145,14 @@ int dyn_setup(const olamgpu_grid* g, const olamgpu_opts* o, cudaStream_t s) {
   OG_CHECK(up(y.volt, g->volt, (size_t)mza * mwa, s, "volt"));
   {
     if (!g->wnx || !g->wnxo2 || !g->vnx || !g->ecvec_vx) { set_error("normals/ecvec missing"); return OLAMGPU_E_ARG; }
-    std::vector<float> wn((size_t)mwa * 3), wno2((size_t)mwa * 3), vn((size_t)mva * 3), ec((size_t)mwa * 21);
+    std::vector<float> wn((size_t)mwa * 3), wno2((size_t)mwa * 3), vn((size_t)mva * 3), ec((size_t)mwa * 28, 0.f);
     for (int i = 0; i < mwa; ++i) {
       wn[i * 3] = g->wnx[i]; wn[i * 3 + 1] = g->wny[i]; wn[i * 3 + 2] = g->wnz[i];
       wno2[i * 3] = g->wnxo2[i]; wno2[i * 3 + 1] = g->wnyo2[i]; wno2[i * 3 + 2] = g->wnzo2[i];
       for (int n = 0; n < 7; ++n) {
-        ec[(i * 7 + n) * 3] = g->ecvec_vx[i * 7 + n];
-        ec[(i * 7 + n) * 3 + 1] = g->ecvec_vy[i * 7 + n];
-        ec[(i * 7 + n) * 3 + 2] = g->ecvec_vz[i * 7 + n];
+        ec[(i * 7 + n) * 4] = g->ecvec_vx[i * 7 + n];
+        ec[(i * 7 + n) * 4 + 1] = g->ecvec_vy[i * 7 + n];
+        ec[(i * 7 + n) * 4 + 2] = g->ecvec_vz[i * 7 + n];
       }
     }
     for (int i = 0; i < mva; ++i) { vn[i * 3] = g->vnx[i]; vn[i * 3 + 1] = g->vny[i]; vn[i * 3 + 2] = g->vnz[i]; }
@@ -989,84 +1300,101 @@ int dyn_state_to_host(unsigned mask, cudaStream_t s) {
                       OLAMGPU_F_VXE | OLAMGPU_F_VMC | OLAMGPU_F_VC | OLAMGPU_F_VMASC | OLAMGPU_F_WMASC | \
                       OLAMGPU_F_TEND)
 
-static int divh_damp(Context& C, float* vmt, double dtm, cudaStream_t s) {
+// a kernel template's instance for the levels of the grid
+#define BY_ROWS(mza, ...)               \
+  do {                                  \
+    if ((mza) <= 32) { constexpr int R = 1; __VA_ARGS__; }      \
+    else if ((mza) <= 64) { constexpr int R = 2; __VA_ARGS__; } \
+    else { constexpr int R = 4; __VA_ARGS__; }                  \
+    OG_LAUNCHED();                      \
+  } while (0)
+
+static bool divh_on(const olamgpu_opts& o) { return o.divh_damp_fact > 1.e-7f && o.divh_damp_level > 0; }
+static bool vort_on(const olamgpu_opts& o) { return !(o.vort_damp_fact < 1.e-7f) && o.vort_damp_level > 0; }
+
+// divh_damp and / or vort_damp of a step dtm, added to the V tendency src ->
+// dst.  With setup also prog_wrtv_rk's V set-up: the Rayleigh term on the
+// tendency and the start momentum vmc0.
+static int v_tendency(Context& C, bool div, bool vor, bool setup, const float* src, float* dst, double dtm,
+                      cudaStream_t s) {
   const olamgpu_opts& o = C.opts;
   const DevGrid& d = C.g;
   Dyn& y = C.dy;
-  if (!(o.divh_damp_fact > 1.e-7f) || o.divh_damp_level <= 0) return OLAMGPU_OK;
-  const int level = o.divh_damp_level;
   const DynK g = dynk(d);
-  const size_t wz = (size_t)d.mza * d.mwa;
-  const unsigned nbv = cdiv((size_t)d.nv_prog * d.mza, 256), nbw = cdiv((size_t)d.nw_prog * d.mza, 256);
-  if (y.div_first) {
+  const int mza = d.mza;
+  const size_t wz = (size_t)mza * d.mwa, mz = (size_t)mza * d.mma;
+  div = div && divh_on(o);
+  vor = vor && vort_on(o);
+  if (div && y.div_first) {
     y.div_first = false;
     cudaMemsetAsync(y.div2d.p, 0, 2 * wz * sizeof(float), s);
     float p = 1.f;
-    for (int i = 0; i < level; ++i) p = p * (-o.divh_damp_fact);
+    for (int i = 0; i < o.divh_damp_level; ++i) p = p * (-o.divh_damp_fact);
     const double facth = -((double)p / dtm);
     const float fact2 = o.divh_damp_fact / (float)dtm;
-    k_div_fdivh<<<nbv, 256, 0, s>>>(g, d.jtv_prog.p, d.nv_prog, y.arw0.p, y.dniv.p, y.zfacit.p, y.dzit.p,
-                                    y.volt.p, facth, level, fact2, y.fdivh.p);
+    k_div_fdivh<<<cdiv((size_t)d.nv_prog * mza, 256), 256, 0, s>>>(g, d.jtv_prog.p, d.nv_prog, y.arw0.p, y.dniv.p,
+                                                                   y.zfacit.p, y.dzit.p, y.volt.p, facth,
+                                                                   o.divh_damp_level, fact2, y.fdivh.p);
     OG_LAUNCHED();
   }
-  float* d1 = y.div2d.p;
-  k_div_accum<<<nbw, 256, 0, s>>>(g, d.jtw_prog.p, d.nw_prog, y.arv.p, y.vmc.p, d1);
-  OG_LAUNCHED();
-  // border divergence for the Laplacian and the apply (vort_div_damp.f90:150)
-  { HField f[1] = {{d1, 4}}; OG_CHECK(halo_exchange_fields(C, HALO_W, f, 1, s)); }
-  const float* dh = d1;
-  if (level > 1) {
-    int ih = 2;
-    for (int nn = 1; nn <= level - 1; ++nn) {
-      const int il = (nn - 1) % 2 + 1;
-      ih = nn % 2 + 1;
-      k_lap_w<<<nbw, 256, 0, s>>>(g, d.jtw_prog.p, d.nw_prog, y.xx_yy.p, y.div2d.p + (il - 1) * wz,
-                                  y.div2d.p + (ih - 1) * wz);
-      OG_LAUNCHED();
-      { HField f[1] = {{y.div2d.p + (ih - 1) * wz, 4}}; OG_CHECK(halo_exchange_fields(C, HALO_W, f, 1, s)); }
-    }
-    dh = y.div2d.p + (ih - 1) * wz;
-  }
-  k_div_apply<<<nbv, 256, 0, s>>>(g, d.jtv_prog.p, d.nv_prog, y.fdivh.p, dh, vmt);
-  OG_LAUNCHED();
-  return OLAMGPU_OK;
-}
-
-static int vort_damp(Context& C, float* vmt, double dtm, cudaStream_t s) {
-  const olamgpu_opts& o = C.opts;
-  const DevGrid& d = C.g;
-  Dyn& y = C.dy;
-  if (o.vort_damp_fact < 1.e-7f || o.vort_damp_level <= 0) return OLAMGPU_OK;
-  const int level = o.vort_damp_level;
-  const DynK g = dynk(d);
-  const size_t mz = (size_t)d.mza * d.mma;
-  if (y.vort_first) {
+  if (vor && y.vort_first) {
     y.vort_first = false;
     k_vort_first_m<<<cdiv(d.nm_prog, 128), 128, 0, s>>>(g, d.jtm_prog.p, d.nm_prog, y.dnv.p, y.arm0.p, y.vfact.p,
                                                         y.lpmmin.p);
     k_vort_first_v<<<cdiv(d.nv_prog, 128), 128, 0, s>>>(g, d.jtv_prog.p, d.nv_prog, y.dniu.p, y.arm0.p, (float)dtm,
-                                                        o.vort_damp_fact, level, y.fvorth.p, y.fvortl.p);
+                                                        o.vort_damp_fact, o.vort_damp_level, y.fvorth.p, y.fvortl.p);
     OG_LAUNCHED(); OG_LAUNCHED();
   }
-  const unsigned nbm = cdiv((size_t)d.nm_prog * d.mza, 256), nbv = cdiv((size_t)d.nv_prog * d.mza, 256);
-  k_vort<<<nbm, 256, 0, s>>>(g, d.jtm_prog.p, d.nm_prog, y.vfact.p, y.vc.p, y.vort2d.p);
-  OG_LAUNCHED();
-  { HField f[1] = {{y.vort2d.p, 4}}; OG_CHECK(halo_exchange_fields(C, HALO_M, f, 1, s)); }
-  int il = 1, ih = 1;
-  if (level > 1) {
-    for (int nn = 1; nn <= level - 1; ++nn) {
-      il = (nn - 1) % 2 + 1;
-      ih = nn % 2 + 1;
-      k_lap_m<<<nbm, 256, 0, s>>>(g, d.jtm_prog.p, d.nm_prog, y.xx_yy_m.p, y.vort2d.p + (il - 1) * mz,
-                                  y.vort2d.p + (ih - 1) * mz);
-      OG_LAUNCHED();
-      { HField f[1] = {{y.vort2d.p + (ih - 1) * mz, 4}}; OG_CHECK(halo_exchange_fields(C, HALO_M, f, 1, s)); }
-    }
+  // the planes each Laplacian step reads and writes: 1 -> 2 -> 1 ...
+  auto plane = [](float* p, size_t n, int i) { return p + (size_t)(i - 1) * n; };
+  DampArgs A;
+  A.wprog = d.jtw_prog.p; A.mprog = d.jtm_prog.p;
+  A.arv = y.arv.p; A.vmc = y.vmc.p; A.vc = y.vc.p;
+  A.xx_yy = y.xx_yy.p; A.xx_yy_m = y.xx_yy_m.p; A.vfact = y.vfact.p;
+  auto run = [&](int step, bool dw, bool dm) -> int {   // step 0: the first planes
+    A.nw = dw ? d.nw_prog : 0;
+    A.nm = dm ? d.nm_prog : 0;
+    A.mblock = cdiv(A.nw, 8);
+    const unsigned nb = A.mblock + cdiv(A.nm, 8);
+    const int il = step == 0 ? 1 : (step - 1) % 2 + 1, ih = step == 0 ? 1 : step % 2 + 1;
+    A.wsrc = plane(y.div2d.p, wz, il); A.wdst = plane(y.div2d.p, wz, ih);
+    A.msrc = plane(y.vort2d.p, mz, il); A.mdst = plane(y.vort2d.p, mz, ih);
+    if (nb == 0) return OLAMGPU_OK;
+    if (step == 0) BY_ROWS(mza, k_damp_first<R><<<nb, 256, 0, s>>>(g, A));
+    else BY_ROWS(mza, k_damp_lap<R><<<nb, 256, 0, s>>>(g, A));
+    // border planes for the Laplacian and the apply (vort_div_damp.f90:150, 208)
+    if (dw) { HField f[1] = {{A.wdst, 4}}; OG_CHECK(halo_exchange_fields(C, HALO_W, f, 1, s)); }
+    if (dm) { HField f[1] = {{A.mdst, 4}}; OG_CHECK(halo_exchange_fields(C, HALO_M, f, 1, s)); }
+    return OLAMGPU_OK;
+  };
+  const int ld = div ? o.divh_damp_level : 0, lv = vor ? o.vort_damp_level : 0;
+  for (int step = 0; step < std::max(ld, lv); ++step) OG_CHECK(run(step, step < ld, step < lv));
+  if (!div && !vor && !setup) return OLAMGPU_OK;
+  VtendArgs V{};
+  V.vprog = d.jtv_prog.p; V.nv = d.nv_prog; V.src = src; V.dst = dst;
+  V.vmc = y.vmc.p; V.rho = C.tp.rho.p; V.vc = y.vc.p;
+  if (setup) {
+    V.vmc0 = y.vmc0.p;
+    V.rayf_cof = (o.rayf_cof && o.vc03d) ? y.rayf_cof.p : nullptr;
+    V.vc03d = y.vc03d.p;
+    V.krayf_bot = o.krayf_bot;
   }
-  k_vort_apply<<<nbv, 256, 0, s>>>(g, d.jtv_prog.p, d.nv_prog, level, y.fvorth.p, y.fvortl.p,
-                                   y.vort2d.p + (il - 1) * mz, y.vort2d.p + (ih - 1) * mz, C.tp.rho.p, vmt);
-  OG_LAUNCHED();
+  if (div) { V.fdivh = y.fdivh.p; V.dh = plane(y.div2d.p, wz, ld == 1 ? 1 : (ld - 1) % 2 + 1); }
+  if (vor) {
+    V.fvorth = y.fvorth.p; V.fvortl = y.fvortl.p; V.vlevel = lv;
+    V.vl = plane(y.vort2d.p, mz, lv == 1 ? 1 : (lv - 2) % 2 + 1);
+    V.vh = plane(y.vort2d.p, mz, lv == 1 ? 1 : (lv - 1) % 2 + 1);
+  }
+  if (d.nv_prog > 0) { k_vtend<<<cdiv((size_t)d.nv_prog * ((mza + 31) / 32), 8), 256, 0, s>>>(g, V); OG_LAUNCHED(); }
   return OLAMGPU_OK;
+}
+
+static void launch_vel_t3d(Context& C, const Shaved& sh, cudaStream_t s) {
+  const DevGrid& d = C.g;
+  Dyn& y = C.dy;
+  BY_ROWS(d.mza, k_vel_t3d<R><<<cdiv(d.nw_prog, 8), 256, 0, s>>>(dynk(d), d.jtw_prog.p, d.nw_prog, C.tp.wc.p, y.vc.p, y.wno2.p,
+                                                                 reinterpret_cast<const float4*>(y.ecv.p), y.vxe.p,
+                                                                 y.vye.p, y.vze.p, sh));
 }
 
 int dyn_prog_wrtv_rk(int istp) {
@@ -1095,8 +1423,10 @@ int dyn_prog_wrtv_rk(int istp) {
   const unsigned nbw = cdiv((size_t)d.nw_prog * mza, 256), nbv = cdiv((size_t)d.nv_prog * mza, 256),
                  nbva = cdiv((size_t)d.nv_wadj * mza, 256);
   OG_PROF("prog_wrtv_rk", s);
-  if (!o.divh_damp_short && istp == 1) { OG_PROF("divh_damp", s); OG_CHECK(divh_damp(C, y.vmt.p, o.dtlm, s)); }
-  if (!o.vort_damp_short && istp == 1) { OG_PROF("vort_damp", s); OG_CHECK(vort_damp(C, y.vmt.p, o.dtlm, s)); }
+  if (istp == 1 && (!o.divh_damp_short || !o.vort_damp_short)) {
+    OG_PROF("v_tendency", s);
+    OG_CHECK(v_tendency(C, !o.divh_damp_short, !o.vort_damp_short, false, y.vmt.p, y.vmt.p, o.dtlm, s));
+  }
   SetupW sw{tp.rho.p, y.thil.p, y.wmc.p, y.thilt.p, y.vmxet.p, y.vmyet.p, y.vmzet.p, y.volt.p, y.rho0.p,
             y.rth0.p, y.wmc0.p, y.sh_th.p, y.sh_vx.p, y.sh_vy.p, y.sh_vz.p, y.rayf_cof.p, y.dn01d.p, y.th01d.p,
             o.krayf_bot};
@@ -1109,20 +1439,18 @@ int dyn_prog_wrtv_rk(int istp) {
                                                                              tp.rho.p, y.vm0.p);
     OG_LAUNCHED();
   }
-  { OG_PROF("setup_w", s); k_setup_w<<<nbw, 256, 0, s>>>(g, d.jtw_prog.p, d.nw_prog, sw); OG_LAUNCHED(); }
-  {
-    OG_PROF("setup_v", s);
-    k_setup_v<<<nbv, 256, 0, s>>>(g, d.jtv_prog.p, d.nv_prog, y.vmc.p, y.vmt.p, y.vmc0.p, y.sh_vmt.p,
-                                  (o.rayf_cof && o.vc03d) ? y.rayf_cof.p : nullptr, y.vc03d.p, y.vc.p, tp.rho.p,
-                                  o.krayf_bot);
-    OG_LAUNCHED();
-  }
+  // Without eddy, Rayleigh or flux-corrected terms the column kernel forms
+  // the start values, the tendencies and the W-face values itself.
+  const bool lean = !y.eddy_on && !rayleigh_th && o.ithil_monot <= 0 && o.iwind_monot <= 0;
+  if (!lean) { OG_PROF("setup_w", s); k_setup_w<<<nbw, 256, 0, s>>>(g, d.jtw_prog.p, d.nw_prog, sw); OG_LAUNCHED(); }
   if (y.eddy_on) {
     OG_PROF("eddy_columns", s);
     OG_CHECK(dyn_eddy_columns(C, rayleigh_th, s));
   }
-  if (o.divh_damp_short) { OG_PROF("divh_damp", s); OG_CHECK(divh_damp(C, y.sh_vmt.p, o.dtsm, s)); }
-  if (o.vort_damp_short) { OG_PROF("vort_damp", s); OG_CHECK(vort_damp(C, y.sh_vmt.p, o.dtsm, s)); }
+  {
+    OG_PROF("v_tendency", s);
+    OG_CHECK(v_tendency(C, o.divh_damp_short != 0, o.vort_damp_short != 0, true, y.vmt.p, y.sh_vmt.p, o.dtsm, s));
+  }
   // start values of the fields fluxes_wrtv_monot limits (prog_wrtv_rk.f90:186-198)
   const bool thil_monot = o.ithil_monot > 0, wind_monot = o.iwind_monot > 0;
   const size_t wzb = (size_t)mza * d.mwa * sizeof(float);
@@ -1147,11 +1475,14 @@ int dyn_prog_wrtv_rk(int istp) {
     const double dt8 = (nrk <= 2 ? xstg2[istage - 1] : xstg3[istage - 1]) * o.dtsm;
     const float dts = (float)dt8;
     const int last = istage == nrk;
-    // vmca = vmc arv is formed where it is read; the last stage also keeps
-    // it (the flux-corrected faces read it) and adds it to vmasc
-    if (last) {
+    // vmca = vmc arv, added to vmasc on the last stage: formed with the face
+    // values, or, on a rank with a halo, whose ring-1 columns have faces
+    // outside jtv_wadj, over that table
+    FaceFlux ffx{y.arv.p, y.vmca.p, last ? tp.vmasc.p : nullptr};
+    if (C.halo.on) {
+      ffx = FaceFlux{};
       OG_PROF("vmca", s);
-      k_vmca<<<nbva, 256, 0, s>>>(g, d.jtv_wadj.p, d.nv_wadj, y.vmc.p, y.arv.p, y.vmca.p, tp.vmasc.p, 1);
+      k_vmca<<<nbva, 256, 0, s>>>(g, d.jtv_wadj.p, d.nv_wadj, y.vmc.p, y.arv.p, y.vmca.p, tp.vmasc.p, last);
       OG_LAUNCHED();
     }
     Four f{{y.thil.p, y.vxe.p, y.vye.p, y.vze.p}};
@@ -1161,7 +1492,7 @@ int dyn_prog_wrtv_rk(int istp) {
                          o.wind_horiz_adv_order};
     unsigned m2 = 0, m3 = 0;
     for (int q = 0; q < 4; ++q) { if (ordf[q] == 2) m2 |= 1u << q; if (ordf[q] >= 3) m3 |= 1u << q; }
-    {
+    if (!lean) {
       OG_PROF("upw4", s);
       k_upw4<<<nbw, 256, 0, s>>>(g, d.jtw_prog.p, d.nw_prog, f, y.wmc.p, y.upw.p);
       OG_LAUNCHED();
@@ -1174,23 +1505,24 @@ int dyn_prog_wrtv_rk(int istp) {
       DynK gg = g;
       const int* gt = d.jtw_prog.p;
       int gn = d.nw_prog;
-      unsigned nbg = nbw;
       if (C.halo.on) {
         gg.off_w = d.off_wwadj;
         gt = d.jtw_wadj.p;
         gn = d.nw_wadj;
-        nbg = cdiv((size_t)gn * mza, 256);
       }
+      const int nch = (mza + 31) / 32;
+      const unsigned nbg = cdiv((size_t)gn * nch, 8);
       VSide vs{d.dxps.p, d.dyps.p, d.xx0_v.p, d.xy0_v.p, d.yy0_v.p};
+      float4* upv = reinterpret_cast<float4*>(y.upv.p);
       const unsigned plain = 0xFu & ~(m2 | m3);
       if (m2 || plain) {
-        k_grad_upv4<2><<<nbg, 256, 0, s>>>(gg, gt, gn, f, m2, plain, d.gxc.p, d.gyc.p, d.xy_hu.p, vs, y.vmc.p,
-                                           y.upv.p);
+        if (m2 == 0xFu) k_grad_upv4<2, true><<<nbg, 256, 0, s>>>(gg, gt, gn, nch, f, m2, plain, d.xy_hu.p, vs, y.vmc.p, upv, ffx);
+        else k_grad_upv4<2, false><<<nbg, 256, 0, s>>>(gg, gt, gn, nch, f, m2, plain, d.xy_hu.p, vs, y.vmc.p, upv, ffx);
         OG_LAUNCHED();
+        ffx = FaceFlux{};   // once a stage
       }
       if (m3) {
-        k_grad_upv4<3><<<nbg, 256, 0, s>>>(gg, gt, gn, f, m3, 0u, d.gxc.p, d.gyc.p, d.xy_hu.p, vs, y.vmc.p,
-                                           y.upv.p);
+        k_grad_upv4<3, false><<<nbg, 256, 0, s>>>(gg, gt, gn, nch, f, m3, 0u, d.xy_hu.p, vs, y.vmc.p, upv, ffx);
         OG_LAUNCHED();
       }
     }
@@ -1215,22 +1547,27 @@ int dyn_prog_wrtv_rk(int istp) {
     A.c8 = dts * (float)A.pc2;
     A.c9 = -dts * dts * (float)A.fr;
     A.prog = d.jtw_prog.p; A.nprog = d.nw_prog;
-    A.vmc = y.vmc.p; A.arv = y.arv.p; A.upv = y.upv.p; A.upw = y.upw.p;
-    A.sh_th = y.sh_th.p; A.sh_vx = y.sh_vx.p; A.sh_vy = y.sh_vy.p; A.sh_vz = y.sh_vz.p;
+    A.vmca = y.vmca.p; A.upv = reinterpret_cast<const float4*>(y.upv.p); A.upw = y.upw.p;
+    A.sh_th = lean ? y.thilt.p : y.sh_th.p; A.sh_vx = lean ? y.vmxet.p : y.sh_vx.p;
+    A.sh_vy = lean ? y.vmyet.p : y.sh_vy.p; A.sh_vz = lean ? y.vmzet.p : y.sh_vz.p;
     A.rk_vx = y.rk_vx.p; A.rk_vy = y.rk_vy.p; A.rk_vz = y.rk_vz.p;
     A.rho = tp.rho.p; A.press = y.press.p; A.rho0 = y.rho0.p; A.rth0 = y.rth0.p;
     A.thil = y.thil.p; A.wc = tp.wc.p; A.wmc = y.wmc.p; A.wmc0 = y.wmc0.p; A.vxe = y.vxe.p; A.vye = y.vye.p;
+    A.vze = y.vze.p;
     A.wmasc = tp.wmasc.p; A.alpha_press = y.alpha_press.p; A.pwfac = y.pwfac.p;
     A.volt = y.volt.p; A.volwi = y.volwi.p; A.arw = y.arw.p; A.wn = y.wn.p;
     A.gdz_wgtm8 = y.gdz_wgtm8.p; A.gdz_wgtp8 = y.gdz_wgtp8.p; A.gdz_wgtm = y.gdz_wgtm.p; A.gdz_wgtp = y.gdz_wgtp.p;
     A.zwgt_bot8 = y.zwgt_bot8.p; A.zwgt_top8 = y.zwgt_top8.p; A.b20 = y.b20.p;
-    const size_t smem = (size_t)WRT_WARPS * mza * 13 * sizeof(double);
-    // eight blocks of four column warps per SM: 64 registers a thread and
-    // the whole shared-memory carveout (8 x 25 KB at 61 levels; above 118
-    // levels a block needs more than the default 48 KB)
-    OG_CUDA(cudaFuncSetAttribute(k_wrt_begs, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    OG_CUDA(cudaFuncSetAttribute(k_wrt_begs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    { OG_PROF("wrt_begs", s); k_wrt_begs<<<cdiv(d.nw_prog, WRT_WARPS), WRT_WARPS * 32, smem, s>>>(g, A); OG_LAUNCHED(); }
+    {
+      OG_PROF("wrt_begs", s);
+      BY_ROWS(mza, {
+        constexpr int cols = WRT_COLS(R);
+        const size_t smem = (size_t)cols * ((R == 1 ? 224 : 128 * R) + 4 * mza) * sizeof(double);   // 11.2 KB or less
+        const unsigned nb = cdiv(d.nw_prog, cols);
+        if (lean) k_wrt_begs<R, true><<<nb, 32 * R * cols, smem, s>>>(g, A);
+        else k_wrt_begs<R, false><<<nb, 32 * R * cols, smem, s>>>(g, A);
+      });
+    }
     if (C.halo.on) {
       // prog_wrtv_rk.f90:418-429: what prog_v_begs reads at border V points
       OG_PROF("halo_exchange", s);
@@ -1250,9 +1587,7 @@ int dyn_prog_wrtv_rk(int istp) {
     }
     {
       OG_PROF("vel_t3d", s);
-      k_vel_t3d<<<nbw, 256, 0, s>>>(g, d.jtw_prog.p, d.nw_prog, tp.wc.p, y.vc.p, y.wno2.p, y.ecv.p, y.vxe.p,
-                                    y.vye.p, y.vze.p, shaved_args(y, tp, 1, dts));
-      OG_LAUNCHED();
+      launch_vel_t3d(C, shaved_args(y, tp, 1, dts), s);
     }
     if (C.halo.on) {   // prog_wrtv_rk.f90:464-472
       OG_PROF("halo_exchange", s);
@@ -1336,12 +1671,7 @@ int dyn_diagvel_t3d() {
   else if (!C.dy.uploaded) { OG_CHECK(dyn_state_to_device(DYN_IN_MASK, s)); C.dy.uploaded = true; }
   const DevGrid& d = C.g;
   Dyn& y = C.dy;
-  if (d.nw_prog > 0) {
-    k_vel_t3d<<<cdiv((size_t)d.nw_prog * d.mza, 256), 256, 0, s>>>(dynk(d), d.jtw_prog.p, d.nw_prog, C.tp.wc.p, y.vc.p,
-                                                                    y.wno2.p, y.ecv.p, y.vxe.p, y.vye.p, y.vze.p,
-                                                                    shaved_args(y, C.tp, 0, 0.f));
-    OG_LAUNCHED();
-  }
+  if (d.nw_prog > 0) launch_vel_t3d(C, shaved_args(y, C.tp, 0, 0.f), s);
   if (C.coherence == OLAMGPU_SYNC_EACH_CALL) {
     OG_CHECK(dyn_state_to_host(OLAMGPU_F_VXE, s));
     OG_CUDA(cudaStreamSynchronize(s));

@@ -53,7 +53,7 @@ struct MonoArgs {
   const float* __restrict__ vmca;   // vmc arv of this stage
   const float* __restrict__ wmc;
   float* __restrict__ upw;          // this field's W-face values
-  float* __restrict__ upv;          // this field's V-face values
+  float* __restrict__ upv;          // this field's V-face values (every fourth float)
   float* __restrict__ scpt;
   float* __restrict__ gx;           // gradient planes (5 x mwa x mza)
   float* __restrict__ hiw;          // high - low on W faces
@@ -149,7 +149,7 @@ __global__ void k_mono_v(const int* __restrict__ vadj, int nv, MonoArgs A) {
     }
   }
   const float h = (neg ? s2 : s1) - low;
-  A.upv[xv] = low;
+  A.upv[4 * xv] = low;
   A.hiv[xv] = h;
   A.sfv[xv] = A.vmca[xv] * h;
 }
@@ -176,7 +176,7 @@ __global__ void k_mono_lim(const int* __restrict__ prog, int nprog, MonoArgs A) 
     const float dv = A.w_dirv[iw * 8 + n];
     const size_t xv = (size_t)iv * mza + kd;
     const float vm = A.vmca[xv];
-    fl = fl + dv * vm * (A.upv[xv] - s);
+    fl = fl + dv * vm * (A.upv[4 * xv] - s);
     fi = fi + fmaxf(dv * A.sfv[xv], 0.f);
     fo = fo + fminf(dv * A.sfv[xv], 0.f);
     if (dv * vm > 0.f) {
@@ -220,7 +220,7 @@ __global__ void k_mono_apply_v(const int* __restrict__ vadj, int nv, MonoArgs A)
   const size_t x1 = (size_t)iw1 * mza + kd, x2 = (size_t)iw2 * mza + kd, xv = (size_t)iv * mza + kd;
   float sc = fminf(A.sin[x2], A.sout[x1]);
   if (A.sfv[xv] < 0.f) sc = fminf(A.sin[x1], A.sout[x2]);
-  A.upv[xv] = A.upv[xv] + A.hiv[xv] * sc;
+  A.upv[4 * xv] = A.upv[4 * xv] + A.hiv[xv] * sc;
 }
 
 int dyn_monot_faces(Context& C, int field, const float* scp, const float* scp0, const float* sct, float dts,
@@ -253,7 +253,7 @@ int dyn_monot_faces(Context& C, int field, const float* scp, const float* scp0, 
   A.scp = scp; A.scp0 = scp0; A.sct = sct; A.rho = C.tp.rho.p; A.rho0 = y.rho0.p; A.vmca = y.vmca.p;
   A.wmc = y.wmc.p;
   A.upw = y.upw.p + (size_t)field * wz;
-  A.upv = y.upv.p + (size_t)field * vz;
+  A.upv = y.upv.p + field;   // (mva, mza, 4)
   A.scpt = y.m_scpt.p; A.gx = y.m_gx.p; A.hiw = y.m_hiw.p; A.sfw = y.m_sfw.p; A.hiv = y.m_hiv.p;
   A.sfv = y.m_sfv.p; A.sin = y.m_sin.p; A.sout = y.m_sout.p;
   const unsigned nbw = cdiv((size_t)d.nw_prog * d.mza, 256), nbva = cdiv((size_t)d.nv_wadj * d.mza, 256);
