@@ -129,11 +129,12 @@ static int grow(DevBuf<float>& b, size_t n) { return b.n >= n ? OLAMGPU_OK : b.a
 
 // Tracers (padded) up to which a stage runs as passes over cells: the tiled
 // kernel gives 8 lanes or more to a column whatever the count, and needs the
-// step's weight records (128 B a cell).  Measured per stage at NXP=100, 60
-// levels, order 2 (tiles + half of the records against cells): 4 tracers 1.26
-// / 0.52 ms, 8: 1.26 / 0.99, 12: 1.27 / 1.43.
+// step's weight records (128 B a cell).  Measured per stage, tiles and half
+// the records against cells: NXP=100, 60 levels, order 2: 4 tracers 1.26 /
+// 0.36 ms, 8: 1.26 / 0.66, 12: 1.27 / 0.97, 16: 1.27 / 1.28; NXP=47, 41
+// levels, order 3: 8: 0.22 / 0.16 ms, 12: 0.23 / 0.21, 16: 0.23 / 0.29.
 #ifndef CELL_NTP_MAX
-#define CELL_NTP_MAX 8
+#define CELL_NTP_MAX 12
 #endif
 
 // scratch of the reference-mirroring passes for a group of nt tracers

@@ -26,6 +26,7 @@
 // written once and read by two cells: 44 B per tracer cell unlimited).
 //
 // Device level index kd = Fortran k - 1.
+#include <algorithm>
 #include <type_traits>
 
 #include "transport_kernels.cuh"
@@ -35,6 +36,7 @@ namespace olamgpu {
 struct CellArgs {
   int mza, mwa;
   int ncol, nq, nch;                // columns, tracer quads (V = 1: 1), item chunks per column
+  int off, flat;                    // cols is off, off + 1, ... (-1: not); every floor is level 1
   const int* __restrict__ cols;
   const int* __restrict__ npoly;
   const int* __restrict__ lpw;
@@ -89,17 +91,36 @@ __device__ __forceinline__ Vec<V> zerov() {
   for (int c = 0; c < V; ++c) r.v[c] = 0.f;
   return r;
 }
+// acc + w x, two tracers per instruction
+template <int V>
+__device__ __forceinline__ Vec<V> fmav(float w, const Vec<V>& x, const Vec<V>& acc) {
+  Vec<V> r;
+  if constexpr (V == 4) {
+    const float2 w2 = make_float2(w, w);
+    const float2 a = __ffma2_rn(w2, make_float2(x.v[0], x.v[1]), make_float2(acc.v[0], acc.v[1]));
+    const float2 b = __ffma2_rn(w2, make_float2(x.v[2], x.v[3]), make_float2(acc.v[2], acc.v[3]));
+    r.v[0] = a.x; r.v[1] = a.y; r.v[2] = b.x; r.v[3] = b.y;
+  } else {
+    r.v[0] = fmaf(w, x.v[0], acc.v[0]);
+  }
+  return r;
+}
+template <int V>
+__device__ __forceinline__ Vec<V> subv(const Vec<V>& x, const Vec<V>& y) { return fmav<V>(-1.f, y, x); }
 
-// a warp's chunk of 32 items of one column: item -> (level, quad)
+// a warp's chunk of 32 items of one column: item -> (level, quad).  OFF: the
+// type of element offsets, unsigned where every array has fewer than 2^32
+// elements (half the address instructions of size_t).
 #define CELL_ITEM(A)                                                                      \
   const unsigned warp_ = blockIdx.x * 8u + (threadIdx.x >> 5);                            \
   const unsigned j_ = warp_ / (unsigned)A.nch;                                            \
   if (j_ >= (unsigned)A.ncol) return;                                                     \
   const unsigned i_ = (warp_ - j_ * (unsigned)A.nch) * 32u + (threadIdx.x & 31u);         \
   const int kd = (int)(i_ / (unsigned)A.nq), q = (int)(i_ - (unsigned)kd * (unsigned)A.nq); \
-  const int iw = __ldg(A.cols + j_);                                                      \
+  const int iw = A.off >= 0 ? A.off + (int)j_ : __ldg(A.cols + j_);                       \
   const int mza = A.mza;                                                                  \
   if (kd >= mza) return;
+#define CELL_FLOOR(A) (A.flat ? 1 : __ldg(A.lpw + iw))
 
 // per-tracer modes of a quad; tracers past the count are PLAIN
 template <int V>
@@ -116,30 +137,33 @@ __device__ __forceinline__ void quad_modes(const CellArgs& A, int q, int (&m)[V]
 #define CELL_EDGES(np, body)                 \
   body(std::integral_constant<int, 6>(), 0); \
   if (np > 6) body(std::integral_constant<int, 1>(), 6);
+#define CELL_EDGES3(np, body)                \
+  body(std::integral_constant<int, 3>(), 0); \
+  body(std::integral_constant<int, 3>(), 3); \
+  if (np > 6) body(std::integral_constant<int, 1>(), 6);
 
 // LIM: the limited last stage -- the face array holds, for a limited tracer,
 // the high-order correction (value minus scp0 of the upwind cell)
-template <int V, int ORDER, bool LIM>
+template <int V, int ORDER, bool LIM, typename OFF>
 __global__ void __launch_bounds__(256) k_face(CellArgs A) {
   CELL_ITEM(A);
   constexpr int M = ORDER == 2 ? 2 : 5;
   const int np = __ldg(A.npoly + iw);
-  const size_t row = (size_t)A.ld;
+  const OFF row = (OFF)A.ld;
   const float* S = A.S + V * q;
-  const Vec<V> s0 = ldv<V>(S + ((size_t)iw * mza + kd) * row);
+  const OFF x0 = ((OFF)iw * mza + kd) * row;
+  const Vec<V> s0 = ldv<V>(S + x0);
   Vec<V> lo = zerov<V>();
   if (LIM) {
     int md[V];
     quad_modes<V>(A, q, md);
-    lo = ldv<V>(A.S0 + ((size_t)iw * mza + kd) * row + V * q);
+    lo = ldv<V>(A.S0 + x0 + V * q);
 #pragma unroll
     for (int c = 0; c < V; ++c) if (md[c] == MODE_PLAIN) lo.v[c] = 0.f;
   }
-  float g[M][V];
+  Vec<V> g[M];
 #pragma unroll
-  for (int m = 0; m < M; ++m)
-#pragma unroll
-    for (int c = 0; c < V; ++c) g[m][c] = 0.f;
+  for (int m = 0; m < M; ++m) g[m] = zerov<V>();
   const int4* E = A.edge + (size_t)iw * (7 * EDGE_W / 4);
   const float4* E3 = A.edge3 + (size_t)iw * (7 * EDGE3_W / 4);
   auto gradient = [&](auto cnt, int n0) {
@@ -150,8 +174,8 @@ __global__ void __launch_bounds__(256) k_face(CellArgs A) {
     for (int i = 0; i < N; ++i) e[i] = __ldg(E + 2 * (n0 + i));   // neighbour, face | side << 31, floor, dirv
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      x[i] = s0;
-      if (kd >= e[i].z) x[i] = ldv<V>(S + ((size_t)e[i].x * mza + kd) * row);
+      x[i] = s0;                                                  // a closed edge adds nothing
+      if (kd >= e[i].z) x[i] = ldv<V>(S + ((OFF)e[i].x * mza + kd) * row);
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -164,12 +188,9 @@ __global__ void __launch_bounds__(256) k_face(CellArgs A) {
         const float4 a = __ldg(E3 + 3 * (n0 + i)), b = __ldg(E3 + 3 * (n0 + i) + 1);
         w[0] = a.x; w[1] = a.y; w[M - 3] = a.z; w[M - 2] = a.w; w[M - 1] = b.x;
       }
+      const Vec<V> d = subv<V>(x[i], s0);
 #pragma unroll
-      for (int c = 0; c < V; ++c) {
-        const float d = kd >= e[i].z ? x[i].v[c] - s0.v[c] : 0.f;
-#pragma unroll
-        for (int m = 0; m < M; ++m) g[m][c] = g[m][c] + w[m] * d;
-      }
+      for (int m = 0; m < M; ++m) g[m] = fmav<V>(w[m], d, g[m]);
     }
   };
   CELL_EDGES(np, gradient);
@@ -181,7 +202,7 @@ __global__ void __launch_bounds__(256) k_face(CellArgs A) {
     for (int i = 0; i < N; ++i) e[i] = __ldg(E + 2 * (n0 + i));
 #pragma unroll
     for (int i = 0; i < N; ++i)
-      vm[i] = kd >= e[i].z ? __ldg(A.vmasc + (size_t)(e[i].y & 0x7fffffff) * mza + kd) : 0.f;
+      vm[i] = kd >= e[i].z ? __ldg(A.vmasc + ((OFF)(e[i].y & 0x7fffffff) * mza + kd)) : 0.f;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       if (kd < e[i].z || (vm[i] < 0.f) != (e[i].y < 0)) continue;  // closed, or the other cell is upwind
@@ -194,15 +215,11 @@ __global__ void __launch_bounds__(256) k_face(CellArgs A) {
         const float4 b = __ldg(E3 + 3 * (n0 + i) + 1), d = __ldg(E3 + 3 * (n0 + i) + 2);
         o[0] = b.y; o[1] = b.z; o[M - 3] = b.w; o[M - 2] = d.x; o[M - 1] = d.y;
       }
-      Vec<V> v;
+      Vec<V> v = s0;
 #pragma unroll
-      for (int c = 0; c < V; ++c) {
-        float x = s0.v[c];
-        x = x + o[0] * g[0][c] + o[1] * g[1][c];
-        if (ORDER == 3) x = x + o[M - 3] * g[M - 3][c] + o[M - 2] * g[M - 2][c] + o[M - 1] * g[M - 1][c];
-        v.v[c] = LIM ? x - lo.v[c] : x;
-      }
-      stv<V>(A.face + (((size_t)(e[i].y & 0x7fffffff) * mza + kd) * A.nq + q) * V, v);
+      for (int m = 0; m < M; ++m) v = fmav<V>(o[m], g[m], v);
+      if (LIM) v = subv<V>(v, lo);
+      stv<V>(A.face + (((OFF)(e[i].y & 0x7fffffff) * mza + kd) * A.nq + q) * V, v);
     }
   };
   CELL_EDGES(np, faces);
@@ -236,31 +253,49 @@ __device__ __forceinline__ float zvalue(const ZFace& z, float sm1, float s0, flo
   return c + dk * z.c1 + dkm1 * z.c2;
 }
 
-// a field's rows kd-M .. kd+M of the column, the end levels repeating
-template <int V, int M>
-__device__ __forceinline__ void window(const float* p, size_t row, int kd, int kb, int mza, Vec<V> (&w)[2 * M + 1]) {
+// a field's rows kd-M .. kd+M of the column, the end levels repeating; base:
+// the column's first element
+template <int V, int M, typename OFF>
+__device__ __forceinline__ void window(const float* p, OFF base, OFF row, int kd, int kb, int mza, Vec<V> (&w)[2 * M + 1]) {
 #pragma unroll
-  for (int m = 0; m < 2 * M + 1; ++m) w[m] = ldv<V>(p + (size_t)min(max(kd - M + m, kb), mza - 1) * row);
+  for (int m = 0; m < 2 * M + 1; ++m) w[m] = ldv<V>(p + (base + (OFF)min(max(kd - M + m, kb), mza - 1) * row));
+}
+
+// the vertical flux wm (lower face) - wp (upper face) of grad_z_quadratic's
+// values as coefficients on S(kd-2 .. kd+2); they add up to wm - wp
+__device__ __forceinline__ void zbeta(const float* a, int mza, int kd, int kb, float wm, float wp, float (&b)[5]) {
+  const ZFace l = zface(a, mza, kd - 1, kb, wm), u = zface(a, mza, kd, kb, wp);
+  // face value c + c1 (S(lev+1) - c) + c2 (c - S(lev-1)), c = S(lev)
+  const float l1 = l.has_up ? l.c1 : 0.f, l2 = l.has_dn ? l.c2 : 0.f, u1 = u.has_up ? u.c1 : 0.f, u2 = u.has_dn ? u.c2 : 0.f;
+  const float lm = -wm * l2, lc = wm * (1.f - l1 + l2), lp = wm * l1;
+  const float um = wp * u2, uc = -wp * (1.f - u1 + u2), up = -wp * u1;
+  const bool bot = kd == kb, top = kd == mza - 1;   // scp_upw(kb-1) = scp(kb), scp_upw(mza) = scp(mza)
+  b[0] = bot || l.down ? 0.f : lm;
+  b[1] = bot ? 0.f : (l.down ? lm : lc);
+  b[2] = bot ? wm : (l.down ? lc : lp);
+  b[3] = bot || !l.down ? 0.f : lp;
+  b[4] = 0.f;
+  b[1] += top || u.down ? 0.f : um;
+  b[2] += top ? -wp : (u.down ? um : uc);
+  b[3] += top ? 0.f : (u.down ? uc : up);
+  b[4] += top || !u.down ? 0.f : up;
 }
 
 // an unlimited stage (scalar_w_column)
-template <int V>
+template <int V, typename OFF>
 __global__ void __launch_bounds__(256) k_update(CellArgs A) {
   CELL_ITEM(A);
-  const int kb = __ldg(A.lpw + iw);
+  const int kb = CELL_FLOOR(A);
   if (kd < kb) return;                                // written by the thread of level kb
   const int np = __ldg(A.npoly + iw);
   const float fexpl = A.ff ? 1.0f - __ldg(A.ff + (size_t)iw * A.nrk + A.istage - 1) : 1.0f;
-  const size_t row = (size_t)A.ld, x = (size_t)iw * mza + kd;
-  const Vec<V> s00 = ldv<V>(A.S0 + x * row + V * q), tend = ldv<V>(A.SCT + x * row + V * q);
+  const OFF row = (OFF)A.ld, cb = (OFF)iw * mza, x = cb + kd;
+  const Vec<V> s00 = ldv<V>(A.S0 + V * q + x * row), tend = ldv<V>(A.SCT + V * q + x * row);
   Vec<V> w[5];
-  window<V, 2>(A.S + (size_t)iw * mza * row + V * q, row, kd, kb, mza, w);
+  window<V, 2, OFF>(A.S + V * q, cb * row, row, kd, kb, mza, w);
   const float wm = __ldg(A.wmasc + x - 1), wp = __ldg(A.wmasc + x);
   const float vt = __ldg(A.volti + x), rh = __ldg(A.rhos + x);
-  const ZFace zl = zface(A.a_w, mza, kd - 1, kb, wm), zu = zface(A.a_w, mza, kd, kb, wp);
-  float fd[V];
-#pragma unroll
-  for (int c = 0; c < V; ++c) fd[c] = 0.f;
+  Vec<V> fd = zerov<V>();
   const int4* E = A.edge + (size_t)iw * (7 * EDGE_W / 4);
   auto edges = [&](auto cnt, int n0) {
     constexpr int N = decltype(cnt)::value;
@@ -271,35 +306,25 @@ __global__ void __launch_bounds__(256) k_update(CellArgs A) {
     for (int i = 0; i < N; ++i) e[i] = __ldg(E + 2 * (n0 + i));
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      const size_t xv = (size_t)(e[i].y & 0x7fffffff) * mza + kd;
+      const OFF xv = (OFF)(e[i].y & 0x7fffffff) * mza + kd;
       vm[i] = 0.f;
       up[i] = s00;
       if (kd >= e[i].z) { vm[i] = __ldg(A.vmasc + xv); up[i] = ldv<V>(A.face + (xv * A.nq + q) * V); }
     }
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const float f = __int_as_float(e[i].w) * vm[i];
-#pragma unroll
-      for (int c = 0; c < V; ++c) {
-        const float d = kd >= e[i].z ? up[i].v[c] - s00.v[c] : 0.f;
-        fd[c] = fd[c] + f * d;
-      }
-    }
+    for (int i = 0; i < N; ++i) fd = fmav<V>(__int_as_float(e[i].w) * vm[i], subv<V>(up[i], s00), fd);
   };
   CELL_EDGES(np, edges);
-  Vec<V> o;
+  // differences from scp0: the coefficients add up to the S0 term's
+  float b[5];
+  zbeta(A.a_w, mza, kd, kb, wm, wp, b);
 #pragma unroll
-  for (int c = 0; c < V; ++c) {
-    // scp_upw(kb-1) = scp(kb), scp_upw(mza) = scp(mza)
-    const float lo = kd == kb ? w[2].v[c] : zvalue<false>(zl, w[0].v[c], w[1].v[c], w[2].v[c], w[3].v[c]);
-    const float up = kd == mza - 1 ? w[2].v[c] : zvalue<false>(zu, w[1].v[c], w[2].v[c], w[3].v[c], w[4].v[c]);
-    const float f = fd[c] + fexpl * (wm * (lo - s00.v[c]) - wp * (up - s00.v[c]));
-    o.v[c] = s00.v[c] + A.dtr * (tend.v[c] + vt * f) / rh;
-  }
-  float* out = A.out + (size_t)iw * mza * row + V * q;
-  stv<V>(out + (size_t)kd * row, o);
+  for (int m = 0; m < 5; ++m) fd = fmav<V>(fexpl * b[m], subv<V>(w[m], s00), fd);
+  const Vec<V> o = fmav<V>(A.dtr / rh, fmav<V>(vt, fd, tend), s00);
+  float* out = A.out + V * q;
+  stv<V>(out + x * row, o);
   if (kd == kb)
-    for (int k = 0; k < kb; ++k) stv<V>(out + (size_t)k * row, o);
+    for (int k = 0; k < kb; ++k) stv<V>(out + (cb + k) * row, o);
 }
 
 // the vertical faces of a limited cell: low-order values and high-order
@@ -318,18 +343,18 @@ __device__ __forceinline__ void lim_faces(int mza, int kd, int kb, const ZFace& 
 
 // scale factors of the limited stage: plane 0 the inflow (monotonic) or
 // outflow (positive-definite) factor, plane 1 the monotonic outflow factor
-template <int V, bool MONOT>
+template <int V, bool MONOT, typename OFF>
 __global__ void __launch_bounds__(256) k_scale(CellArgs A) {
   CELL_ITEM(A);
-  const int kb = __ldg(A.lpw + iw);
+  const int kb = CELL_FLOOR(A);
   if (kd < kb) return;
   const int np = __ldg(A.npoly + iw);
   const float fimpl = __ldg(A.ff + (size_t)iw * A.nrk + A.istage - 1), fexpl = 1.0f - fimpl;
-  const size_t row = (size_t)A.ld, x = (size_t)iw * mza + kd;
+  const OFF row = (OFF)A.ld, cb = (OFF)iw * mza, x = cb + kd;
   const float* S0 = A.S0 + V * q;
   Vec<V> w[5], z[3];
-  window<V, 2>(A.S + (size_t)iw * mza * row + V * q, row, kd, kb, mza, w);
-  window<V, 1>(S0 + (size_t)iw * mza * row, row, kd, kb, mza, z);
+  window<V, 2, OFF>(A.S + V * q, cb * row, row, kd, kb, mza, w);
+  window<V, 1, OFF>(S0, cb * row, row, kd, kb, mza, z);
   const float wm = __ldg(A.wmasc + x - 1), wp = __ldg(A.wmasc + x);
   const float rh = __ldg(A.rhos + x), vt = __ldg(A.volti + x);
   const ZFace zl = zface(A.a_w, mza, kd - 1, kb, wm), zu = zface(A.a_w, mza, kd, kb, wp);
@@ -353,14 +378,14 @@ __global__ void __launch_bounds__(256) k_scale(CellArgs A) {
     for (int i = 0; i < N; ++i) e[i] = __ldg(E + 2 * (n0 + i));
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      const size_t xv = (size_t)(e[i].y & 0x7fffffff) * mza + kd;
+      const OFF xv = (OFF)(e[i].y & 0x7fffffff) * mza + kd;
       vm[i] = 0.f;
       hv[i] = zerov<V>();
       sn[i] = z[1];
       if (kd >= e[i].z) {
         vm[i] = __ldg(A.vmasc + xv);
         hv[i] = ldv<V>(A.face + (xv * A.nq + q) * V);
-        sn[i] = ldv<V>(S0 + ((size_t)e[i].x * mza + kd) * row);
+        sn[i] = ldv<V>(S0 + ((OFF)e[i].x * mza + kd) * row);
       }
     }
 #pragma unroll
@@ -431,18 +456,18 @@ __global__ void __launch_bounds__(256) k_scale(CellArgs A) {
 // the update of the limited stage: the scaled faces and the tendency.  PLAIN
 // tracers of the group (without pdef under the positive-definite option)
 // take the unlimited update.
-template <int V, bool MONOT>
+template <int V, bool MONOT, typename OFF>
 __global__ void __launch_bounds__(256) k_update_lim(CellArgs A) {
   CELL_ITEM(A);
-  const int kb = __ldg(A.lpw + iw);
+  const int kb = CELL_FLOOR(A);
   if (kd < kb) return;
   const int np = __ldg(A.npoly + iw);
   const float fimpl = __ldg(A.ff + (size_t)iw * A.nrk + A.istage - 1), fexpl = 1.0f - fimpl;
-  const size_t row = (size_t)A.ld, x = (size_t)iw * mza + kd;
+  const OFF row = (OFF)A.ld, cb = (OFF)iw * mza, x = cb + kd;
   const size_t plane = (size_t)A.mwa * mza * A.nq * V;
   const float* S0 = A.S0 + V * q;
   const float* sc = A.scale + (size_t)V * q;
-  const size_t srow = (size_t)A.nq * V;
+  const OFF srow = (OFF)A.nq * V;
   int md[V];
   bool plain = false;
   if (MONOT) {
@@ -454,10 +479,10 @@ __global__ void __launch_bounds__(256) k_update_lim(CellArgs A) {
     for (int c = 0; c < V; ++c) plain |= md[c] == MODE_PLAIN;
   }
   Vec<V> w[5], z[3], a[3], b[3];
-  window<V, 2>(A.S + (size_t)iw * mza * row + V * q, row, kd, kb, mza, w);
-  window<V, 1>(S0 + (size_t)iw * mza * row, row, kd, kb, mza, z);
-  window<V, 1>(sc + (size_t)iw * mza * srow, srow, kd, kb, mza, a);
-  if (MONOT) window<V, 1>(sc + plane + (size_t)iw * mza * srow, srow, kd, kb, mza, b);
+  window<V, 2, OFF>(A.S + V * q, cb * row, row, kd, kb, mza, w);
+  window<V, 1, OFF>(S0, cb * row, row, kd, kb, mza, z);
+  window<V, 1, OFF>(sc, cb * srow, srow, kd, kb, mza, a);
+  if (MONOT) window<V, 1, OFF>(sc + plane, cb * srow, srow, kd, kb, mza, b);
   const float wm = __ldg(A.wmasc + x - 1), wp = __ldg(A.wmasc + x);
   const float vt = __ldg(A.volti + x), rh = __ldg(A.rhos + x);
   const ZFace zl = zface(A.a_w, mza, kd - 1, kb, wm), zu = zface(A.a_w, mza, kd, kb, wp);
@@ -465,51 +490,50 @@ __global__ void __launch_bounds__(256) k_update_lim(CellArgs A) {
 #pragma unroll
   for (int c = 0; c < V; ++c) fd[c] = 0.f;
   const int4* E = A.edge + (size_t)iw * (7 * EDGE_W / 4);
-  auto edges = [&](auto cnt, int n0) {
+  auto edges = [&](auto cnt, int n0) {   // three at a time: four or five quads each
     constexpr int N = decltype(cnt)::value;
+    int4 e[N];
+    float vm[N];
+    Vec<V> hv[N], sn[N], an[N], bn[N];
 #pragma unroll
-    for (int h = 0; h < N; h += 3) {                   // three edges in flight: four values each
-      constexpr int H = N < 3 ? N : 3;
-      int4 e[H];
-      float vm[H];
-      Vec<V> hv[H], sn[H], an[H], bn[H];
+    for (int i = 0; i < N; ++i) e[i] = __ldg(E + 2 * (n0 + i));
 #pragma unroll
-      for (int i = 0; i < H; ++i) e[i] = __ldg(E + 2 * (n0 + h + i));
-#pragma unroll
-      for (int i = 0; i < H; ++i) {
-        const size_t xv = (size_t)(e[i].y & 0x7fffffff) * mza + kd, xn = (size_t)e[i].x * mza + kd;
-        vm[i] = 0.f;
-        hv[i] = an[i] = bn[i] = zerov<V>();
-        sn[i] = z[1];
-        if (kd >= e[i].z) {
-          vm[i] = __ldg(A.vmasc + xv);
-          hv[i] = ldv<V>(A.face + (xv * A.nq + q) * V);
-          sn[i] = ldv<V>(S0 + xn * row);
-          an[i] = ldv<V>(sc + xn * srow);
-          if (MONOT) bn[i] = ldv<V>(sc + plane + xn * srow);
-        }
+    for (int i = 0; i < N; ++i) {
+      const OFF xv = (OFF)(e[i].y & 0x7fffffff) * mza + kd, xn = (OFF)e[i].x * mza + kd;
+      vm[i] = 0.f;
+      hv[i] = an[i] = bn[i] = zerov<V>();
+      sn[i] = z[1];
+      if (kd >= e[i].z) {
+        vm[i] = __ldg(A.vmasc + xv);
+        hv[i] = ldv<V>(A.face + (xv * A.nq + q) * V);
+        sn[i] = ldv<V>(S0 + xn * row);
+        an[i] = ldv<V>(sc + xn * srow);
+        if (MONOT) bn[i] = ldv<V>(sc + plane + xn * srow);
       }
+    }
 #pragma unroll
-      for (int i = 0; i < H; ++i) {
-        const float f = __int_as_float(e[i].w) * vm[i];
-        const bool second = e[i].y < 0;                // this cell is side 2 of the face
-        const bool far = (vm[i] < 0.f) != second;
+    for (int i = 0; i < N; ++i) {
+      const bool open = kd >= e[i].z;
+      const float f = __int_as_float(e[i].w) * vm[i];
+      const bool second = e[i].y < 0;                  // this cell is side 2 of the face
+      const bool far = (vm[i] < 0.f) != second;
 #pragma unroll
-        for (int c = 0; c < V; ++c) {
-          // the correction runs from side 1 to side 2, or back where it is negative
-          const bool back = vm[i] * hv[i].v[c] < 0.f;
-          const bool from_here = back == second;       // this cell gives the corrected flux
-          const float s = MONOT ? (from_here ? fminf(an[i].v[c], b[1].v[c]) : fminf(a[1].v[c], bn[i].v[c]))
-                                : (from_here ? a[1].v[c] : an[i].v[c]);
-          const float lo = far ? sn[i].v[c] : z[1].v[c];
-          const float up = md[c] == MODE_PLAIN ? hv[i].v[c] : lo + hv[i].v[c] * s;
-          fd[c] = fd[c] + (kd >= e[i].z ? f * (up - z[1].v[c]) : 0.f);
-        }
+      for (int c = 0; c < V; ++c) {
+        // the correction runs from side 1 to side 2, or back where it is negative
+        const bool back = vm[i] * hv[i].v[c] < 0.f;
+        const bool from_here = back == second;         // this cell gives the corrected flux
+        const float s = MONOT ? (from_here ? fminf(an[i].v[c], b[1].v[c]) : fminf(a[1].v[c], bn[i].v[c]))
+                              : (from_here ? a[1].v[c] : an[i].v[c]);
+        // low-order value minus scp0, 0 where this cell is upwind
+        const float lo = far ? sn[i].v[c] : z[1].v[c];
+        const float up = md[c] == MODE_PLAIN ? hv[i].v[c] : lo + hv[i].v[c] * s;
+        if (open) fd[c] = fd[c] + f * (up - z[1].v[c]);
       }
     }
   };
-  CELL_EDGES(np, edges);
+  CELL_EDGES3(np, edges);
   Vec<V> o, tend = zerov<V>();
+  const float dr = A.dtr / rh;
   if (plain) tend = ldv<V>(A.SCT + x * row + V * q);
 #pragma unroll
   for (int c = 0; c < V; ++c) {
@@ -520,7 +544,7 @@ __global__ void __launch_bounds__(256) k_update_lim(CellArgs A) {
       const float ul = kd == kb ? s[2] : zvalue<false>(zl, s[0], s[1], s[2], s[3]);
       const float uu = kd == mza - 1 ? s[2] : zvalue<false>(zu, s[1], s[2], s[3], s[4]);
       const float f = fd[c] + fexpl * (wm * (ul - s00) - wp * (uu - s00));
-      o.v[c] = s00 + A.dtr * (tend.v[c] + vt * f) / rh;
+      o.v[c] = s00 + dr * (tend.v[c] + vt * f);
       continue;
     }
     float lo[2], hi[2];
@@ -539,20 +563,20 @@ __global__ void __launch_bounds__(256) k_update_lim(CellArgs A) {
     float f = fd[c];
     if (fimpl > .001f) f = f + fexpl * (wm * (ul - s00) - wp * (uu - s00));
     else f = f + wm * (ul - s00) - wp * (uu - s00);
-    o.v[c] = s00 + A.dtr * vt * f / rh;
+    o.v[c] = s00 + dr * vt * f;
   }
-  float* out = A.out + (size_t)iw * mza * row + V * q;
-  stv<V>(out + (size_t)kd * row, o);
+  float* out = A.out + V * q;
+  stv<V>(out + x * row, o);
   // Below the floor the reference updates in place: scp(2:kb-1) = scp(kb) in
   // the explicit branch only (an unlimited tracer: scp(1:kb-1)), and levels
   // it does not write keep the stage input.
   if (kd == kb)
     for (int k = 0; k < kb; ++k) {
-      Vec<V> y = ldv<V>(A.S + ((size_t)iw * mza + k) * row + V * q);
+      Vec<V> y = ldv<V>(A.S + V * q + (cb + k) * row);
 #pragma unroll
       for (int c = 0; c < V; ++c)
         if (md[c] == MODE_PLAIN || (!(fimpl > .001f) && k >= 1)) y.v[c] = o.v[c];
-      stv<V>(out + (size_t)k * row, y);
+      stv<V>(out + (cb + k) * row, y);
     }
 }
 
@@ -560,7 +584,7 @@ __global__ void __launch_bounds__(256) k_update_lim(CellArgs A) {
 // (scalar_transport_rk.F90:297-314), in place
 __global__ void __launch_bounds__(256) k_preupdate(CellArgs A, float* __restrict__ S0, const float* __restrict__ rho_old) {
   CELL_ITEM(A);
-  const int kb = __ldg(A.lpw + iw);
+  const int kb = CELL_FLOOR(A);
   if (kd < kb) return;
   constexpr int V = 4;
   const size_t row = (size_t)A.ld;
@@ -594,17 +618,18 @@ static CellArgs cell_args(const DevGrid& d, int nq, int V) {
   A.edge = reinterpret_cast<const int4*>(d.edge.p);
   A.volti = d.volti.p;
   A.ld = nq * V;
+  A.flat = ctx().tp.flat ? 1 : 0;
   return A;
 }
 
-static void over(CellArgs& A, const DevBuf<int>& cols, int n) { A.cols = cols.p; A.ncol = n; }
+static void over(CellArgs& A, const DevBuf<int>& cols, int n, int off) { A.cols = cols.p; A.ncol = n; A.off = off; }
 static unsigned cell_blocks(const CellArgs& A) { return cdiv((size_t)A.ncol * A.nch, 8); }
 
 bool cell_stage_available(const DevGrid& d, int order) {
   return d.edge.p && (order == 2 || (order == 3 && d.edge3_b.p));
 }
 
-template <int V>
+template <int V, typename OFF>
 static int run_stage(const DevGrid& d, int order, const CellStage& c, cudaStream_t s) {
   const int nq = V == 1 ? 1 : (c.nt + 3) / 4;
   CellArgs A = cell_args(d, nq, V);
@@ -616,16 +641,16 @@ static int run_stage(const DevGrid& d, int order, const CellStage& c, cudaStream
   A.a_w = monot ? d.a_wu.p : d.a_w.p;
   A.edge3 = reinterpret_cast<const float4*>(monot ? d.edge3_u.p : d.edge3_b.p);
   // every face's upwind cell is in jtw_wadj
-  over(A, d.jtw_wadj, d.nw_wadj);
+  over(A, d.jtw_wadj, d.nw_wadj, d.off_wwadj);
   {
     OG_PROF(lim ? "lim_face" : "cell_face", s);
     const unsigned nb = cell_blocks(A);
     if (!lim) {
-      if (order == 2) k_face<V, 2, false><<<nb, 256, 0, s>>>(A);
-      else k_face<V, 3, false><<<nb, 256, 0, s>>>(A);
+      if (order == 2) k_face<V, 2, false, OFF><<<nb, 256, 0, s>>>(A);
+      else k_face<V, 3, false, OFF><<<nb, 256, 0, s>>>(A);
     } else if constexpr (V == 4) {
-      if (order == 2) k_face<V, 2, true><<<nb, 256, 0, s>>>(A);
-      else k_face<V, 3, true><<<nb, 256, 0, s>>>(A);
+      if (order == 2) k_face<V, 2, true, OFF><<<nb, 256, 0, s>>>(A);
+      else k_face<V, 3, true, OFF><<<nb, 256, 0, s>>>(A);
     }
     OG_LAUNCHED();
   }
@@ -634,19 +659,19 @@ static int run_stage(const DevGrid& d, int order, const CellStage& c, cudaStream
       // the factors of both cells of every face of a prognosed column
       OG_PROF("lim_scale", s);
       const unsigned nb = cell_blocks(A);
-      if (monot) k_scale<V, true><<<nb, 256, 0, s>>>(A);
-      else k_scale<V, false><<<nb, 256, 0, s>>>(A);
+      if (monot) k_scale<V, true, OFF><<<nb, 256, 0, s>>>(A);
+      else k_scale<V, false, OFF><<<nb, 256, 0, s>>>(A);
       OG_LAUNCHED();
     }
   }
-  over(A, d.jtw_prog, d.nw_prog);
+  over(A, d.jtw_prog, d.nw_prog, d.off_wprog);
   {
     OG_PROF(lim ? "lim_update" : "cell_update", s);
     const unsigned nb = cell_blocks(A);
-    if (!lim) k_update<V><<<nb, 256, 0, s>>>(A);
+    if (!lim) k_update<V, OFF><<<nb, 256, 0, s>>>(A);
     else if constexpr (V == 4) {
-      if (monot) k_update_lim<V, true><<<nb, 256, 0, s>>>(A);
-      else k_update_lim<V, false><<<nb, 256, 0, s>>>(A);
+      if (monot) k_update_lim<V, true, OFF><<<nb, 256, 0, s>>>(A);
+      else k_update_lim<V, false, OFF><<<nb, 256, 0, s>>>(A);
     }
     OG_LAUNCHED();
   }
@@ -657,7 +682,9 @@ static int run_stage(const DevGrid& d, int order, const CellStage& c, cudaStream
 int launch_cell_stage(const DevGrid& d, int order, const CellStage& c, cudaStream_t s) {
   if (d.nw_prog <= 0 || c.nt <= 0) return OLAMGPU_OK;
   if (c.ld == 1 && c.limited) { set_error("cell stage: limited stages run the batched layout"); return OLAMGPU_E_UNSUPPORTED; }
-  return c.ld == 1 ? run_stage<1>(d, order, c, s) : run_stage<4>(d, order, c, s);
+  if (c.ld == 1) return run_stage<1, unsigned>(d, order, c, s);   // one plane: under 2^32 elements
+  const double most = (double)d.mza * std::max((double)d.mwa * std::max(c.ld, 2 * cell_width(c.nt)), (double)d.mva * cell_width(c.nt));
+  return most < 4294967296.0 ? run_stage<4, unsigned>(d, order, c, s) : run_stage<4, size_t>(d, order, c, s);
 }
 
 void launch_cell_preupdate(const DevGrid& d, const Transport& tp, float* S0, const float* SCT, int ld, int nt,
@@ -665,7 +692,7 @@ void launch_cell_preupdate(const DevGrid& d, const Transport& tp, float* S0, con
   if (d.nw_wadj <= 0 || nt <= 0) return;
   CellArgs A = cell_args(d, (nt + 3) / 4, 4);
   A.ld = ld; A.nt = nt; A.mode = mode; A.SCT = SCT; A.dtr = dtr;
-  over(A, d.jtw_wadj, d.nw_wadj);
+  over(A, d.jtw_wadj, d.nw_wadj, d.off_wwadj);
   OG_PROF("lim_preupdate", s);
   k_preupdate<<<cell_blocks(A), 256, 0, s>>>(A, S0, tp.rho_old.p);
   OG_LAUNCHED();

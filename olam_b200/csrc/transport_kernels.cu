@@ -57,6 +57,7 @@ struct PrepArgs {
   GridK g;
   const int4* edge;                // edge records (EDGE_W words)
   const int* prog; int nprog;
+  int off, flat;                   // prog is off, off + 1, ... (-1: not); every floor is level 1
   const float* vmasc; const float* wmasc; const float* rho_old; const float* wc;
   const double* rho;
   int nrk; float dt; Dtlr dtlr;
@@ -86,12 +87,15 @@ __global__ void __launch_bounds__(256) k_prepare(PrepArgs A) {
   const int mza = g.mza, nrk = A.nrk;
   unsigned long long kc = 0, kh = 0, kw = 0, nc = 0, nh = 0, nwn = 0;
   if (j < A.nprog) {
-    const int iw = A.prog[j], np = g.npoly[iw], kb = g.lpw[iw];
+    const int iw = A.off >= 0 ? A.off + j : A.prog[j], np = g.npoly[iw], kb = A.flat ? 1 : g.lpw[iw];
     const size_t cb = (size_t)iw * mza, plane = (size_t)g.mwa * mza;
     int4 e[7];
 #pragma unroll
     for (int n = 0; n < 7; ++n) e[n] = __ldg(A.edge + ((size_t)iw * 7 + n) * (EDGE_W / 4));
     float fimp[3] = {0.f, 0.f, 0.f};
+    // the lane's largest values and where it met them first
+    float mc = 0.f, mh = 0.f, mw = 0.f;
+    unsigned int oc = 0, oh = 0, ow = 0;
     for (int kd = kb + lane; kd < mza; kd += 32) {
       float vm[7];
 #pragma unroll
@@ -111,19 +115,20 @@ __global__ void __launch_bounds__(256) k_prepare(PrepArgs A) {
       float cflw = (fmaxf(wp, 0.f) - fminf(wm, 0.f)) * dovr;
       const float cfl = cflh + cflw;
       cflw = fmaxf(cflw, .1f);
-      fimp[nrk - 1] = fmaxf(fimp[nrk - 1], (cfl - 0.98f) / cflw);
-      fimp[nrk - 2] = fmaxf(fimp[nrk - 2], (cfl - 1.98f) / cflw);
-      if (nrk == 3) fimp[0] = fmaxf(fimp[0], (cfl - 2.98f) / cflw);
+      if (cfl > 0.98f) {   // below it every fraction is negative, and 0 the least
+        fimp[nrk - 1] = fmaxf(fimp[nrk - 1], (cfl - 0.98f) / cflw);
+        fimp[nrk - 2] = fmaxf(fimp[nrk - 2], (cfl - 1.98f) / cflw);
+        if (nrk == 3) fimp[0] = fmaxf(fimp[0], (cfl - 2.98f) / cflw);
+      }
       const unsigned int order = (unsigned int)j * (unsigned int)mza + (unsigned int)kd;
-      const unsigned long long low = 0xffffffffull - order;
-      if (cfl != cfl) nc = max(nc, order + 1ull);
-      else if (cfl > 0.f) kc = max(kc, ((unsigned long long)__float_as_uint(cfl) << 32) | low);
-      if (cflh != cflh) nh = max(nh, order + 1ull);
-      else if (cflh > 0.f) kh = max(kh, ((unsigned long long)__float_as_uint(cflh) << 32) | low);
+      if (cfl != cfl) nc = order + 1ull;
+      else if (cfl > mc) { mc = cfl; oc = order; }
+      if (cflh != cflh) nh = order + 1ull;
+      else if (cflh > mh) { mh = cflh; oh = order; }
       if (A.wc) {
-        const float w = __ldg(A.wc + cb + kd);
-        if (w != w) nwn = max(nwn, order + 1ull);
-        else if (fabsf(w) > 0.f) kw = max(kw, ((unsigned long long)__float_as_uint(fabsf(w)) << 32) | low);
+        const float w = fabsf(__ldg(A.wc + cb + kd));
+        if (w != w) nwn = order + 1ull;
+        else if (w > mw) { mw = w; ow = order; }
       }
       float* r = A.rhos + cb + kd;
       if (nrk == 3) {
@@ -135,6 +140,12 @@ __global__ void __launch_bounds__(256) k_prepare(PrepArgs A) {
         r[plane] = rhof;
       }
     }
+    auto key = [](float v, unsigned int o) {
+      return v > 0.f ? ((unsigned long long)__float_as_uint(v) << 32) | (0xffffffffull - o) : 0ull;
+    };
+    kc = key(mc, oc);
+    kh = key(mh, oh);
+    kw = key(mw, ow);
 #pragma unroll
     for (int n = 0; n < 3; ++n)
 #pragma unroll
@@ -181,9 +192,14 @@ __global__ void __launch_bounds__(256) k_prepare(PrepArgs A) {
         }
       }
     }
-    kc = warp_max_u64(kc); nc = warp_max_u64(nc);
-    kh = warp_max_u64(kh); nh = warp_max_u64(nh);
-    kw = warp_max_u64(kw); nwn = warp_max_u64(nwn);
+    kc = warp_max_u64(kc);
+    kh = warp_max_u64(kh);
+    kw = warp_max_u64(kw);
+    if (__any_sync(0xffffffffu, (nc | nh | nwn) != 0)) {
+      nc = warp_max_u64(nc);
+      nh = warp_max_u64(nh);
+      nwn = warp_max_u64(nwn);
+    }
   }
   if (lane == 0) {
     part[0][warp] = kc; part[1][warp] = nc; part[2][warp] = kh;
@@ -207,6 +223,7 @@ void launch_prepare(const DevGrid& d, Transport& tp, int nrk, float dtl, const f
   A.g = gridk(d);
   A.edge = reinterpret_cast<const int4*>(d.edge.p);
   A.prog = d.jtw_prog.p; A.nprog = d.nw_prog;
+  A.off = d.off_wprog; A.flat = tp.flat ? 1 : 0;
   A.vmasc = tp.vmasc.p; A.wmasc = tp.wmasc.p; A.rho_old = tp.rho_old.p; A.wc = tp.wc.p; A.rho = tp.rho.p;
   A.nrk = nrk; A.dt = dtl;
   A.dtlr = Dtlr{{dtlr[0], dtlr[1], nrk > 2 ? dtlr[2] : 0.f}};
