@@ -597,6 +597,9 @@ struct WrtArgs {
   const double* zwgt_bot8; const double* zwgt_top8; const float* b20;
 };
 
+// warps per SM the column kernel is compiled for: 72 registers (at NXP=100, 60
+// levels 320 us; 24 warps and 80 registers 363, 32 warps and 64 registers 349)
+#define WRT_OCC 28
 // columns per block: four one-warp columns, else one
 #define WRT_COLS(NW) ((NW) == 1 ? 4 : 1)
 
@@ -715,7 +718,7 @@ __device__ __forceinline__ void column_solve<4>(double* P, int n, int i, double 
 // prog_wrtv_rk.f90:1085-1126) are formed from the column's own rows, so that
 // the set-up pass and the W-face pass are not run.
 template <int NW, bool LEAN>
-__global__ void __launch_bounds__(32 * NW * WRT_COLS(NW), 24 / (NW * WRT_COLS(NW))) k_wrt_begs(DynK g, WrtArgs A) {
+__global__ void __launch_bounds__(32 * NW * WRT_COLS(NW), WRT_OCC / (NW * WRT_COLS(NW))) k_wrt_begs(DynK g, WrtArgs A) {
   extern __shared__ double wsm[];
   constexpr int LANES = 32 * NW;
   const int grp = threadIdx.x / LANES, i = threadIdx.x - grp * LANES;   // the column of the block, the lane of the column

@@ -132,10 +132,8 @@ static int grow(DevBuf<float>& b, size_t n) { return b.n >= n ? OLAMGPU_OK : b.a
 // step's weight records (128 B a cell).  Measured per stage, tiles and half
 // the records against cells: NXP=100, 60 levels, order 2: 4 tracers 1.26 /
 // 0.36 ms, 8: 1.26 / 0.66, 12: 1.27 / 0.97, 16: 1.27 / 1.28; NXP=47, 41
-// levels, order 3: 8: 0.22 / 0.16 ms, 12: 0.23 / 0.21, 16: 0.23 / 0.29.
-#ifndef CELL_NTP_MAX
-#define CELL_NTP_MAX 12
-#endif
+// levels, order 3: 8: 0.22 / 0.16 ms, 12: 0.21 / 0.21, 16: 0.23 / 0.29.
+static int cell_ntp_max(int order) { return order == 2 ? 12 : 8; }
 
 // scratch of the reference-mirroring passes for a group of nt tracers
 static int ensure_pass_scratch(Context& C, int nt, int order) {
@@ -375,7 +373,7 @@ int transport_run(const float* rho_old_host, olamgpu_cfl_diag* diag) {
     return OLAMGPU_E_UNSUPPORTED;
   }
   // few tracers in the tiled form run as passes over cells
-  bool cells = tiled && tr.ntp <= CELL_NTP_MAX && tp.autotune && !C.halo.on && cell_stage_available(d, order);
+  bool cells = tiled && tr.ntp <= cell_ntp_max(order) && tp.autotune && !C.halo.on && cell_stage_available(d, order);
   if (batched && !tiled && d.ew_order != order)
     OG_CHECK(build_fused_weights(&C.hgrid, C.g, order, s));
 

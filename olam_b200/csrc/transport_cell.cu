@@ -137,6 +137,11 @@ __device__ __forceinline__ void quad_modes(const CellArgs& A, int q, int (&m)[V]
 #define CELL_EDGES(np, body)                 \
   body(std::integral_constant<int, 6>(), 0); \
   if (np > 6) body(std::integral_constant<int, 1>(), 6);
+#define CELL_EDGES2(np, body)                \
+  body(std::integral_constant<int, 2>(), 0); \
+  body(std::integral_constant<int, 2>(), 2); \
+  body(std::integral_constant<int, 2>(), 4); \
+  if (np > 6) body(std::integral_constant<int, 1>(), 6);
 #define CELL_EDGES3(np, body)                \
   body(std::integral_constant<int, 3>(), 0); \
   body(std::integral_constant<int, 3>(), 3); \
@@ -145,7 +150,7 @@ __device__ __forceinline__ void quad_modes(const CellArgs& A, int q, int (&m)[V]
 // LIM: the limited last stage -- the face array holds, for a limited tracer,
 // the high-order correction (value minus scp0 of the upwind cell)
 template <int V, int ORDER, bool LIM, typename OFF>
-__global__ void __launch_bounds__(256) k_face(CellArgs A) {
+__global__ void __launch_bounds__(256, ORDER == 2 ? 4 : 3) k_face(CellArgs A) {
   CELL_ITEM(A);
   constexpr int M = ORDER == 2 ? 2 : 5;
   const int np = __ldg(A.npoly + iw);
@@ -193,7 +198,8 @@ __global__ void __launch_bounds__(256) k_face(CellArgs A) {
       for (int m = 0; m < M; ++m) g[m] = fmav<V>(w[m], d, g[m]);
     }
   };
-  CELL_EDGES(np, gradient);
+  if constexpr (ORDER == 2) { CELL_EDGES(np, gradient); }
+  else { CELL_EDGES3(np, gradient); }
   auto faces = [&](auto cnt, int n0) {
     constexpr int N = decltype(cnt)::value;
     int4 e[N];
@@ -342,30 +348,46 @@ __device__ __forceinline__ void lim_faces(int mza, int kd, int kb, const ZFace& 
 }
 
 // scale factors of the limited stage: plane 0 the inflow (monotonic) or
-// outflow (positive-definite) factor, plane 1 the monotonic outflow factor
+// outflow (positive-definite) factor, plane 1 the monotonic outflow factor.
+// The vertical faces come first, so that their nine rows are spent before the
+// edges' values are loaded (80 registers, 24 warps an SM, against 128-163).
 template <int V, bool MONOT, typename OFF>
-__global__ void __launch_bounds__(256) k_scale(CellArgs A) {
+__global__ void __launch_bounds__(256, 3) k_scale(CellArgs A) {
   CELL_ITEM(A);
   const int kb = CELL_FLOOR(A);
   if (kd < kb) return;
   const int np = __ldg(A.npoly + iw);
   const float fimpl = __ldg(A.ff + (size_t)iw * A.nrk + A.istage - 1), fexpl = 1.0f - fimpl;
+  const bool impl = fimpl > .001f;
   const OFF row = (OFF)A.ld, cb = (OFF)iw * mza, x = cb + kd;
   const float* S0 = A.S0 + V * q;
-  Vec<V> w[5], z[3];
-  window<V, 2, OFF>(A.S + V * q, cb * row, row, kd, kb, mza, w);
-  window<V, 1, OFF>(S0, cb * row, row, kd, kb, mza, z);
   const float wm = __ldg(A.wmasc + x - 1), wp = __ldg(A.wmasc + x);
   const float rh = __ldg(A.rhos + x), vt = __ldg(A.volti + x);
-  const ZFace zl = zface(A.a_w, mza, kd - 1, kb, wm), zu = zface(A.a_w, mza, kd, kb, wp);
   float fl[V], fin[V], fout[V], smax[V], smin[V];
+  Vec<V> s00;
+  {
+    Vec<V> w[5], z[3];
+    window<V, 2, OFF>(A.S + V * q, cb * row, row, kd, kb, mza, w);
+    window<V, 1, OFF>(S0, cb * row, row, kd, kb, mza, z);
+    const ZFace zl = zface(A.a_w, mza, kd - 1, kb, wm), zu = zface(A.a_w, mza, kd, kb, wp);
+    s00 = z[1];
 #pragma unroll
-  for (int c = 0; c < V; ++c) {
-    fl[c] = fin[c] = fout[c] = 0.f;
-    smax[c] = smin[c] = z[1].v[c];
-    if (MONOT) {
-      if (kd >= kb + 1 && wm > 0.f) { smax[c] = fmaxf(smax[c], z[0].v[c]); smin[c] = fminf(smin[c], z[0].v[c]); }
-      if (kd <= mza - 2 && wp < 0.f) { smax[c] = fmaxf(smax[c], z[2].v[c]); smin[c] = fminf(smin[c], z[2].v[c]); }
+    for (int c = 0; c < V; ++c) {
+      const float s[5] = {w[0].v[c], w[1].v[c], w[2].v[c], w[3].v[c], w[4].v[c]};
+      const float z3[3] = {z[0].v[c], z[1].v[c], z[2].v[c]};
+      smax[c] = smin[c] = z3[1];
+      if (MONOT) {
+        if (kd >= kb + 1 && wm > 0.f) { smax[c] = fmaxf(smax[c], z3[0]); smin[c] = fminf(smin[c], z3[0]); }
+        if (kd <= mza - 2 && wp < 0.f) { smax[c] = fmaxf(smax[c], z3[2]); smin[c] = fminf(smin[c], z3[2]); }
+      }
+      float lo[2], hi[2];
+      lim_faces<MONOT>(mza, kd, kb, zl, zu, s, z3, lo, hi);
+      // 0 at the column's ends
+      const float sfm = kd == kb ? 0.f : fexpl * wm * hi[0], sfp = kd == mza - 1 ? 0.f : fexpl * wp * hi[1];
+      fin[c] = fmaxf(sfm, 0.f) - fminf(sfp, 0.f);
+      fout[c] = fminf(sfm, 0.f) - fmaxf(sfp, 0.f);
+      const float lv = wm * (lo[0] - z3[1]) - wp * (lo[1] - z3[1]);
+      fl[c] = impl ? fexpl * lv + fimpl * z3[1] * (wp - wm) : lv;
     }
   }
   const int4* E = A.edge + (size_t)iw * (7 * EDGE_W / 4);
@@ -381,7 +403,7 @@ __global__ void __launch_bounds__(256) k_scale(CellArgs A) {
       const OFF xv = (OFF)(e[i].y & 0x7fffffff) * mza + kd;
       vm[i] = 0.f;
       hv[i] = zerov<V>();
-      sn[i] = z[1];
+      sn[i] = s00;
       if (kd >= e[i].z) {
         vm[i] = __ldg(A.vmasc + xv);
         hv[i] = ldv<V>(A.face + (xv * A.nq + q) * V);
@@ -396,7 +418,7 @@ __global__ void __launch_bounds__(256) k_scale(CellArgs A) {
       const bool inflow = MONOT && dv * vm[i] > 0.f;
 #pragma unroll
       for (int c = 0; c < V; ++c) {
-        if (far) fl[c] = fl[c] + dv * vm[i] * (sn[i].v[c] - z[1].v[c]);
+        if (far) fl[c] = fl[c] + dv * vm[i] * (sn[i].v[c] - s00.v[c]);
         const float sf = dv * (vm[i] * hv[i].v[c]);
         if (MONOT) fin[c] = fin[c] + fmaxf(sf, 0.f);
         fout[c] = fout[c] + fminf(sf, 0.f);
@@ -404,46 +426,24 @@ __global__ void __launch_bounds__(256) k_scale(CellArgs A) {
       }
     }
   };
-  CELL_EDGES(np, edges);
+  CELL_EDGES3(np, edges);
   const float dtrp = (1.0f + kEps1) * A.dtr;
+  // the monotonic bounds of an implicit column count its mass change
+  const float rhb = MONOT && impl ? rh + A.dtr * vt * (fimpl * (wp - wm)) : rh;
   Vec<V> r0, r1;
 #pragma unroll
   for (int c = 0; c < V; ++c) {
-    const float s[5] = {w[0].v[c], w[1].v[c], w[2].v[c], w[3].v[c], w[4].v[c]};
-    const float z3[3] = {z[0].v[c], z[1].v[c], z[2].v[c]};
-    const float s00 = z3[1];
-    float lo[2], hi[2];
-    lim_faces<MONOT>(mza, kd, kb, zl, zu, s, z3, lo, hi);
-    // 0 at the column's ends
-    const float sfm = kd == kb ? 0.f : fexpl * wm * hi[0], sfp = kd == mza - 1 ? 0.f : fexpl * wp * hi[1];
-    float f = fl[c];
-    float mx = rh * smax[c], mn = rh * smin[c];
-    if (fimpl > .001f) {
-      const float dwi = fimpl * (wp - wm);
-      if (MONOT) {
-        f = f + fexpl * (wm * (lo[0] - s00) - wp * (lo[1] - s00)) + s00 * dwi;
-        const float imp = rh + A.dtr * vt * dwi;
-        mx = imp * smax[c];
-        mn = imp * smin[c];
-      } else {
-        f = f + fexpl * (wm * (lo[0] - s00) - wp * (lo[1] - s00)) + fimpl * s00 * (wp - wm);
-      }
-    } else {
-      f = f + wm * (lo[0] - s00) - wp * (lo[1] - s00);
-    }
-    const float gin = fin[c] + fmaxf(sfm, 0.f) - fminf(sfp, 0.f);
-    const float gout = fout[c] + fminf(sfm, 0.f) - fmaxf(sfp, 0.f);
-    const float low = s00 * rh + A.dtr * vt * f;
+    const float low = s00.v[c] * rh + A.dtr * vt * fl[c];
     if (MONOT) {
-      const float flux_in = fmaxf(dtrp * vt * gin, kEps0);
-      const float flux_out = fminf(dtrp * vt * gout, -kEps0);
+      const float flux_in = fmaxf(dtrp * vt * fin[c], kEps0);
+      const float flux_out = fminf(dtrp * vt * fout[c], -kEps0);
       const float epsr = kEps1 * fabsf(low);
-      const float sc_in = fmaxf(mx - (low + epsr) - kEps0, 0.f);
-      const float sc_out = fminf(mn - (low - epsr) + kEps0, 0.f);
+      const float sc_in = fmaxf(rhb * smax[c] - (low + epsr) - kEps0, 0.f);
+      const float sc_out = fminf(rhb * smin[c] - (low - epsr) + kEps0, 0.f);
       r0.v[c] = fminf(1.f, sc_in / fmaxf(flux_in, 0.01f * sc_in));
       r1.v[c] = fminf(1.f, sc_out / fminf(flux_out, 0.01f * sc_out));
     } else {
-      const float flux_out = fmaxf(-dtrp * vt * gout, kEps0);
+      const float flux_out = fmaxf(-dtrp * vt * fout[c], kEps0);
       const float sc_out = fmaxf((1.0f - kEps1) * low - kEps0, 0.f);
       r0.v[c] = fminf(1.f, sc_out / fmaxf(flux_out, 0.01f * sc_out));
     }
@@ -457,40 +457,66 @@ __global__ void __launch_bounds__(256) k_scale(CellArgs A) {
 // tracers of the group (without pdef under the positive-definite option)
 // take the unlimited update.
 template <int V, bool MONOT, typename OFF>
-__global__ void __launch_bounds__(256) k_update_lim(CellArgs A) {
+__global__ void __launch_bounds__(256, 3) k_update_lim(CellArgs A) {
   CELL_ITEM(A);
   const int kb = CELL_FLOOR(A);
   if (kd < kb) return;
   const int np = __ldg(A.npoly + iw);
   const float fimpl = __ldg(A.ff + (size_t)iw * A.nrk + A.istage - 1), fexpl = 1.0f - fimpl;
+  const bool impl = fimpl > .001f;
   const OFF row = (OFF)A.ld, cb = (OFF)iw * mza, x = cb + kd;
   const size_t plane = (size_t)A.mwa * mza * A.nq * V;
   const float* S0 = A.S0 + V * q;
   const float* sc = A.scale + (size_t)V * q;
   const OFF srow = (OFF)A.nq * V;
-  int md[V];
-  bool plain = false;
-  if (MONOT) {
-#pragma unroll
-    for (int c = 0; c < V; ++c) md[c] = MODE_MONOT;
-  } else {
+  unsigned pl = 0;                                     // the quad's PLAIN tracers
+  if (!MONOT) {
+    int md[V];
     quad_modes<V>(A, q, md);
 #pragma unroll
-    for (int c = 0; c < V; ++c) plain |= md[c] == MODE_PLAIN;
+    for (int c = 0; c < V; ++c) if (md[c] == MODE_PLAIN) pl |= 1u << c;
   }
-  Vec<V> w[5], z[3], a[3], b[3];
-  window<V, 2, OFF>(A.S + V * q, cb * row, row, kd, kb, mza, w);
-  window<V, 1, OFF>(S0, cb * row, row, kd, kb, mza, z);
-  window<V, 1, OFF>(sc, cb * srow, srow, kd, kb, mza, a);
-  if (MONOT) window<V, 1, OFF>(sc + plane, cb * srow, srow, kd, kb, mza, b);
   const float wm = __ldg(A.wmasc + x - 1), wp = __ldg(A.wmasc + x);
   const float vt = __ldg(A.volti + x), rh = __ldg(A.rhos + x);
-  const ZFace zl = zface(A.a_w, mza, kd - 1, kb, wm), zu = zface(A.a_w, mza, kd, kb, wp);
+  Vec<V> s00, a0, b0;                                  // scp0 and the factors of this cell
   float fd[V];
+  {
+    Vec<V> w[5], z[3], a[3], b[3];
+    window<V, 2, OFF>(A.S + V * q, cb * row, row, kd, kb, mza, w);
+    window<V, 1, OFF>(S0, cb * row, row, kd, kb, mza, z);
+    window<V, 1, OFF>(sc, cb * srow, srow, kd, kb, mza, a);
+    if (MONOT) window<V, 1, OFF>(sc + plane, cb * srow, srow, kd, kb, mza, b);
+    const ZFace zl = zface(A.a_w, mza, kd - 1, kb, wm), zu = zface(A.a_w, mza, kd, kb, wp);
+    s00 = z[1];
+    a0 = a[1];
+    b0 = MONOT ? b[1] : a[1];
 #pragma unroll
-  for (int c = 0; c < V; ++c) fd[c] = 0.f;
+    for (int c = 0; c < V; ++c) {
+      const float s[5] = {w[0].v[c], w[1].v[c], w[2].v[c], w[3].v[c], w[4].v[c]};
+      const float z3[3] = {z[0].v[c], z[1].v[c], z[2].v[c]};
+      float lo[2], hi[2];
+      lim_faces<MONOT>(mza, kd, kb, zl, zu, s, z3, lo, hi);
+      const bool bm = fexpl * wm * hi[0] < 0.f, bp = fexpl * wp * hi[1] < 0.f;
+      float cm, cp;
+      if (MONOT) {
+        cm = bm ? fminf(a[0].v[c], b[1].v[c]) : fminf(a[1].v[c], b[0].v[c]);
+        cp = bp ? fminf(a[1].v[c], b[2].v[c]) : fminf(a[2].v[c], b[1].v[c]);
+      } else {
+        cm = bm ? a[1].v[c] : a[0].v[c];
+        cp = bp ? a[2].v[c] : a[1].v[c];
+      }
+      float ul = kd == kb ? lo[0] : lo[0] + hi[0] * cm;
+      float uu = kd == mza - 1 ? lo[1] : lo[1] + hi[1] * cp;
+      if (!MONOT && ((pl >> c) & 1u)) {
+        ul = kd == kb ? s[2] : zvalue<false>(zl, s[0], s[1], s[2], s[3]);
+        uu = kd == mza - 1 ? s[2] : zvalue<false>(zu, s[1], s[2], s[3], s[4]);
+      }
+      const float f = wm * (ul - z3[1]) - wp * (uu - z3[1]);
+      fd[c] = impl || ((pl >> c) & 1u) ? fexpl * f : f;
+    }
+  }
   const int4* E = A.edge + (size_t)iw * (7 * EDGE_W / 4);
-  auto edges = [&](auto cnt, int n0) {   // three at a time: four or five quads each
+  auto edges = [&](auto cnt, int n0) {   // two or three at a time: five or four quads each
     constexpr int N = decltype(cnt)::value;
     int4 e[N];
     float vm[N];
@@ -502,13 +528,14 @@ __global__ void __launch_bounds__(256) k_update_lim(CellArgs A) {
       const OFF xv = (OFF)(e[i].y & 0x7fffffff) * mza + kd, xn = (OFF)e[i].x * mza + kd;
       vm[i] = 0.f;
       hv[i] = an[i] = bn[i] = zerov<V>();
-      sn[i] = z[1];
+      sn[i] = s00;
       if (kd >= e[i].z) {
         vm[i] = __ldg(A.vmasc + xv);
         hv[i] = ldv<V>(A.face + (xv * A.nq + q) * V);
-        sn[i] = ldv<V>(S0 + xn * row);
         an[i] = ldv<V>(sc + xn * srow);
         if (MONOT) bn[i] = ldv<V>(sc + plane + xn * srow);
+        // scp0 of the neighbour where it is upwind
+        if ((vm[i] < 0.f) != (e[i].y < 0)) sn[i] = ldv<V>(S0 + xn * row);
       }
     }
 #pragma unroll
@@ -516,55 +543,26 @@ __global__ void __launch_bounds__(256) k_update_lim(CellArgs A) {
       const bool open = kd >= e[i].z;
       const float f = __int_as_float(e[i].w) * vm[i];
       const bool second = e[i].y < 0;                  // this cell is side 2 of the face
-      const bool far = (vm[i] < 0.f) != second;
 #pragma unroll
       for (int c = 0; c < V; ++c) {
         // the correction runs from side 1 to side 2, or back where it is negative
         const bool back = vm[i] * hv[i].v[c] < 0.f;
         const bool from_here = back == second;         // this cell gives the corrected flux
-        const float s = MONOT ? (from_here ? fminf(an[i].v[c], b[1].v[c]) : fminf(a[1].v[c], bn[i].v[c]))
-                              : (from_here ? a[1].v[c] : an[i].v[c]);
-        // low-order value minus scp0, 0 where this cell is upwind
-        const float lo = far ? sn[i].v[c] : z[1].v[c];
-        const float up = md[c] == MODE_PLAIN ? hv[i].v[c] : lo + hv[i].v[c] * s;
-        if (open) fd[c] = fd[c] + f * (up - z[1].v[c]);
+        const float s = MONOT ? (from_here ? fminf(an[i].v[c], b0.v[c]) : fminf(a0.v[c], bn[i].v[c]))
+                              : (from_here ? a0.v[c] : an[i].v[c]);
+        const float up = (pl >> c) & 1u ? hv[i].v[c] : sn[i].v[c] + hv[i].v[c] * s;
+        if (open) fd[c] = fd[c] + f * (up - s00.v[c]);
       }
     }
   };
-  CELL_EDGES3(np, edges);
+  if constexpr (MONOT) { CELL_EDGES2(np, edges); }
+  else { CELL_EDGES3(np, edges); }
   Vec<V> o, tend = zerov<V>();
+  if (pl) tend = ldv<V>(A.SCT + V * q + x * row);
   const float dr = A.dtr / rh;
-  if (plain) tend = ldv<V>(A.SCT + x * row + V * q);
 #pragma unroll
-  for (int c = 0; c < V; ++c) {
-    const float s[5] = {w[0].v[c], w[1].v[c], w[2].v[c], w[3].v[c], w[4].v[c]};
-    const float z3[3] = {z[0].v[c], z[1].v[c], z[2].v[c]};
-    const float s00 = z3[1];
-    if (md[c] == MODE_PLAIN) {
-      const float ul = kd == kb ? s[2] : zvalue<false>(zl, s[0], s[1], s[2], s[3]);
-      const float uu = kd == mza - 1 ? s[2] : zvalue<false>(zu, s[1], s[2], s[3], s[4]);
-      const float f = fd[c] + fexpl * (wm * (ul - s00) - wp * (uu - s00));
-      o.v[c] = s00 + dr * (tend.v[c] + vt * f);
-      continue;
-    }
-    float lo[2], hi[2];
-    lim_faces<MONOT>(mza, kd, kb, zl, zu, s, z3, lo, hi);
-    const bool bm = fexpl * wm * hi[0] < 0.f, bp = fexpl * wp * hi[1] < 0.f;
-    float cm, cp;
-    if (MONOT) {
-      cm = bm ? fminf(a[0].v[c], b[1].v[c]) : fminf(a[1].v[c], b[0].v[c]);
-      cp = bp ? fminf(a[1].v[c], b[2].v[c]) : fminf(a[2].v[c], b[1].v[c]);
-    } else {
-      cm = bm ? a[1].v[c] : a[0].v[c];
-      cp = bp ? a[2].v[c] : a[1].v[c];
-    }
-    const float ul = kd == kb ? lo[0] : lo[0] + hi[0] * cm;
-    const float uu = kd == mza - 1 ? lo[1] : lo[1] + hi[1] * cp;
-    float f = fd[c];
-    if (fimpl > .001f) f = f + fexpl * (wm * (ul - s00) - wp * (uu - s00));
-    else f = f + wm * (ul - s00) - wp * (uu - s00);
-    o.v[c] = s00 + dr * vt * f;
-  }
+  for (int c = 0; c < V; ++c)
+    o.v[c] = (pl >> c) & 1u ? s00.v[c] + dr * (tend.v[c] + vt * fd[c]) : s00.v[c] + dr * vt * fd[c];
   float* out = A.out + V * q;
   stv<V>(out + x * row, o);
   // Below the floor the reference updates in place: scp(2:kb-1) = scp(kb) in
@@ -575,7 +573,7 @@ __global__ void __launch_bounds__(256) k_update_lim(CellArgs A) {
       Vec<V> y = ldv<V>(A.S + V * q + (cb + k) * row);
 #pragma unroll
       for (int c = 0; c < V; ++c)
-        if (md[c] == MODE_PLAIN || (!(fimpl > .001f) && k >= 1)) y.v[c] = o.v[c];
+        if (((pl >> c) & 1u) || (!impl && k >= 1)) y.v[c] = o.v[c];
       stv<V>(out + (cb + k) * row, y);
     }
 }
