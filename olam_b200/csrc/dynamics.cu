@@ -74,6 +74,17 @@ static DynK dynk(const DevGrid& d) {
   return k;
 }
 
+// The edge records of the column 2048 on, which a later wave of warps runs,
+// into L2 now: they are the first thing a warp waits for (NXP=100, 60 levels:
+// faces 222 -> 209 us, velocities 80 -> 74; 1024 or 4096 columns the same).
+// The column kernel and the dampings gain nothing by it.
+#define EDGES_AHEAD 2048
+__device__ __forceinline__ void edges_ahead(const DynK& g, const int4* E, int iw) {
+  const int lane = threadIdx.x & 31;
+  if (lane < 2 && iw + EDGES_AHEAD < g.mwa)
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(E + (size_t)EDGES_AHEAD * (7 * EDGE_W / 4) + 7 * lane));
+}
+
 // thread per (table entry j, level kd); n * mza < 2^31 (dyn_setup checks)
 #define PK(j, kd, n)                                               \
   const unsigned i_ = blockIdx.x * blockDim.x + threadIdx.x;       \
@@ -441,6 +452,7 @@ k_grad_upv4(DynK g, const int* __restrict__ prog, int nprog, int nch, Four s, un
   const int iw = WTAB((int)j), np = g.npoly[iw];
   const unsigned x = (unsigned)iw * (unsigned)mza + kd;
   const int4* E = g.edge + (size_t)iw * (7 * EDGE_W / 4);
+  edges_ahead(g, E, iw);
   float c0[4], a[4][NPL];
 #pragma unroll
   for (int f = 0; f < 4; ++f) {
@@ -991,6 +1003,7 @@ __global__ void __launch_bounds__(256) k_vel_t3d(DynK g, const int* __restrict__
   const int iw = WTAB((int)w_), kb = LPW(iw), np = g.npoly[iw];
   const size_t cb = (size_t)iw * mza;
   const int4* E = g.edge + (size_t)iw * (7 * EDGE_W / 4);
+  edges_ahead(g, E, iw);
   const float wx = wno2[iw * 3], wy = wno2[iw * 3 + 1], wz = wno2[iw * 3 + 2];
   const int lve = sh.lve2 ? sh.lve2[iw] : 0;
   int4 e[6];
