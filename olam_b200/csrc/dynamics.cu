@@ -213,6 +213,7 @@ __global__ void __launch_bounds__(256) k_damp_first(DynK g, DampArgs A) {
     int4 e[6];
 #pragma unroll
     for (int n = 0; n < 6; ++n) e[n] = __ldg(E + 2 * n);
+    grid_wait();
     float d[R], vt[R], ar[R][6], vm[R][6];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -252,6 +253,7 @@ __global__ void __launch_bounds__(256) k_damp_first(DynK g, DampArgs A) {
     for (int q = 0; q < 3; ++q) { iv[q] = g.m_iv[im * 3 + q]; f[q] = A.vfact[im * 3 + q]; }
 #pragma unroll
     for (int q = 0; q < 3; ++q) lv[q] = LPV(iv[q]);
+    grid_wait();
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -286,6 +288,7 @@ __global__ void __launch_bounds__(256) k_damp_lap(DynK g, DampArgs A) {
     float c[6];
 #pragma unroll
     for (int n = 0; n < 6; ++n) { e[n] = __ldg(E + 2 * n); c[n] = A.xx_yy[iw * 7 + n]; }
+    grid_wait();
     float s[R], x[R][6];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -322,6 +325,7 @@ __global__ void __launch_bounds__(256) k_damp_lap(DynK g, DampArgs A) {
       c[q] = A.xx_yy_m[im * 3 + q];
       lv[q] = LPV(g.m_iv[im * 3 + q]);
     }
+    grid_wait();
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int kd = lane + 32 * r;
@@ -371,6 +375,7 @@ __global__ void __launch_bounds__(256) k_vtend(DynK g, VtendArgs A) {
   const int iv = VPTAB((int)j), kv = LPV(iv);
   const int2 iw = *reinterpret_cast<const int2*>(g.v_iw + iv * 2), im = *reinterpret_cast<const int2*>(g.v_im + iv * 2);
   const size_t x = (size_t)iv * mza + kd;
+  grid_wait();
   const bool open = kd >= kv, div = A.dh && open, vor = A.fvorth && open;
   const bool ray = A.rayf_cof && kd >= A.krayf_bot - 1;
   float t = A.src[x], v0 = 0.f, fd = 0.f, d1 = 0.f, d2 = 0.f, v1 = 0.f, v2 = 0.f, fv = 0.f;
@@ -440,8 +445,8 @@ struct FaceFlux { const float* arv; float* vmca; float* vmasc; };
 template <int ORD, bool ALL>
 __global__ void __launch_bounds__(256, ORD == 2 ? 4 : 2)
 k_grad_upv4(DynK g, const int* __restrict__ prog, int nprog, int nch, Four s, unsigned gmask_,
-                            unsigned pmask, const float* __restrict__ xy_hu, VSide c, const float* __restrict__ vmc,
-                            float4* __restrict__ upv, FaceFlux ff) {
+                            unsigned pmask, const float* __restrict__ xy_hu, VSide c, const float* vmc,
+                            float4* upv, FaceFlux ff) {
   constexpr int NPL = ORD == 2 ? 2 : 5;
   const unsigned gmask = ALL ? 0xFu : gmask_;
   const unsigned w_ = blockIdx.x * 8u + (threadIdx.x >> 5);
@@ -453,6 +458,7 @@ k_grad_upv4(DynK g, const int* __restrict__ prog, int nprog, int nch, Four s, un
   const unsigned x = (unsigned)iw * (unsigned)mza + kd;
   const int4* E = g.edge + (size_t)iw * (7 * EDGE_W / 4);
   edges_ahead(g, E, iw);
+  grid_wait();
   float c0[4], a[4][NPL];
 #pragma unroll
   for (int f = 0; f < 4; ++f) {
@@ -766,6 +772,7 @@ __global__ void __launch_bounds__(32 * NW * WRT_COLS(NW), WRT_OCC / (NW * WRT_CO
   int4 e[6];
 #pragma unroll
   for (int n = 0; n < 6; ++n) e[n] = __ldg(E + 2 * n);
+  grid_wait();
   float th = A.sh_th[x], vx = A.sh_vx[x], vy = A.sh_vy[x], vz = A.sh_vz[x];
   const double rho = A.rho[x], volt = A.volt[x];
   const float thil = A.thil[x], vye = A.vye[x], vxe = A.vxe[x], alpha = A.alpha_press[x];
@@ -787,8 +794,8 @@ __global__ void __launch_bounds__(32 * NW * WRT_COLS(NW), WRT_OCC / (NW * WRT_CO
     fu[n] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (kd >= e[n].z) {
       const size_t xv = (size_t)(e[n].y & 0x7fffffff) * mza + kd;
-      vm[n] = __ldg(A.vmca + xv);
-      fu[n] = __ldg(A.upv + xv);
+      vm[n] = A.vmca[xv];
+      fu[n] = A.upv[xv];
     }
   }
   if (LEAN) {
@@ -817,7 +824,7 @@ __global__ void __launch_bounds__(32 * NW * WRT_COLS(NW), WRT_OCC / (NW * WRT_CO
     const int4 q = __ldg(E + 12);
     if (kd >= q.z) {
       const size_t xv = (size_t)(q.y & 0x7fffffff) * mza + kd;
-      add(q, __ldg(A.vmca + xv), __ldg(A.upv + xv));
+      add(q, A.vmca[xv], A.upv[xv]);
     }
   }
   const float mass = (float)(rho * volt);
@@ -930,17 +937,18 @@ __global__ void __launch_bounds__(32 * NW * WRT_COLS(NW), WRT_OCC / (NW * WRT_CO
 }
 
 // prog_v_begs (prog_wrtv_rk.f90:888-946)
-__global__ void k_prog_v(DynK g, const int* __restrict__ vprog, int nv, float dts, const float* __restrict__ vmc0,
-                         const float* __restrict__ vmt_short, const double* __restrict__ press,
+__global__ void k_prog_v(DynK g, const int* __restrict__ vprog, int nv, float dts, const float* vmc0,
+                         const float* vmt_short, const double* press,
                          const float* __restrict__ pvfac, const float* __restrict__ vn,
-                         const float* __restrict__ rkx, const float* __restrict__ rky,
-                         const float* __restrict__ rkz, const float* __restrict__ volvi,
-                         const double* __restrict__ rho, float* __restrict__ vmc, float* __restrict__ vc) {
+                         const float* rkx, const float* rky,
+                         const float* rkz, const float* __restrict__ volvi,
+                         const double* rho, float* vmc, float* vc) {
   PK(j, kd, nv);
   const int iv = VPTAB(j);
   if (kd < LPV(iv)) return;
   const int mza = g.mza;
   const int iw1 = g.v_iw[iv * 2], iw2 = g.v_iw[iv * 2 + 1];
+  grid_wait();
   const size_t x = (size_t)iv * mza + kd, x1 = (size_t)iw1 * mza + kd, x2 = (size_t)iw2 * mza + kd;
   const float pgf = (float)(press[x1] - press[x2]) * pvfac[x];
   const float v = vmc0[x] + dts * (vmt_short[x] + pgf +
@@ -994,10 +1002,10 @@ static Shaved shaved_args(const Dyn& y, const Transport& tp, int prog, float dts
 // component of the cell's prognosed velocity at that level
 // ecv: four floats per edge (x, y, z, 0), 7 edges per column
 template <int R>
-__global__ void __launch_bounds__(256) k_vel_t3d(DynK g, const int* __restrict__ prog, int nprog, const float* __restrict__ wc,
-                          const float* __restrict__ vc, const float* __restrict__ wno2,
-                          const float4* __restrict__ ecv, float* __restrict__ vxe, float* __restrict__ vye,
-                          float* __restrict__ vze, Shaved sh) {
+__global__ void __launch_bounds__(256) k_vel_t3d(DynK g, const int* __restrict__ prog, int nprog, const float* wc,
+                          const float* vc, const float* __restrict__ wno2,
+                          const float4* __restrict__ ecv, float* vxe, float* vye,
+                          float* vze, Shaved sh) {
   WARP_POINT(nprog, 0u);
   const int mza = g.mza;
   const int iw = WTAB((int)w_), kb = LPW(iw), np = g.npoly[iw];
@@ -1010,6 +1018,7 @@ __global__ void __launch_bounds__(256) k_vel_t3d(DynK g, const int* __restrict__
   float4 ec[6];
 #pragma unroll
   for (int n = 0; n < 6; ++n) { e[n] = __ldg(E + 2 * n); ec[n] = __ldg(ecv + iw * 7 + n); }
+  grid_wait();
   float wl[R], wu[R], v[R][6];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -1068,6 +1077,7 @@ __global__ void __launch_bounds__(256) k_vel_t3d(DynK g, const int* __restrict__
 // tend0 (timestep.f90:430-496) for the hot-path arrays
 __global__ void k_tend0_w(DynK g, float* thilt, float* vmxet, float* vmyet, float* vmzet,
                           const double* rho, float* rho_old, float* wmasc) {
+  grid_wait();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)(g.mwa - 1) * g.mza) return;
   const int iw = 1 + (int)(i / g.mza), kd = (int)(i % g.mza);
@@ -1079,6 +1089,7 @@ __global__ void k_tend0_w(DynK g, float* thilt, float* vmxet, float* vmyet, floa
 }
 
 __global__ void k_tend0_v(DynK g, float* vmt, float* vmasc) {
+  grid_wait();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)(g.mva - 1) * g.mza) return;
   const int iv = 1 + (int)(i / g.mza), kd = (int)(i % g.mza);
@@ -1090,6 +1101,7 @@ __global__ void k_tend0_v(DynK g, float* vmt, float* vmasc) {
 
 // timeavg_momsc (timestep.f90:563-612)
 __global__ void k_timeavg_v(DynK g, const int* __restrict__ vadj, int nv, float a, float* vmasc) {
+  grid_wait();
   PK(j, kd, nv);
   const int iv = VATAB(j);
   if (kd < LPV(iv)) return;
@@ -1097,6 +1109,7 @@ __global__ void k_timeavg_v(DynK g, const int* __restrict__ vadj, int nv, float 
 }
 
 __global__ void k_timeavg_w(DynK g, const int* __restrict__ prog, int nprog, float a, float* wmasc) {
+  grid_wait();
   PK(j, kd, nprog);
   const int iw = WTAB(j);
   if (kd < LPW(iw) || kd > g.mza - 2) return;
@@ -1376,8 +1389,8 @@ static int v_tendency(Context& C, bool div, bool vor, bool setup, const float* s
     A.wsrc = plane(y.div2d.p, wz, il); A.wdst = plane(y.div2d.p, wz, ih);
     A.msrc = plane(y.vort2d.p, mz, il); A.mdst = plane(y.vort2d.p, mz, ih);
     if (nb == 0) return OLAMGPU_OK;
-    if (step == 0) BY_ROWS(mza, k_damp_first<R><<<nb, 256, 0, s>>>(g, A));
-    else BY_ROWS(mza, k_damp_lap<R><<<nb, 256, 0, s>>>(g, A));
+    if (step == 0) BY_ROWS(mza, launch_next(k_damp_first<R>, nb, 256, 0, s, g, A));
+    else BY_ROWS(mza, launch_next(k_damp_lap<R>, nb, 256, 0, s, g, A));
     // border planes for the Laplacian and the apply (vort_div_damp.f90:150, 208)
     if (dw) { HField f[1] = {{A.wdst, 4}}; OG_CHECK(halo_exchange_fields(C, HALO_W, f, 1, s)); }
     if (dm) { HField f[1] = {{A.mdst, 4}}; OG_CHECK(halo_exchange_fields(C, HALO_M, f, 1, s)); }
@@ -1401,14 +1414,14 @@ static int v_tendency(Context& C, bool div, bool vor, bool setup, const float* s
     V.vl = plane(y.vort2d.p, mz, lv == 1 ? 1 : (lv - 2) % 2 + 1);
     V.vh = plane(y.vort2d.p, mz, lv == 1 ? 1 : (lv - 1) % 2 + 1);
   }
-  if (d.nv_prog > 0) { k_vtend<<<cdiv((size_t)d.nv_prog * ((mza + 31) / 32), 8), 256, 0, s>>>(g, V); OG_LAUNCHED(); }
+  if (d.nv_prog > 0) { launch_next(k_vtend, cdiv((size_t)d.nv_prog * ((mza + 31) / 32), 8), 256, 0, s, g, V); OG_LAUNCHED(); }
   return OLAMGPU_OK;
 }
 
 static void launch_vel_t3d(Context& C, const Shaved& sh, cudaStream_t s) {
   const DevGrid& d = C.g;
   Dyn& y = C.dy;
-  BY_ROWS(d.mza, k_vel_t3d<R><<<cdiv(d.nw_prog, 8), 256, 0, s>>>(dynk(d), d.jtw_prog.p, d.nw_prog, C.tp.wc.p, y.vc.p, y.wno2.p,
+  BY_ROWS(d.mza, launch_next(k_vel_t3d<R>, cdiv(d.nw_prog, 8), 256, 0, s, dynk(d), d.jtw_prog.p, d.nw_prog, C.tp.wc.p, y.vc.p, y.wno2.p,
                                                                  reinterpret_cast<const float4*>(y.ecv.p), y.vxe.p,
                                                                  y.vye.p, y.vze.p, sh));
 }
@@ -1532,13 +1545,13 @@ int dyn_prog_wrtv_rk(int istp) {
       float4* upv = reinterpret_cast<float4*>(y.upv.p);
       const unsigned plain = 0xFu & ~(m2 | m3);
       if (m2 || plain) {
-        if (m2 == 0xFu) k_grad_upv4<2, true><<<nbg, 256, 0, s>>>(gg, gt, gn, nch, f, m2, plain, d.xy_hu.p, vs, y.vmc.p, upv, ffx);
-        else k_grad_upv4<2, false><<<nbg, 256, 0, s>>>(gg, gt, gn, nch, f, m2, plain, d.xy_hu.p, vs, y.vmc.p, upv, ffx);
+        if (m2 == 0xFu) launch_next(k_grad_upv4<2, true>, nbg, 256, 0, s, gg, gt, gn, nch, f, m2, plain, d.xy_hu.p, vs, y.vmc.p, upv, ffx);
+        else launch_next(k_grad_upv4<2, false>, nbg, 256, 0, s, gg, gt, gn, nch, f, m2, plain, d.xy_hu.p, vs, y.vmc.p, upv, ffx);
         OG_LAUNCHED();
         ffx = FaceFlux{};   // once a stage
       }
       if (m3) {
-        k_grad_upv4<3, false><<<nbg, 256, 0, s>>>(gg, gt, gn, nch, f, m3, 0u, d.xy_hu.p, vs, y.vmc.p, upv, ffx);
+        launch_next(k_grad_upv4<3, false>, nbg, 256, 0, s, gg, gt, gn, nch, f, m3, 0u, d.xy_hu.p, vs, y.vmc.p, upv, ffx);
         OG_LAUNCHED();
       }
     }
@@ -1580,8 +1593,8 @@ int dyn_prog_wrtv_rk(int istp) {
         constexpr int cols = WRT_COLS(R);
         const size_t smem = (size_t)cols * ((R == 1 ? 224 : 128 * R) + 4 * mza) * sizeof(double);   // 11.2 KB or less
         const unsigned nb = cdiv(d.nw_prog, cols);
-        if (lean) k_wrt_begs<R, true><<<nb, 32 * R * cols, smem, s>>>(g, A);
-        else k_wrt_begs<R, false><<<nb, 32 * R * cols, smem, s>>>(g, A);
+        if (lean) launch_next(k_wrt_begs<R, true>, nb, 32 * R * cols, smem, s, g, A);
+        else launch_next(k_wrt_begs<R, false>, nb, 32 * R * cols, smem, s, g, A);
       });
     }
     if (C.halo.on) {
@@ -1592,7 +1605,7 @@ int dyn_prog_wrtv_rk(int istp) {
     }
     {
       OG_PROF("prog_v", s);
-      k_prog_v<<<nbv, 256, 0, s>>>(g, d.jtv_prog.p, d.nv_prog, dts, y.vmc0.p, y.sh_vmt.p, y.press.p, y.pvfac.p,
+      launch_next(k_prog_v, nbv, 256, 0, s, g, d.jtv_prog.p, d.nv_prog, dts, y.vmc0.p, y.sh_vmt.p, y.press.p, y.pvfac.p,
                                    y.vn.p, y.rk_vx.p, y.rk_vy.p, y.rk_vz.p, y.volvi.p, tp.rho.p, y.vmc.p, y.vc.p);
       OG_LAUNCHED();
     }
@@ -1635,10 +1648,10 @@ int dyn_tend0(float* rho_old_host) {
   const DynK g = dynk(C.g);
   Dyn& y = C.dy;
   Transport& tp = C.tp;
-  k_tend0_w<<<cdiv((size_t)(C.g.mwa - 1) * C.g.mza, 256), 256, 0, s>>>(g, y.thilt.p, y.vmxet.p, y.vmyet.p,
+  launch_next(k_tend0_w, cdiv((size_t)(C.g.mwa - 1) * C.g.mza, 256), 256, 0, s, g, y.thilt.p, y.vmxet.p, y.vmyet.p,
                                                                       y.vmzet.p, tp.rho.p, tp.rho_old.p,
                                                                       tp.wmasc.p);
-  k_tend0_v<<<cdiv((size_t)(C.g.mva - 1) * C.g.mza, 256), 256, 0, s>>>(g, y.vmt.p, tp.vmasc.p);
+  launch_next(k_tend0_v, cdiv((size_t)(C.g.mva - 1) * C.g.mza, 256), 256, 0, s, g, y.vmt.p, tp.vmasc.p);
   OG_LAUNCHED(); OG_LAUNCHED();
   // scalar tendencies var_t = 0 for k >= lpw (the device copies)
   // (a window's adjoint lends the per-tracer arrays' memory out while it
@@ -1667,8 +1680,8 @@ int dyn_timeavg_momsc() {
   else if (!C.dy.uploaded) { OG_CHECK(dyn_state_to_device(DYN_IN_MASK, s)); C.dy.uploaded = true; }
   const DynK g = dynk(C.g);
   const float a = (float)C.opts.nacoust;
-  k_timeavg_v<<<cdiv((size_t)C.g.nv_wadj * C.g.mza, 256), 256, 0, s>>>(g, C.g.jtv_wadj.p, C.g.nv_wadj, a, C.tp.vmasc.p);
-  k_timeavg_w<<<cdiv((size_t)C.g.nw_prog * C.g.mza, 256), 256, 0, s>>>(g, C.g.jtw_prog.p, C.g.nw_prog, a, C.tp.wmasc.p);
+  launch_next(k_timeavg_v, cdiv((size_t)C.g.nv_wadj * C.g.mza, 256), 256, 0, s, g, C.g.jtv_wadj.p, C.g.nv_wadj, a, C.tp.vmasc.p);
+  launch_next(k_timeavg_w, cdiv((size_t)C.g.nw_prog * C.g.mza, 256), 256, 0, s, g, C.g.jtw_prog.p, C.g.nw_prog, a, C.tp.wmasc.p);
   OG_LAUNCHED(); OG_LAUNCHED();
   if (C.coherence == OLAMGPU_SYNC_EACH_CALL) {
     OG_CHECK(dyn_state_to_host(OLAMGPU_F_VMASC | OLAMGPU_F_WMASC, s));

@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/olamgpu.h"
@@ -600,6 +601,36 @@ int upload(DevBuf<T>& b, const T* h, size_t n, cudaStream_t s) {
   if (n) OG_CUDA(cudaMemcpyAsync(b.p, h, n * sizeof(T), cudaMemcpyHostToDevice, s));
   return OLAMGPU_OK;
 }
+
+// Launch of a kernel that may start while the kernel before it on the stream
+// ends (programmatic dependent launch): its blocks are placed as the other's
+// last ones run.  Such a kernel calls grid_wait() before it reads or writes
+// anything another kernel writes (tables of the set-up may be read before),
+// and reads such data with ordinary loads: the non-coherent path (__ldg,
+// __restrict__) is for what nothing writes while the kernel is resident.  At
+// least one thread of every launch reaches grid_wait, so a kernel ends after
+// the one before it.
+template <typename... P, typename... Q>
+inline void launch_next(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, Q&&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute a{};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &a;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, k, std::forward<Q>(args)...);   // errors are read with cudaGetLastError, as of <<<>>>
+}
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.launch_dependents;\n");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+#endif
 
 inline unsigned int cdiv(size_t a, size_t b) { return (unsigned int)((a + b - 1) / b); }
 

@@ -42,19 +42,19 @@ struct CellArgs {
   const int* __restrict__ lpw;
   const int4* __restrict__ edge;    // EDGE_W words per edge
   const float4* __restrict__ edge3; // order 3: EDGE3_W words per edge
-  const float* __restrict__ vmasc;
-  const float* __restrict__ wmasc;
+  const float* vmasc;
+  const float* wmasc;
   const float* __restrict__ volti;
   const float* __restrict__ a_w;    // bounded or unbounded, as the pass needs
-  const float* __restrict__ rhos;
-  const float* __restrict__ ff;     // (mwa, nrk), NULL: every column explicit
+  const float* rhos;
+  const float* ff;     // (mwa, nrk), NULL: every column explicit
   const int* __restrict__ mode;     // limited stage: mode of each tracer
-  const float* __restrict__ S;
-  const float* __restrict__ S0;
-  const float* __restrict__ SCT;
-  float* __restrict__ out;
-  float* __restrict__ face;         // (mva, mza, nq V)
-  float* __restrict__ scale;        // (mwa, mza, nq V), two planes with the monotonic limiter
+  const float* S;
+  const float* S0;
+  const float* SCT;
+  float* out;
+  float* face;         // (mva, mza, nq V)
+  float* scale;        // (mwa, mza, nq V), two planes with the monotonic limiter
   int ld, nt;                       // row length of S, S0, SCT, out; tracers
   int istage, nrk;
   float dtr;
@@ -67,17 +67,12 @@ template <int V>
 __device__ __forceinline__ Vec<V> ldv(const float* p) {
   Vec<V> r;
   if constexpr (V == 4) {
-    const float4 x = __ldg(reinterpret_cast<const float4*>(p));
+    const float4 x = *reinterpret_cast<const float4*>(p);
     r.v[0] = x.x; r.v[1] = x.y; r.v[2] = x.z; r.v[3] = x.w;
   } else {
-    r.v[0] = __ldg(p);
+    r.v[0] = *p;
   }
   return r;
-}
-// of an array that the kernel also writes
-__device__ __forceinline__ Vec<4> ldv_rw(const float* p) {
-  const float4 x = *reinterpret_cast<const float4*>(p);
-  return Vec<4>{{x.x, x.y, x.z, x.w}};
 }
 template <int V>
 __device__ __forceinline__ void stv(float* p, const Vec<V>& r) {
@@ -119,6 +114,7 @@ __device__ __forceinline__ Vec<V> subv(const Vec<V>& x, const Vec<V>& y) { retur
   const int kd = (int)(i_ / (unsigned)A.nq), q = (int)(i_ - (unsigned)kd * (unsigned)A.nq); \
   const int iw = A.off >= 0 ? A.off + (int)j_ : __ldg(A.cols + j_);                       \
   const int mza = A.mza;                                                                  \
+  grid_wait();                                                                            \
   if (kd >= mza) return;
 #define CELL_FLOOR(A) (A.flat ? 1 : __ldg(A.lpw + iw))
 
@@ -208,7 +204,7 @@ __global__ void __launch_bounds__(256, ORDER == 2 ? 4 : 3) k_face(CellArgs A) {
     for (int i = 0; i < N; ++i) e[i] = __ldg(E + 2 * (n0 + i));
 #pragma unroll
     for (int i = 0; i < N; ++i)
-      vm[i] = kd >= e[i].z ? __ldg(A.vmasc + ((OFF)(e[i].y & 0x7fffffff) * mza + kd)) : 0.f;
+      vm[i] = kd >= e[i].z ? A.vmasc[(OFF)(e[i].y & 0x7fffffff) * mza + kd] : 0.f;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       if (kd < e[i].z || (vm[i] < 0.f) != (e[i].y < 0)) continue;  // closed, or the other cell is upwind
@@ -294,13 +290,13 @@ __global__ void __launch_bounds__(256) k_update(CellArgs A) {
   const int kb = CELL_FLOOR(A);
   if (kd < kb) return;                                // written by the thread of level kb
   const int np = __ldg(A.npoly + iw);
-  const float fexpl = A.ff ? 1.0f - __ldg(A.ff + (size_t)iw * A.nrk + A.istage - 1) : 1.0f;
+  const float fexpl = A.ff ? 1.0f - A.ff[(size_t)iw * A.nrk + A.istage - 1] : 1.0f;
   const OFF row = (OFF)A.ld, cb = (OFF)iw * mza, x = cb + kd;
   const Vec<V> s00 = ldv<V>(A.S0 + V * q + x * row), tend = ldv<V>(A.SCT + V * q + x * row);
   Vec<V> w[5];
   window<V, 2, OFF>(A.S + V * q, cb * row, row, kd, kb, mza, w);
-  const float wm = __ldg(A.wmasc + x - 1), wp = __ldg(A.wmasc + x);
-  const float vt = __ldg(A.volti + x), rh = __ldg(A.rhos + x);
+  const float wm = A.wmasc[x - 1], wp = A.wmasc[x];
+  const float vt = __ldg(A.volti + x), rh = A.rhos[x];
   Vec<V> fd = zerov<V>();
   const int4* E = A.edge + (size_t)iw * (7 * EDGE_W / 4);
   auto edges = [&](auto cnt, int n0) {
@@ -315,7 +311,7 @@ __global__ void __launch_bounds__(256) k_update(CellArgs A) {
       const OFF xv = (OFF)(e[i].y & 0x7fffffff) * mza + kd;
       vm[i] = 0.f;
       up[i] = s00;
-      if (kd >= e[i].z) { vm[i] = __ldg(A.vmasc + xv); up[i] = ldv<V>(A.face + (xv * A.nq + q) * V); }
+      if (kd >= e[i].z) { vm[i] = A.vmasc[xv]; up[i] = ldv<V>(A.face + (xv * A.nq + q) * V); }
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) fd = fmav<V>(__int_as_float(e[i].w) * vm[i], subv<V>(up[i], s00), fd);
@@ -357,12 +353,12 @@ __global__ void __launch_bounds__(256, 3) k_scale(CellArgs A) {
   const int kb = CELL_FLOOR(A);
   if (kd < kb) return;
   const int np = __ldg(A.npoly + iw);
-  const float fimpl = __ldg(A.ff + (size_t)iw * A.nrk + A.istage - 1), fexpl = 1.0f - fimpl;
+  const float fimpl = A.ff[(size_t)iw * A.nrk + A.istage - 1], fexpl = 1.0f - fimpl;
   const bool impl = fimpl > .001f;
   const OFF row = (OFF)A.ld, cb = (OFF)iw * mza, x = cb + kd;
   const float* S0 = A.S0 + V * q;
-  const float wm = __ldg(A.wmasc + x - 1), wp = __ldg(A.wmasc + x);
-  const float rh = __ldg(A.rhos + x), vt = __ldg(A.volti + x);
+  const float wm = A.wmasc[x - 1], wp = A.wmasc[x];
+  const float rh = A.rhos[x], vt = __ldg(A.volti + x);
   float fl[V], fin[V], fout[V], smax[V], smin[V];
   Vec<V> s00;
   {
@@ -405,7 +401,7 @@ __global__ void __launch_bounds__(256, 3) k_scale(CellArgs A) {
       hv[i] = zerov<V>();
       sn[i] = s00;
       if (kd >= e[i].z) {
-        vm[i] = __ldg(A.vmasc + xv);
+        vm[i] = A.vmasc[xv];
         hv[i] = ldv<V>(A.face + (xv * A.nq + q) * V);
         sn[i] = ldv<V>(S0 + ((OFF)e[i].x * mza + kd) * row);
       }
@@ -462,7 +458,7 @@ __global__ void __launch_bounds__(256, 3) k_update_lim(CellArgs A) {
   const int kb = CELL_FLOOR(A);
   if (kd < kb) return;
   const int np = __ldg(A.npoly + iw);
-  const float fimpl = __ldg(A.ff + (size_t)iw * A.nrk + A.istage - 1), fexpl = 1.0f - fimpl;
+  const float fimpl = A.ff[(size_t)iw * A.nrk + A.istage - 1], fexpl = 1.0f - fimpl;
   const bool impl = fimpl > .001f;
   const OFF row = (OFF)A.ld, cb = (OFF)iw * mza, x = cb + kd;
   const size_t plane = (size_t)A.mwa * mza * A.nq * V;
@@ -476,8 +472,8 @@ __global__ void __launch_bounds__(256, 3) k_update_lim(CellArgs A) {
 #pragma unroll
     for (int c = 0; c < V; ++c) if (md[c] == MODE_PLAIN) pl |= 1u << c;
   }
-  const float wm = __ldg(A.wmasc + x - 1), wp = __ldg(A.wmasc + x);
-  const float vt = __ldg(A.volti + x), rh = __ldg(A.rhos + x);
+  const float wm = A.wmasc[x - 1], wp = A.wmasc[x];
+  const float vt = __ldg(A.volti + x), rh = A.rhos[x];
   Vec<V> s00, a0, b0;                                  // scp0 and the factors of this cell
   float fd[V];
   {
@@ -530,7 +526,7 @@ __global__ void __launch_bounds__(256, 3) k_update_lim(CellArgs A) {
       hv[i] = an[i] = bn[i] = zerov<V>();
       sn[i] = s00;
       if (kd >= e[i].z) {
-        vm[i] = __ldg(A.vmasc + xv);
+        vm[i] = A.vmasc[xv];
         hv[i] = ldv<V>(A.face + (xv * A.nq + q) * V);
         an[i] = ldv<V>(sc + xn * srow);
         if (MONOT) bn[i] = ldv<V>(sc + plane + xn * srow);
@@ -580,16 +576,16 @@ __global__ void __launch_bounds__(256, 3) k_update_lim(CellArgs A) {
 
 // last-stage low-order pre-update of scp0 for the tracers flagged in mode
 // (scalar_transport_rk.F90:297-314), in place
-__global__ void __launch_bounds__(256) k_preupdate(CellArgs A, float* __restrict__ S0, const float* __restrict__ rho_old) {
+__global__ void __launch_bounds__(256) k_preupdate(CellArgs A, float* S0, const float* rho_old) {
   CELL_ITEM(A);
   const int kb = CELL_FLOOR(A);
   if (kd < kb) return;
   constexpr int V = 4;
   const size_t row = (size_t)A.ld;
   float* p = S0 + (size_t)iw * mza * row + V * q;
-  Vec<V> s = ldv_rw(p + (size_t)kd * row);
+  Vec<V> s = ldv<V>(p + (size_t)kd * row);
   const Vec<V> t = ldv<V>(A.SCT + ((size_t)iw * mza + kd) * row + V * q);
-  const float ro = __ldg(rho_old + (size_t)iw * mza + kd);
+  const float ro = rho_old[(size_t)iw * mza + kd];
   int md[V];
   quad_modes<V>(A, q, md);
 #pragma unroll
@@ -597,7 +593,7 @@ __global__ void __launch_bounds__(256) k_preupdate(CellArgs A, float* __restrict
   stv<V>(p + (size_t)kd * row, s);
   if (kd == kb)
     for (int k = 1; k < kb; ++k) {
-      Vec<V> y = ldv_rw(p + (size_t)k * row);
+      Vec<V> y = ldv<V>(p + (size_t)k * row);
 #pragma unroll
       for (int c = 0; c < V; ++c) if (md[c]) y.v[c] = s.v[c];
       stv<V>(p + (size_t)k * row, y);
@@ -644,11 +640,11 @@ static int run_stage(const DevGrid& d, int order, const CellStage& c, cudaStream
     OG_PROF(lim ? "lim_face" : "cell_face", s);
     const unsigned nb = cell_blocks(A);
     if (!lim) {
-      if (order == 2) k_face<V, 2, false, OFF><<<nb, 256, 0, s>>>(A);
-      else k_face<V, 3, false, OFF><<<nb, 256, 0, s>>>(A);
+      if (order == 2) launch_next(k_face<V, 2, false, OFF>, nb, 256, 0, s, A);
+      else launch_next(k_face<V, 3, false, OFF>, nb, 256, 0, s, A);
     } else if constexpr (V == 4) {
-      if (order == 2) k_face<V, 2, true, OFF><<<nb, 256, 0, s>>>(A);
-      else k_face<V, 3, true, OFF><<<nb, 256, 0, s>>>(A);
+      if (order == 2) launch_next(k_face<V, 2, true, OFF>, nb, 256, 0, s, A);
+      else launch_next(k_face<V, 3, true, OFF>, nb, 256, 0, s, A);
     }
     OG_LAUNCHED();
   }
@@ -657,8 +653,8 @@ static int run_stage(const DevGrid& d, int order, const CellStage& c, cudaStream
       // the factors of both cells of every face of a prognosed column
       OG_PROF("lim_scale", s);
       const unsigned nb = cell_blocks(A);
-      if (monot) k_scale<V, true, OFF><<<nb, 256, 0, s>>>(A);
-      else k_scale<V, false, OFF><<<nb, 256, 0, s>>>(A);
+      if (monot) launch_next(k_scale<V, true, OFF>, nb, 256, 0, s, A);
+      else launch_next(k_scale<V, false, OFF>, nb, 256, 0, s, A);
       OG_LAUNCHED();
     }
   }
@@ -666,10 +662,10 @@ static int run_stage(const DevGrid& d, int order, const CellStage& c, cudaStream
   {
     OG_PROF(lim ? "lim_update" : "cell_update", s);
     const unsigned nb = cell_blocks(A);
-    if (!lim) k_update<V, OFF><<<nb, 256, 0, s>>>(A);
+    if (!lim) launch_next(k_update<V, OFF>, nb, 256, 0, s, A);
     else if constexpr (V == 4) {
-      if (monot) k_update_lim<V, true, OFF><<<nb, 256, 0, s>>>(A);
-      else k_update_lim<V, false, OFF><<<nb, 256, 0, s>>>(A);
+      if (monot) launch_next(k_update_lim<V, true, OFF>, nb, 256, 0, s, A);
+      else launch_next(k_update_lim<V, false, OFF>, nb, 256, 0, s, A);
     }
     OG_LAUNCHED();
   }
@@ -692,7 +688,7 @@ void launch_cell_preupdate(const DevGrid& d, const Transport& tp, float* S0, con
   A.ld = ld; A.nt = nt; A.mode = mode; A.SCT = SCT; A.dtr = dtr;
   over(A, d.jtw_wadj, d.nw_wadj, d.off_wwadj);
   OG_PROF("lim_preupdate", s);
-  k_preupdate<<<cell_blocks(A), 256, 0, s>>>(A, S0, tp.rho_old.p);
+  launch_next(k_preupdate, cell_blocks(A), 256, 0, s, A, S0, tp.rho_old.p);
   OG_LAUNCHED();
 }
 

@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(256) k_prepare(PrepArgs A) {
     int4 e[7];
 #pragma unroll
     for (int n = 0; n < 7; ++n) e[n] = __ldg(A.edge + ((size_t)iw * 7 + n) * (EDGE_W / 4));
+    grid_wait();
     float fimp[3] = {0.f, 0.f, 0.f};
     // the lane's largest values and where it met them first
     float mc = 0.f, mh = 0.f, mw = 0.f;
@@ -101,11 +102,11 @@ __global__ void __launch_bounds__(256) k_prepare(PrepArgs A) {
 #pragma unroll
       for (int n = 0; n < 7; ++n) {
         vm[n] = 0.f;
-        if (n < np && kd >= e[n].z) vm[n] = __ldg(A.vmasc + (size_t)(e[n].y & 0x7fffffff) * mza + kd);
+        if (n < np && kd >= e[n].z) vm[n] = A.vmasc[(size_t)(e[n].y & 0x7fffffff) * mza + kd];
       }
-      const float ro = __ldg(A.rho_old + cb + kd), vt = __ldg(g.volti + cb + kd);
-      const float wp = __ldg(A.wmasc + cb + kd), wm = __ldg(A.wmasc + cb + kd - 1);
-      const float rhof = (float)__ldg(A.rho + cb + kd);
+      const float ro = A.rho_old[cb + kd], vt = __ldg(g.volti + cb + kd);
+      const float wp = A.wmasc[cb + kd], wm = A.wmasc[cb + kd - 1];
+      const float rhof = (float)A.rho[cb + kd];
       float cflh = 0.f;
 #pragma unroll
       for (int n = 0; n < 7; ++n)
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(256) k_prepare(PrepArgs A) {
       if (cflh != cflh) nh = order + 1ull;
       else if (cflh > mh) { mh = cflh; oh = order; }
       if (A.wc) {
-        const float w = fabsf(__ldg(A.wc + cb + kd));
+        const float w = fabsf(A.wc[cb + kd]);
         if (w != w) nwn = order + 1ull;
         else if (w > mw) { mw = w; ow = order; }
       }
@@ -229,16 +230,17 @@ void launch_prepare(const DevGrid& d, Transport& tp, int nrk, float dtl, const f
   A.dtlr = Dtlr{{dtlr[0], dtlr[1], nrk > 2 ? dtlr[2] : 0.f}};
   A.ff = tp.ff.p; A.rhos = tp.rhos.p; A.red = tp.cfl_loc.p;
   A.list = tp.imp_list.p; A.count = tp.imp_count.p; A.b = tp.imp_b.p;
-  k_prepare<<<cdiv(d.nw_prog, 8), 256, 0, s>>>(A);
+  launch_next(k_prepare, cdiv(d.nw_prog, 8), 256, 0, s, A);
   OG_LAUNCHED();
 }
 
 // implicit vertical transport (scalar_transport_rk.F90:347-375) with
 // tridif_fini (tridiag_lib.f90:344-364); one thread per (column, tracer).
-__global__ void k_implicit_solve(GridK g, const int* __restrict__ list, const int* __restrict__ count,
-                                 const float* __restrict__ b, const float* __restrict__ ff,
-                                 const float* __restrict__ wmasc, const float* __restrict__ rhos_st,
+__global__ void k_implicit_solve(GridK g, const int* list, const int* count,
+                                 const float* b, const float* ff,
+                                 const float* wmasc, const float* rhos_st,
                                  int nrk, int istage, float dtr, CTView scp0, TView scp, int nt) {
+  grid_wait();
   const size_t all = (size_t)*count * nt;
   const int mza = g.mza;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < all; i += (size_t)gridDim.x * blockDim.x) {
@@ -282,7 +284,7 @@ void launch_implicit_solve(const DevGrid& d, const Transport& tp, int nrk, int i
   const size_t n = std::min<size_t>((size_t)d.nw_prog * nt, (size_t)128 * 16 * 148 * 4);
   size_t plane = (size_t)d.mwa * d.mza;
   const float* b = tp.imp_b.p + (size_t)(istage - 1) * d.mwa * 3 * d.mza;
-  k_implicit_solve<<<cdiv(n, 128), 128, 0, s>>>(gridk(d), tp.imp_list.p + (size_t)(istage - 1) * d.mwa,
+  launch_next(k_implicit_solve, cdiv(n, 128), 128, 0, s, gridk(d), tp.imp_list.p + (size_t)(istage - 1) * d.mwa,
                                                 tp.imp_count.p + (istage - 1), b, tp.ff.p, tp.wmasc.p,
                                                 tp.rhos.p + (size_t)(istage - 1) * plane, nrk, istage,
                                                 dtr, scp0, scp, nt);
