@@ -943,19 +943,21 @@ __global__ void k_prog_v(DynK g, const int* __restrict__ vprog, int nv, float dt
                          const float* rkx, const float* rky,
                          const float* rkz, const float* __restrict__ volvi,
                          const double* rho, float* vmc, float* vc) {
+  grid_wait();
   PK(j, kd, nv);
   const int iv = VPTAB(j);
   if (kd < LPV(iv)) return;
   const int mza = g.mza;
   const int iw1 = g.v_iw[iv * 2], iw2 = g.v_iw[iv * 2 + 1];
-  grid_wait();
   const size_t x = (size_t)iv * mza + kd, x1 = (size_t)iw1 * mza + kd, x2 = (size_t)iw2 * mza + kd;
+  // every load before the first store (the arrays may alias for the compiler)
+  const double rs = rho[x1] + rho[x2];
   const float pgf = (float)(press[x1] - press[x2]) * pvfac[x];
   const float v = vmc0[x] + dts * (vmt_short[x] + pgf +
                                    (vn[iv * 3] * (rkx[x1] + rkx[x2]) + vn[iv * 3 + 1] * (rky[x1] + rky[x2]) +
                                     vn[iv * 3 + 2] * (rkz[x1] + rkz[x2])) * volvi[x]);
   vmc[x] = v;
-  vc[x] = 2.0f * v / (float)(rho[x1] + rho[x2]);
+  vc[x] = 2.0f * v / (float)rs;
 }
 
 // Prognostic shaved-cell method (prog_wrtv_rk.f90:202-211): the momentum of
@@ -1006,6 +1008,7 @@ __global__ void __launch_bounds__(256) k_vel_t3d(DynK g, const int* __restrict__
                           const float* vc, const float* __restrict__ wno2,
                           const float4* __restrict__ ecv, float* vxe, float* vye,
                           float* vze, Shaved sh) {
+  grid_wait();
   WARP_POINT(nprog, 0u);
   const int mza = g.mza;
   const int iw = WTAB((int)w_), kb = LPW(iw), np = g.npoly[iw];
@@ -1018,7 +1021,6 @@ __global__ void __launch_bounds__(256) k_vel_t3d(DynK g, const int* __restrict__
   float4 ec[6];
 #pragma unroll
   for (int n = 0; n < 6; ++n) { e[n] = __ldg(E + 2 * n); ec[n] = __ldg(ecv + iw * 7 + n); }
-  grid_wait();
   float wl[R], wu[R], v[R][6];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
