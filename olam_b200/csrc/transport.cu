@@ -128,12 +128,12 @@ int tracers_to_host(cudaStream_t s) {
 static int grow(DevBuf<float>& b, size_t n) { return b.n >= n ? OLAMGPU_OK : b.alloc(n); }
 
 // Tracers (padded) up to which a stage runs as passes over cells: the tiled
-// kernel gives 8 lanes or more to a column whatever the count, and needs the
+// kernel gives 4 lanes or more to a column whatever the count, and needs the
 // step's weight records (128 B a cell).  Measured per stage, tiles and half
-// the records against cells: NXP=100, 60 levels, order 2: 4 tracers 1.26 /
-// 0.36 ms, 8: 1.26 / 0.66, 12: 1.27 / 0.97, 16: 1.27 / 1.28; NXP=47, 41
-// levels, order 3: 8: 0.22 / 0.16 ms, 12: 0.21 / 0.21, 16: 0.23 / 0.29.
-static int cell_ntp_max(int order) { return order == 2 ? 12 : 8; }
+// the records against cells: NXP=100, 60 levels, order 2: 4 tracers 0.82 /
+// 0.36 ms, 8: 0.82 / 0.66, 12: 0.82 / 0.97; NXP=47, 41 levels, order 3: 4:
+// 0.16 / 0.11 ms, 8: 0.16 / 0.16, 12: 0.16 / 0.21.
+static int cell_ntp_max(int order) { return order == 2 ? 8 : 4; }
 
 // scratch of the reference-mirroring passes for a group of nt tracers
 static int ensure_pass_scratch(Context& C, int nt, int order) {

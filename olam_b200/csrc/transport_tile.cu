@@ -220,8 +220,13 @@ int launch_tile_weights(const DevGrid& d, Transport& tp, const float* rhos, cuda
 // KS chunks run by different blocks (A.ks).
 // OFF: the type of element offsets into the batched arrays -- unsigned when
 // they all fit in 32 bits (fewer address instructions), else long long.
+// LPC = 4 (16 tracers, eight columns a warp, blocks of four warps): up to 16
+// tracers in 32-column tiles, whose eight-lane form leaves half its lanes
+// idle (1.07 -> 0.63 ms a stage at NXP=100, 60 levels, 16 tracers).  There the records are staged with the 128-byte swizzle
+// (16-byte chunk c of the row at address a goes to chunk c ^ (a >> 7 & 7)), so
+// that the eight columns of a warp read theirs from different banks.
 template <int NC, int LPC, typename OFF, bool SPLIT, int NW = TILE_NW>
-__global__ void __launch_bounds__(NW * 32, NW > TILE_NW ? 1 : (NC == 1 ? 3 : 2))
+__global__ void __launch_bounds__(NW * 32, NW > TILE_NW ? 1 : (NW < TILE_NW ? 6 : (NC == 1 ? 3 : 2)))
     k_tile(TileArgs A, const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmR) {
   extern __shared__ __align__(16) unsigned char smraw[];
   // every four-row gather's shared-memory destination on a 128-byte boundary
@@ -232,6 +237,7 @@ __global__ void __launch_bounds__(NW * 32, NW > TILE_NW ? 1 : (NC == 1 ? 3 : 2))
   constexpr int T = TW * NC;
   constexpr int G = 4 * LPC;                 // tracers of the block's group
   constexpr int RB = 4 * G;                  // bytes of a staged row
+  constexpr bool SWZ = LPC == 4;             // the records are swizzled
   // block order: tile, then level chunk, then tracer group (the groups of a
   // tile run side by side, so its records are read once from HBM)
   const int ngrp = A.ngrp, nks = SPLIT ? A.ks : 1;
@@ -361,10 +367,11 @@ __global__ void __launch_bounds__(NW * 32, NW > TILE_NW ? 1 : (NC == 1 ? 3 : 2))
       if (c >= nT) continue;
       // the column's window holds no level below its floor
       if (kd == kbc[n]) m2[n] = m1[n] = zero4();
-      const float* rc = Rc + c * TILE_WR;
-      const float4 r5 = reinterpret_cast<const float4*>(rc)[5];   // SW, volti/rhos, 1/rhos, D
-      const float4 r6 = reinterpret_cast<const float4*>(rc)[6];   // beta0 .. beta3
-      const float2 r7 = reinterpret_cast<const float2*>(rc)[14];  // beta4, omega
+      const float4* rc = reinterpret_cast<const float4*>(Rc + c * TILE_WR);
+      const int sw = SWZ ? (int)((smem_addr(rc) >> 7) & 7u) : 0;
+      const float4 r5 = rc[5 ^ sw];   // SW, volti/rhos, 1/rhos, D
+      const float4 r6 = rc[6 ^ sw];   // beta0 .. beta3
+      const float2 r7 = *reinterpret_cast<const float2*>(rc + (7 ^ sw));  // beta4, omega
       const float fx = FEX[c];
       const F4 s0 = lds4(Ul, c * RB);
       // horizontal: sum_j W_j S(slot j) + D S - SW S0
@@ -373,7 +380,7 @@ __global__ void __launch_bounds__(NW * 32, NW > TILE_NW ? 1 : (NC == 1 ? 3 : 2))
 #pragma unroll
       for (int q = 0; q < TILE_NS / 4; ++q) {
         const int4 so = reinterpret_cast<const int4*>(sl)[q];
-        const float4 w4 = reinterpret_cast<const float4*>(rc)[q];
+        const float4 w4 = rc[q ^ sw];
         // a slot whose weight is zero at this level (a face whose upwind
         // side does not reach it) is not read
         if (w4.x != 0.f) fd = fma4s(w4.x, lds4(Ul, so.x), fd);
@@ -737,7 +744,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
 
 // a 2-D map over nrows rows of width floats with boxes of one row of box
 // floats, for four-row gathers
-static int row_map(CUtensorMap* m, const float* base, int width, size_t nrows, int box) {
+static int row_map(CUtensorMap* m, const float* base, int width, size_t nrows, int box, bool swizzle = false) {
   auto enc = tmap_encoder();
   if (!enc) { set_error("cuTensorMapEncodeTiled is not available"); return OLAMGPU_E_CUDA; }
   const cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)nrows};
@@ -745,7 +752,8 @@ static int row_map(CUtensorMap* m, const float* base, int width, size_t nrows, i
   const cuuint32_t boxd[2] = {(cuuint32_t)box, 1};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, boxd, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")"); return OLAMGPU_E_CUDA; }
   return OLAMGPU_OK;
@@ -763,6 +771,7 @@ static TileKern tile_kernel_s(int T, int G, bool off32) {
   // 32-column tiles of 128 tracers: a block of 16 warps, one per SM
   if (T == 32 && G == 128) return off32 ? k_tile<2, 32, unsigned, SPLIT, 16> : k_tile<2, 32, long long, SPLIT, 16>;
   if (T == 32 && G == 64) return off32 ? k_tile<2, 16, unsigned, SPLIT> : k_tile<2, 16, long long, SPLIT>;
+  if (T == 32 && G == 16) return off32 ? k_tile<1, 4, unsigned, SPLIT, 4> : k_tile<1, 4, long long, SPLIT, 4>;
   if (T == 32 && G == 32) return off32 ? k_tile<1, 8, unsigned, SPLIT> : k_tile<1, 8, long long, SPLIT>;
   if (T == 16 && G == 64) return off32 ? k_tile<1, 16, unsigned, SPLIT> : k_tile<1, 16, long long, SPLIT>;
   if (T == 16 && G == 128) return off32 ? k_tile<2, 32, unsigned, SPLIT> : k_tile<2, 32, long long, SPLIT>;
@@ -771,7 +780,7 @@ static TileKern tile_kernel_s(int T, int G, bool off32) {
   return nullptr;
 }
 // threads of a shape's block
-static unsigned tile_threads(int T, int G) { return (T == 32 && G == 128) ? 512u : (unsigned)TILE_THREADS; }
+static unsigned tile_threads(int T, int G) { return (T == 32 && G == 128) ? 512u : (G == 16 ? 128u : (unsigned)TILE_THREADS); }
 // the kernel of a shape; the level sweep is split (KS > 1) only in its own instance
 static TileKern tile_kernel(int T, int G, bool off32, int KS = 1) {
   return KS > 1 ? tile_kernel_s<true>(T, G, off32) : tile_kernel_s<false>(T, G, off32);
@@ -801,7 +810,10 @@ int launch_tile_stage(const DevGrid& d, const Transport& tp, const float* S, con
     set_error("tile stage: the weight records of the step were not formed");
     return OLAMGPU_E_STATE;
   }
-  const int G = G_force > 0 ? G_force : d.tile_G;
+  int G = G_force > 0 ? G_force : d.tile_G;
+  // the 32-tracer shape with at most 16 tracers: four lanes a column
+  const bool narrow = d.tile_T == 32 && G == 32 && ntp <= 16;
+  if (narrow) G = 16;
   const int KS = std::max(1, d.tile_KS);
   TileArgs A;
   A.mza = d.mza; A.ntp = ntp; A.nrk = nrk; A.istage = istage; A.kb = 1; A.ks = KS;
@@ -848,7 +860,7 @@ int launch_tile_stage(const DevGrid& d, const Transport& tp, const float* S, con
   }
   alignas(64) CUtensorMap tmS, tmR;
   OG_CHECK(row_map(&tmS, S, ntp, (size_t)d.mwa * d.mza, G));
-  OG_CHECK(row_map(&tmR, tp.wrec.p, TILE_WR, (size_t)d.mwa * d.mza, TILE_WR));
+  OG_CHECK(row_map(&tmR, tp.wrec.p, TILE_WR, (size_t)d.mwa * d.mza, TILE_WR, narrow));
   OG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<nblk, tile_threads(d.tile_T, G), smem, s>>>(A, tmS, tmR);
   OG_LAUNCHED();
