@@ -46,7 +46,7 @@
 namespace olamgpu {
 
 struct WeightArgs {
-  int mza, T, kb, ntiles;
+  int mza, T, kb, ntiles, flat;     // flat: every floor is level 1
   const int* __restrict__ lpw;      // lowest prognosed device level of each W column
   const int* __restrict__ lpv;      // and of each V face
   const float* __restrict__ band;   // terrain bands' slot weights (TILE_AW each)
@@ -98,89 +98,107 @@ struct TileArgs {
 // so that a stage is
 //   scp = S0 + dtr / rhos sct + dtr volti / rhos (sum_j W_j S(slot j) + D S
 //         - SW S0 + fexpl (sum_q beta_q S(kd-2+q) + omega S0)).
-// Four tile columns per block of 256 threads, a thread per level.
+// A warp per tile column and 32 levels, a level per lane; the column's tables
+// are uniform or nearly uniform reads through L1, and the warp's 32 records, a
+// contiguous 4 KB, go through shared memory (rows padded to 144 bytes: no bank
+// conflicts either way) and out in whole lines.
+// Bound: HBM writes (128 B a cell; 780 MB at NXP=100, 60 levels, which a fill
+// writes in 111 us).  Four columns a block with their tables in shared memory
+// and each record stored from its thread took 385 us (a chain of dependent
+// reads in front of a block barrier, 16-byte stores 128 bytes apart), this 321.
+#define WEIGHT_ROW 36
 __global__ void __launch_bounds__(256) k_weights(WeightArgs A) {
-  __shared__ int wall[4][TILE_TCW];
-  __shared__ __align__(16) float amall[4][TILE_AW];
-  const int sub = threadIdx.x >> 6, lt = threadIdx.x & 63;
-  const size_t r = (size_t)blockIdx.x * 4 + sub;   // tile-column record
+  __shared__ __align__(16) float rows[8][32 * WEIGHT_ROW];
+  const int lane = threadIdx.x & 31, mza = A.mza;
+  const unsigned nch = ((unsigned)mza + 31u) / 32u;
+  const size_t w = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5), r = w / nch;   // tile-column record
+  const int k0 = 32 * (int)(w - r * nch);
   const int t = (int)(r / A.T), i = (int)(r - (size_t)t * A.T);
-  const bool live = t < A.ntiles && i < A.hdr[t].w;   // not padding of the last tile
-  int* w = wall[sub];
-  float* am = amall[sub];
-  if (live) {
-    for (int q = lt; q < TILE_TCW; q += 64) w[q] = __ldg(A.tc + r * TILE_TCW + q);
-    for (int q = lt; q < TILE_AW; q += 64) am[q] = __ldg(A.amat + r * TILE_AW + q);
+  if (t >= A.ntiles) return;
+  const int4* tc = reinterpret_cast<const int4*>(A.tc + r * TILE_TCW);
+  const int4 head = __ldg(tc), e0 = __ldg(tc + 6), e1 = __ldg(tc + 7), e2 = __ldg(tc + 8), bd = __ldg(tc + 9);
+  const int nT = __ldg(&A.hdr[t].w);
+  if (i >= nT) return;                                        // padding of the last tile
+  const int iw = head.x, side = head.y, np = head.z;
+  const int kb = A.flat ? A.kb : max(A.kb, __ldg(A.lpw + iw));   // the column's own floor
+  if (k0 + 32 <= kb) return;
+  const int boff = bd.x, nband = bd.y;
+  const int ev[6] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y};
+  const float dv[6] = {__int_as_float(e1.z), __int_as_float(e1.w), __int_as_float(e2.x),
+                       __int_as_float(e2.y), __int_as_float(e2.z), __int_as_float(e2.w)};
+  const int kd = min(max(k0 + lane, kb), mza - 1);            // lanes outside repeat an end level, not stored
+  const size_t x = (size_t)iw * mza + kd;
+  float vm[6];
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    vm[f] = 0.f;
+    if (f < np && (A.flat || kd >= __ldg(A.lpv + ev[f]))) vm[f] = __ldg(A.vmasc + (size_t)ev[f] * mza + kd);
   }
-  __syncthreads();
-  if (!live) return;
-  const int iw = w[TILE_TC_IW], np = w[TILE_TC_NP], side = w[TILE_TC_SIDE];
-  const int mza = A.mza, kb = max(A.kb, __ldg(A.lpw + iw));   // the column's own floor
-  const int nband = w[TILE_TC_NB], boff = w[TILE_TC_BOFF];
-  for (int kd = kb + lt; kd < mza; kd += 64) {
-    float dvvm[6];
-    int up[6];
-    float sw = 0.f;
+  const float wkm1 = __ldg(A.wmasc + x - 1), wk0 = __ldg(A.wmasc + x);
+  const float rh = __ldg(A.rhos + x), vt = __ldg(A.volti + x);
+  // the terrain band of level kd (bands end at increasing levels; past the
+  // last one every term is above ground)
+  int b = 0;
+  while (b < nband && kd >= __ldg(A.band_lev + boff + b)) ++b;
+  const float4* am = reinterpret_cast<const float4*>(b < nband ? A.band + (size_t)(boff + b) * TILE_AW : A.amat + r * TILE_AW);
+  float dvvm[6], sw = 0.f;
+  const float4* row[6];
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    dvvm[f] = dv[f] * vm[f];
+    // 1: the neighbour across face f is upwind
+    const int up = ((vm[f] < 0.f ? 1 : 0) != ((side >> f) & 1)) ? 1 : 0;
+    row[f] = am + (f * 2 + up) * (TILE_NS / 4);
+    sw = fmaf(dv[f], vm[f], sw);
+  }
+  float* own = rows[threadIdx.x >> 5];
+  float4* o = reinterpret_cast<float4*>(own + lane * WEIGHT_ROW);
+  float sumw = 0.f;
+  // four slots at a time (16-byte reads of the face rows of A)
+#pragma unroll
+  for (int q = 0; q < TILE_NS / 4; ++q) {
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int f = 0; f < 6; ++f) {
-      const int iv = w[TILE_TC_EV + f];
-      const float vm = (f < np && kd >= __ldg(A.lpv + iv)) ? __ldg(A.vmasc + (size_t)iv * mza + kd) : 0.f;
-      dvvm[f] = __int_as_float(w[TILE_TC_DV + f]) * vm;
-      // 1: the neighbour across face f is upwind
-      up[f] = ((vm < 0.f ? 1 : 0) != ((side >> f) & 1)) ? 1 : 0;
-      sw = fmaf(__int_as_float(w[TILE_TC_DV + f]), vm, sw);
+      const float4 a = __ldg(row[f] + q);
+      acc.x = fmaf(dvvm[f], a.x, acc.x);
+      acc.y = fmaf(dvvm[f], a.y, acc.y);
+      acc.z = fmaf(dvvm[f], a.z, acc.z);
+      acc.w = fmaf(dvvm[f], a.w, acc.w);
     }
-    const size_t x = (size_t)iw * mza + kd;
-    float* o = A.wrec + x * TILE_WR;
-    float sumw = 0.f;
-    // four slots at a time (16-byte reads of the face rows of A)
-    auto slot_weights = [&](const float4* am4) {
+    sumw += acc.x;
+    sumw += acc.y;
+    sumw += acc.z;
+    sumw += acc.w;
+    o[q] = acc;
+  }
+  // vertical faces: grad_z_quadratic at level lev from (lev-1, lev, lev+1),
+  // S(lev) + c1' (S(lev+1) - S(lev)) + c2' (S(lev) - S(lev-1)), the primes
+  // zeroing the differences across the column's ends
+  float beta[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+  auto face = [&](float wf, int lev, bool bot, int q0) {   // q0: beta index of S(lev-1)
+    const float c1 = lev <= mza - 2 ? __ldg(A.a_w + lev + (bot ? 0 : 2) * mza) : 0.f;
+    const float c2 = lev >= kb + 1 ? __ldg(A.a_w + lev + (bot ? 1 : 3) * mza) : 0.f;
+    beta[q0] -= wf * c2;
+    beta[q0 + 1] += wf * (1.f - c1 + c2);
+    beta[q0 + 2] += wf * c1;
+  };
+  if (kd == kb) beta[2] += wkm1;                   // scp_upw(kb-1) = scp(kb)
+  else if (wkm1 < 0.f) face(wkm1, kd, true, 1);    // scpb(kd) from (kd-1, kd, kd+1)
+  else face(wkm1, kd - 1, false, 0);               // scpt(kd-1) from (kd-2, kd-1, kd)
+  if (kd == mza - 1) beta[2] -= wk0;               // scp_upw(mza) = scp(mza)
+  else if (wk0 < 0.f) face(-wk0, kd + 1, true, 2); // scpb(kd+1) from (kd, kd+1, kd+2)
+  else face(-wk0, kd, false, 1);                   // scpt(kd) from (kd-1, kd, kd+1)
+  o[5] = make_float4(sw, vt / rh, 1.0f / rh, sw - sumw);
+  o[6] = make_float4(beta[0], beta[1], beta[2], beta[3]);
+  o[7] = make_float4(beta[4], wk0 - wkm1, wkm1, wk0);
+  __syncwarp();
+  float4* dst = reinterpret_cast<float4*>(A.wrec + ((size_t)iw * mza + k0) * TILE_WR);
 #pragma unroll
-      for (int q = 0; q < TILE_NS / 4; ++q) {
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int f = 0; f < 6; ++f) {
-          const float4 a = am4[(f * 2 + up[f]) * (TILE_NS / 4) + q];
-          acc.x = fmaf(dvvm[f], a.x, acc.x);
-          acc.y = fmaf(dvvm[f], a.y, acc.y);
-          acc.z = fmaf(dvvm[f], a.z, acc.z);
-          acc.w = fmaf(dvvm[f], a.w, acc.w);
-        }
-        sumw += acc.x;
-        sumw += acc.y;
-        sumw += acc.z;
-        sumw += acc.w;
-        reinterpret_cast<float4*>(o)[q] = acc;
-      }
-    };
-    // the terrain band of level kd (bands end at increasing levels; past
-    // the last one every term is above ground)
-    int b = 0;
-    while (b < nband && kd >= __ldg(A.band_lev + boff + b)) ++b;
-    if (b < nband) slot_weights(reinterpret_cast<const float4*>(A.band + (size_t)(boff + b) * TILE_AW));
-    else slot_weights(reinterpret_cast<const float4*>(am));
-    // vertical faces: grad_z_quadratic at level lev from (lev-1, lev, lev+1),
-    // S(lev) + c1' (S(lev+1) - S(lev)) + c2' (S(lev) - S(lev-1)), the primes
-    // zeroing the differences across the column's ends
-    float beta[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    auto face = [&](float wf, int lev, bool bot, int q0) {   // q0: beta index of S(lev-1)
-      const float c1 = lev <= mza - 2 ? __ldg(A.a_w + lev + (bot ? 0 : 2) * mza) : 0.f;
-      const float c2 = lev >= kb + 1 ? __ldg(A.a_w + lev + (bot ? 1 : 3) * mza) : 0.f;
-      beta[q0] -= wf * c2;
-      beta[q0 + 1] += wf * (1.f - c1 + c2);
-      beta[q0 + 2] += wf * c1;
-    };
-    const float wkm1 = __ldg(A.wmasc + x - 1), wk0 = __ldg(A.wmasc + x);
-    if (kd == kb) beta[2] += wkm1;                   // scp_upw(kb-1) = scp(kb)
-    else if (wkm1 < 0.f) face(wkm1, kd, true, 1);    // scpb(kd) from (kd-1, kd, kd+1)
-    else face(wkm1, kd - 1, false, 0);               // scpt(kd-1) from (kd-2, kd-1, kd)
-    if (kd == mza - 1) beta[2] -= wk0;               // scp_upw(mza) = scp(mza)
-    else if (wk0 < 0.f) face(-wk0, kd + 1, true, 2); // scpb(kd+1) from (kd, kd+1, kd+2)
-    else face(-wk0, kd, false, 1);                   // scpt(kd) from (kd-1, kd, kd+1)
-    const float rh = __ldg(A.rhos + x);
-    reinterpret_cast<float4*>(o)[5] = make_float4(sw, __ldg(A.volti + x) / rh, 1.0f / rh, sw - sumw);
-    reinterpret_cast<float4*>(o)[6] = make_float4(beta[0], beta[1], beta[2], beta[3]);
-    reinterpret_cast<float4*>(o)[7] = make_float4(beta[4], wk0 - wkm1, wkm1, wk0);
+  for (int p = 0; p < 8; ++p) {
+    const int rw = 4 * p + (lane >> 3), col = lane & 7;
+    if (k0 + rw >= kb && k0 + rw < mza)
+      dst[rw * (TILE_WR / 4) + col] = *reinterpret_cast<const float4*>(own + rw * WEIGHT_ROW + 4 * col);
   }
 }
 
@@ -201,7 +219,8 @@ int launch_tile_weights(const DevGrid& d, Transport& tp, const float* rhos, cuda
   W.wrec = tp.wrec.p;
   W.lpw = d.lpw.p; W.lpv = d.lpv.p;
   W.band = d.tile_band.p; W.band_lev = d.tile_band_lev.p;
-  k_weights<<<cdiv((size_t)d.ntiles * d.tile_T, 4), 256, 0, s>>>(W);
+  W.flat = tp.flat ? 1 : 0;
+  k_weights<<<cdiv((size_t)d.ntiles * d.tile_T * ((d.mza + 31) / 32), 8), 256, 0, s>>>(W);
   OG_LAUNCHED();
   // the paired kernel reads the pairs' records, formed from these
   if (d.tile_pairk && d.tile_paired && d.tile_T == 16) OG_CHECK(launch_pair_records(d, tp, s));
