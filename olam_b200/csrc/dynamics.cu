@@ -52,7 +52,7 @@ struct DynK {
   // flat: lpw = lpv = 2 everywhere (device level 1), no table read needed;
   // off_*: the loop table is the contiguous run off, off + 1, ... (a
   // global domain), no table read needed; -1 otherwise
-  int flat, off_w, off_vp, off_va;
+  int flat, off_w, off_vp, off_va, off_m;
 };
 
 // lowest device level of a W / V point; a loop table's j-th entry
@@ -60,6 +60,7 @@ struct DynK {
 #define LPV(i) (g.flat ? 1 : g.lpv[i])
 #define WTAB(j) (g.off_w >= 0 ? g.off_w + (j) : prog[j])
 #define VPTAB(j) (g.off_vp >= 0 ? g.off_vp + (j) : vprog[j])
+#define MTAB(j) (g.off_m >= 0 ? g.off_m + (j) : mprog[j])
 #define VATAB(j) (g.off_va >= 0 ? g.off_va + (j) : vadj[j])
 
 static DynK dynk(const DevGrid& d) {
@@ -71,6 +72,7 @@ static DynK dynk(const DevGrid& d) {
   k.edge = reinterpret_cast<const int4*>(d.edge.p);
   k.flat = ctx().tp.flat ? 1 : 0;
   k.off_w = d.off_wprog; k.off_vp = d.off_vprog; k.off_va = d.off_vwadj;
+  k.off_m = d.off_mprog;
   return k;
 }
 
@@ -246,7 +248,8 @@ __global__ void __launch_bounds__(256) k_damp_first(DynK g, DampArgs A) {
     }
   } else {
     WARP_POINT(A.nm, A.mblock);
-    const int im = A.mprog[w_];
+    const int* mprog = A.mprog;
+    const int im = MTAB((int)w_);
     int iv[3], lv[3];
     float f[3], x[R][3];
 #pragma unroll
@@ -315,7 +318,8 @@ __global__ void __launch_bounds__(256) k_damp_lap(DynK g, DampArgs A) {
     }
   } else {
     WARP_POINT(A.nm, A.mblock);
-    const int im = A.mprog[w_];
+    const int* mprog = A.mprog;
+    const int im = MTAB((int)w_);
     const size_t cb = (size_t)im * mza;
     int nb[3], lv[3];
     float c[3], s[R], x[R][3];
