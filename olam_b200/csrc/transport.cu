@@ -244,7 +244,13 @@ void transport_release_pipeline() {
   tp.ptab_t.release();
 }
 
-// The per-call step in tracer groups of 64 (one tile group each): the
+// Tracers per group of the per-call step: above 64 tracers one tile group of
+// 64, else 8, whose stages run as passes over cells -- the copies take ten
+// times as long as either, so what counts is how early the first result
+// leaves (NXP=60, 60 levels, 24 tracers: 23.2 -> 20.7 ms around the call).
+static int pipeline_group(int n) { return n > 64 ? 64 : 8; }
+
+// The per-call step in tracer groups (pipeline_group): the
 // host->device copies of a group's scp and sct (stream s_up), its gather
 // into the batched layout, its RK stages and its scatter back (the library
 // stream), and the device->host copies of its result (stream s_dn) are
@@ -258,7 +264,8 @@ static int pipelined_step(Context& C, const float* dtlr, const float* rhos_nrk) 
   cudaStream_t s = C.stream;
   const int nrk = C.opts.nrk_scal, ntp = tr.ntp, n = tr.n;
   const size_t npk = (size_t)d.mza * d.mwa, plane = npk * sizeof(float);
-  const int ngrp = (ntp + 63) / 64;
+  const int gw = pipeline_group(n), ngrp = (ntp + gw - 1) / gw;
+  const bool cells = gw < 64;
   if (!tp.s_up) OG_CUDA(cudaStreamCreateWithFlags(&tp.s_up, cudaStreamNonBlocking));
   if (!tp.s_dn) OG_CUDA(cudaStreamCreateWithFlags(&tp.s_dn, cudaStreamNonBlocking));
   while ((int)tp.ev.size() < 2 * ngrp + 1) {
@@ -277,8 +284,8 @@ static int pipelined_step(Context& C, const float* dtlr, const float* rhos_nrk) 
     OG_CUDA(cudaMemcpyAsync(tp.ptab_t.p, ht.data(), n * sizeof(float*), cudaMemcpyHostToDevice, s));
     OG_CUDA(cudaStreamSynchronize(s));   // the host vectors die here
   }
-  { OG_PROF("tile_weights", s); OG_CHECK(launch_tile_weights(d, tp, rhos_nrk, s)); }
-  if (tp.autotune && tp.tuned_ntp != ntp) {
+  if (!cells) { OG_PROF("tile_weights", s); OG_CHECK(launch_tile_weights(d, tp, rhos_nrk, s)); }
+  if (!cells && tp.autotune && tp.tuned_ntp != ntp) {
     // the shape on this step's inputs: the tracers' device copies and the
     // step's records (a rotation buffer as the scratch output)
     OG_CHECK(ensure_q(s));
@@ -301,7 +308,7 @@ static int pipelined_step(Context& C, const float* dtlr, const float* rhos_nrk) 
   const int fin = bout[nrk - 1];
   // copies in may start at once: the previous call has ended
   for (int g = 0; g < ngrp; ++g) {
-    const int tb = 64 * g, tc = std::min(64, n - tb), width = std::min(64, ntp - tb);
+    const int tb = gw * g, tc = std::min(gw, n - tb), width = std::min(gw, ntp - tb);
     if (tc <= 0) break;
     for (int i = tb; i < tb + tc; ++i) {
       OG_CUDA(cudaMemcpyAsync(tr.p[i].p, tr.h_p[i], plane, cudaMemcpyHostToDevice, tp.s_up));
@@ -318,13 +325,26 @@ static int pipelined_step(Context& C, const float* dtlr, const float* rhos_nrk) 
       float* OUT = tr.q[bout[istage - 1]].p;
       {
         OG_PROF(istage == 1 ? "tile_stage1" : "tile_stage", s);
-        OG_CHECK(launch_tile_stage(d, tp, IN, A, tr.qt.p, OUT, ntp, istage, nrk, dtr, C.status.p, s, g, 1, 64));
+        if (cells) {
+          CellStage c{};
+          c.S = IN + tb; c.S0 = A + tb; c.SCT = tr.qt.p + tb; c.out = OUT + tb;
+          c.ld = ntp; c.nt = width;
+          c.vmasc = tp.vmasc.p; c.wmasc = tp.wmasc.p; c.rhos = rhos_nrk; c.ff = tp.ff.p;
+          c.face = tp.upv.p;
+          c.istage = istage; c.nrk = nrk; c.dtr = dtr;
+          OG_CHECK(launch_cell_stage(d, C.opts.scal_horiz_adv_order, c, s));
+        } else {
+          OG_CHECK(launch_tile_stage(d, tp, IN, A, tr.qt.p, OUT, ntp, istage, nrk, dtr, C.status.p, s, g, 1, 64));
+        }
       }
       {
         OG_PROF("implicit_solve", s);
         launch_implicit_solve(d, tp, nrk, istage, dtr, CTView{A, ntp, tb}, TView{OUT, ntp, tb}, width, s);
       }
     }
+    // points outside jtw_prog keep their values (a later group's own are
+    // copied again when it has them)
+    launch_copy_cols(d.w_nonprog.p, d.n_nonprog, A, tr.q[fin].p, (size_t)d.mza * ntp, s);
     launch_scatter_q_range(tr.q[fin].p + tb, tp.ptab_p.p + tb, tc, width, ntp, npk, s);
     OG_CUDA(cudaEventRecord(tp.ev[2 * g + 1], s));
     OG_CUDA(cudaStreamWaitEvent(tp.s_dn, tp.ev[2 * g + 1], 0));
@@ -378,11 +398,20 @@ int transport_run(const float* rho_old_host, olamgpu_cfl_diag* diag) {
     OG_CHECK(build_fused_weights(&C.hgrid, C.g, order, s));
 
   // per-call step (SYNC_EACH_CALL) of the tiled, unlimited step on a global
-  // domain: the tracers go through in groups of 64 so that the copies in,
-  // the step and the copies out of different groups overlap
-  const bool pipelined = C.coherence == OLAMGPU_SYNC_EACH_CALL && tiled && C.opts.iscal_monot == 0 &&
-                         !tp.have_turb && !C.halo.on && d.n_nonprog == 0 && tr.n > 64 &&
-                         tile_shape_fits(d, 64);   // its groups are 64 tracers wide
+  // domain: the tracers go through in groups so that the copies in, the step
+  // and the copies out of different groups overlap
+  bool pipelined = C.coherence == OLAMGPU_SYNC_EACH_CALL && tiled && C.opts.iscal_monot == 0 && !tp.have_turb &&
+                   !C.halo.on;
+  if (tr.n > 64) {
+    pipelined = pipelined && tile_shape_fits(d, 64);   // its groups are 64 tracers wide
+  } else {
+    // groups of cell passes; a forced shape keeps the tiles
+    pipelined = pipelined && tr.n > pipeline_group(tr.n) && tp.autotune && cell_stage_available(d, order);
+    if (pipelined && grow(tp.upv, (size_t)mva * mza * pipeline_group(tr.n)) != OLAMGPU_OK) {
+      cudaGetLastError();   // no room for the face values
+      pipelined = false;
+    }
+  }
   float dtlr[3];
   OG_CHECK(transport_prepare(C, rho_old_host, !pipelined, dtlr));
   const float* rhos_nrk = tp.rhos.p + (size_t)(nrk - 1) * wz;

@@ -1,0 +1,107 @@
+"""GPU parity, against the FP64 oracle, of the paths chosen by tracer count and
+level count: stages as passes over cells (few tracers, the limited last stage
+with tracers of both modes in a quad), the narrow form of the tiled stage (up
+to 16 tracers), the grouped per-call step, and the acoustic step's kernels at
+the level counts where a lane's or a column's share changes (32, 33, 64, 65
+levels).
+
+Tolerances are the repository's: 1e-5 normwise for the transport and the
+thermodynamic fields, five times the oracle's own FP32-FP64 spread (at least
+1e-5) for the momentum fields."""
+import numpy as np
+import pytest
+
+import oracle_lib
+from conftest import relerr, small_case
+from olam_b200 import abi
+from olam_b200.lib import HostState, OlamGpu
+from test_dynamics_gpu import check_fields, dyn_case, gpu_long_steps, oracle_long_steps
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+
+def case(nlev, ntr, w_amp, terrain):
+    g, st = small_case(nxp=5, nlev=nlev, ntr=ntr, w_amp=w_amp, seed=23)
+    if terrain:
+        from olam_b200.synth.grid import with_terrain
+        g = with_terrain(g, terrain)
+    return g, st
+
+
+def run(g, st, opts, pdef=None, coherence=abi.RESIDENT, steps=1):
+    dev = OlamGpu(abi.FortranGrid(g), opts, HostState(vmasc=st.vmasc, wmasc=st.wmasc, rho=st.rho, wc=st.wc))
+    try:
+        dev.set_coherence(coherence)
+        rng = np.random.default_rng(3)
+        var_p = [t.copy() for t in st.tracers]
+        var_t = [(1e-6 * t * rng.standard_normal((t.shape[0], 1))).astype(np.float32) for t in st.tracers]
+        sct = [t.copy() for t in var_t]
+        dev.register_scalars(var_p, var_t, pdef=pdef)
+        for _ in range(steps):
+            dev.scalar_transport_rk(st.rho_old)
+        if coherence == abi.RESIDENT:
+            dev.sync_to_host(abi.F_SCALARS)
+        return np.stack(var_p), sct
+    finally:
+        dev.close()
+
+
+def check(out, ref):
+    for n in range(len(ref)):
+        assert relerr(out[n][1:], ref[n][1:]) < TOL, (n, relerr(out[n][1:], ref[n][1:]))
+
+
+# one tracer, a whole quad, a quad and one, the last counts of the cell passes
+# and the first and last of the narrow tiles; levels below, at and above a
+# warp's 32; w_amp 3: vertical CFL above 1, so implicit columns
+@pytest.mark.parametrize("ntr,nlev,order,nrk,w_amp,terrain", [
+    (1, 12, 2, 2, 0.05, 0), (1, 31, 3, 3, 3.0, 0), (4, 32, 2, 3, 0.05, 3), (5, 33, 3, 2, 0.05, 3),
+    (8, 12, 2, 2, 3.0, 3), (9, 12, 2, 2, 0.05, 0), (16, 33, 3, 3, 0.05, 3), (17, 12, 2, 2, 0.05, 0)])
+def test_stage_by_tracer_count(ntr, nlev, order, nrk, w_amp, terrain):
+    g, st = case(nlev, ntr, w_amp, terrain)
+    opts = abi.make_opts(1800.0, nrk_scal=nrk, scal_order=order)
+    out, sct = run(g, st, opts)
+    check(out, oracle_lib.scalar_transport(abi.FortranGrid(g), opts, st.tracers, sct, st, fp64=True))
+
+
+# limited and unlimited tracers in one quad (pdef), ragged counts, implicit
+# columns, terrain
+@pytest.mark.parametrize("monot,ntr,order,w_amp,terrain", [
+    (2, 1, 2, 0.05, 0), (2, 6, 3, 3.0, 0), (2, 5, 2, 0.05, 3), (1, 3, 2, 3.0, 0), (1, 9, 3, 0.05, 3)])
+def test_limited_stage(monot, ntr, order, w_amp, terrain):
+    g, st = case(33, ntr, w_amp, terrain)
+    pdef = [1 if n % 3 else 0 for n in range(ntr)] if monot == 2 and ntr > 1 else [1] * ntr
+    opts = abi.make_opts(1800.0, scal_order=order, iscal_monot=monot)
+    out, sct = run(g, st, opts, pdef=pdef)
+    ref = [oracle_lib.scalar_transport(abi.FortranGrid(g), abi.make_opts(1800.0, scal_order=order,
+                                                                         iscal_monot=monot if p or monot == 1 else 0),
+                                       [t], [s], st, fp64=True)[0]
+           for t, s, p in zip(st.tracers, sct, pdef)]
+    check(out, ref)
+
+
+# the per-call step in groups: the first count above a group, a ragged last
+# group, and the last count before the wide groups
+@pytest.mark.parametrize("ntr,order,w_amp", [(9, 2, 0.05), (21, 3, 3.0), (64, 2, 0.05)])
+def test_per_call_groups(ntr, order, w_amp):
+    g, st = case(12, ntr, w_amp, 0)
+    opts = abi.make_opts(1800.0, scal_order=order)
+    out, sct = run(g, st, opts, coherence=abi.SYNC_EACH_CALL)
+    check(out, oracle_lib.scalar_transport(abi.FortranGrid(g), opts, st.tracers, sct, st, fp64=True))
+
+
+# mza = nlev + 1 at the sizes where the rows per lane and the warps per column
+# change, with and without the column kernel's folded set-up
+@pytest.mark.parametrize("nlev,kw", [(31, {}), (32, {}), (63, {}), (64, {}), (32, dict(ithil_monot=1))])
+def test_acoustic_step_by_level_count(nlev, kw):
+    g, ds = dyn_case(nxp=4, nlev=nlev, seed=8)
+    fg = abi.FortranGrid(g)
+    assert g.mza == nlev + 1
+    opts = abi.make_opts(300.0, nacoust=4, **kw)
+    arrays = oracle_lib.dyn_arrays(g, ds)
+    o64, _ = oracle_long_steps(fg, opts, arrays, 1, True)
+    o32, _ = oracle_long_steps(fg, opts, arrays, 1, False)
+    hs, _ = gpu_long_steps(fg, opts, arrays, 1, abi.SYNC_EACH_CALL)
+    check_fields(hs, o32, o64)
