@@ -52,7 +52,7 @@ struct DynK {
   // flat: lpw = lpv = 2 everywhere (device level 1), no table read needed;
   // off_*: the loop table is the contiguous run off, off + 1, ... (a
   // global domain), no table read needed; -1 otherwise
-  int flat, off_w, off_vp, off_va, off_m;
+  int flat, off_w, off_vp, off_va;
 };
 
 // lowest device level of a W / V point; a loop table's j-th entry
@@ -60,7 +60,6 @@ struct DynK {
 #define LPV(i) (g.flat ? 1 : g.lpv[i])
 #define WTAB(j) (g.off_w >= 0 ? g.off_w + (j) : prog[j])
 #define VPTAB(j) (g.off_vp >= 0 ? g.off_vp + (j) : vprog[j])
-#define MTAB(j) (g.off_m >= 0 ? g.off_m + (j) : mprog[j])
 #define VATAB(j) (g.off_va >= 0 ? g.off_va + (j) : vadj[j])
 
 static DynK dynk(const DevGrid& d) {
@@ -72,7 +71,6 @@ static DynK dynk(const DevGrid& d) {
   k.edge = reinterpret_cast<const int4*>(d.edge.p);
   k.flat = ctx().tp.flat ? 1 : 0;
   k.off_w = d.off_wprog; k.off_vp = d.off_vprog; k.off_va = d.off_vwadj;
-  k.off_m = d.off_mprog;
   return k;
 }
 
@@ -191,7 +189,7 @@ __global__ void k_vort_first_v(DynK g, const int* __restrict__ vprog, int nv, co
 
 struct DampArgs {
   const int* wprog; int nw;           // divergence of the W columns
-  const int* mprog; int nm;           // vorticity at the M points
+  const int* mprog; int nm, off_m;    // vorticity at the M points (off_m: the table is off_m, off_m + 1, ..., or -1)
   unsigned mblock;                    // first block of the M part
   const float* arv; const float* vmc; const float* vc;
   const float* xx_yy; const float* xx_yy_m; const float* vfact;
@@ -248,8 +246,7 @@ __global__ void __launch_bounds__(256) k_damp_first(DynK g, DampArgs A) {
     }
   } else {
     WARP_POINT(A.nm, A.mblock);
-    const int* mprog = A.mprog;
-    const int im = MTAB((int)w_);
+    const int im = A.off_m >= 0 ? A.off_m + (int)w_ : A.mprog[w_];
     int iv[3], lv[3];
     float f[3], x[R][3];
 #pragma unroll
@@ -318,8 +315,7 @@ __global__ void __launch_bounds__(256) k_damp_lap(DynK g, DampArgs A) {
     }
   } else {
     WARP_POINT(A.nm, A.mblock);
-    const int* mprog = A.mprog;
-    const int im = MTAB((int)w_);
+    const int im = A.off_m >= 0 ? A.off_m + (int)w_ : A.mprog[w_];
     const size_t cb = (size_t)im * mza;
     int nb[3], lv[3];
     float c[3], s[R], x[R][3];
@@ -1383,7 +1379,7 @@ static int v_tendency(Context& C, bool div, bool vor, bool setup, const float* s
   // the planes each Laplacian step reads and writes: 1 -> 2 -> 1 ...
   auto plane = [](float* p, size_t n, int i) { return p + (size_t)(i - 1) * n; };
   DampArgs A;
-  A.wprog = d.jtw_prog.p; A.mprog = d.jtm_prog.p;
+  A.wprog = d.jtw_prog.p; A.mprog = d.jtm_prog.p; A.off_m = d.off_mprog;
   A.arv = y.arv.p; A.vmc = y.vmc.p; A.vc = y.vc.p;
   A.xx_yy = y.xx_yy.p; A.xx_yy_m = y.xx_yy_m.p; A.vfact = y.vfact.p;
   auto run = [&](int step, bool dw, bool dm) -> int {   // step 0: the first planes
