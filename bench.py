@@ -185,15 +185,18 @@ def make_case(a):
 
 
 def acoustic_bytes(g):
-    """Bytes each acoustic-step launch must move at least (every array
-    element it reads or writes once; stage-averaged for wrt_begs over the 3
-    RK stages), per kernel scope."""
+    """Bytes each acoustic-step scope must move at least (every array element
+    it reads or writes once, averaged over the 3 RK stages where a stage
+    differs), without eddy, Rayleigh or flux-corrected terms and with both
+    dampings at level 3.  v_tendency holds four launches: the first planes,
+    two Laplacian steps and the V tendency."""
     cw = prognostic_cells(g)                                            # above-ground W and V cells
     cv = int((g.mza + 1 - g.lpv[1:].astype(np.int64)).sum())
+    cm = (g.mma - 1) * (g.mza - 1)                                      # cells at M points
     return {
-        "setup_w": 76 * cw, "setup_v": 16 * cv, "vmca": 20 * cv, "upw4": 36 * cw,
-        "grad_upv4": 16 * cw + 20 * cv, "wrt_begs": (136 + 16 / 3) * cw + 24 * cv, "prog_v": 24 * cv + 28 * cw,
-        "vel_t3d": 16 * cw + 4 * cv,
+        "v_tendency": (12 + 2 * 8 + 12) * cw + (4 + 2 * 8 + 8) * cm + (12 + 20) * cv,
+        "grad_upv4": 16 * cw + (28 + 8 / 3) * cv, "wrt_begs": (136 + 8 / 3) * cw + 20 * cv,
+        "prog_v": 24 * cv + 28 * cw, "vel_t3d": 16 * cw + 4 * cv,
     }
 
 

@@ -2,22 +2,27 @@
 // device (omodel/prog_wrtv_rk.f90:36-488, omodel/timestep.f90:430-612).
 //
 // Kernel per reference routine, each over the reference's loop table:
-//   k_setup_w / k_setup_v   column set-up and Rayleigh terms   (prog_wrtv_rk.f90:166-303)
-//   k_div_* / k_lap_w       divh_damp                          (vort_div_damp.f90:1-230)
-//   k_vort_* / k_lap_m      vort_damp                          (vort_div_damp.f90:234-445)
-//   k_vmca                  vmca and vmasc on the last stage   (prog_wrtv_rk.f90:320-368); the
-//                           stage copies *_rk = *_short and vmca of the other stages are
-//                           formed inside k_wrt_begs
-//   k_upw4, k_grad_upv4     fluxes_wrtv for thil, vxe, vye, vze (:950-1129), the four
-//                           fields of one stage in one launch each (the
-//                           gradients and the V-face values in one pass over
-//                           the W cells); on the last stage the fields with
-//                           ithil_monot / iwind_monot > 0 take
+//   k_damp_first, k_damp_lap  divh_damp and vort_damp          (vort_div_damp.f90:1-445):
+//                           the two first passes in one launch, the two
+//                           Laplacians of a step in one
+//   k_vtend                 the V points' set-up and Rayleigh terms with both dampings
+//                           (prog_wrtv_rk.f90:166-303)
+//   k_setup_w               the W columns' set-up (same lines); on the lean path
+//                           k_wrt_begs forms it on the first stage
+//   k_grad_upv4             fluxes_wrtv for thil, vxe, vye, vze (:950-1129), the four
+//                           fields of one stage in one launch: the gradients
+//                           and the V-face values in one pass over the W
+//                           cells, with vmca of the stage and its share of
+//                           vmasc (:320-368); on the last stage the fields
+//                           with ithil_monot / iwind_monot > 0 take
 //                           dynamics_monot.cu's values
-//   k_wrt_begs              prog_wrt_begs (:494-884): one warp per column, lanes over
-//                           levels for the explicit terms and for the
-//                           tridiagonal solve (tridiffo, tridiag_lib.f90:10-36,
-//                           by parallel cyclic reduction)
+//   k_vmca                  vmca / vmasc on a rank with a halo
+//   k_upw4                  the vertical face values where the column kernel does not
+//                           form them (eddy, Rayleigh or flux-corrected terms)
+//   k_wrt_begs              prog_wrt_begs (:494-884): lanes over levels for the explicit
+//                           terms and for the tridiagonal solve (tridiffo,
+//                           tridiag_lib.f90:10-36, by parallel cyclic
+//                           reduction), one or two warps per column
 //   k_prog_v                prog_v_begs (:888-946)
 //   k_vel_t3d               vel_t3d_hex (vel_t3d.f90:39-108)
 // With eddy diffusion registered, dynamics_eddy.cu's k_eddy_w follows

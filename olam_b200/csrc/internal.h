@@ -358,7 +358,9 @@ struct Dyn {
   DevBuf<float> wmc0, vmc0, vmca;
   DevBuf<float> sh_th, sh_vx, sh_vy, sh_vz, sh_vmt;    // *_short
   DevBuf<float> rk_vx, rk_vy, rk_vz;                   // *_rk (thilt_rk stays in registers)
-  DevBuf<float> upw, upv;        // 4 fields: thil, vxe, vye, vze
+  // 4 fields thil, vxe, vye, vze: upv with the field fastest (one 16-byte
+  // word per V point and level); upw field by field
+  DevBuf<float> upw, upv;
   DevBuf<float> div2d, fdivh, vort2d, fvorth, fvortl, vfact;
   DevBuf<int> lpmmin;
   // prognostic shaved-cell method: lve2 of every W column and the start

@@ -1,12 +1,14 @@
 // transport.cu -- scalar_transport_rk driver (omodel/scalar_transport_rk.F90:30-385).
 //
 // Call sequence per long step, all on the library stream:
-//   check_cfls -> ff_implic and the CFL maxima           (:113)
-//   rhos(:,:,1..nrk)                                     (:117-152)
-//   implicit-column factorisation per stage             (:164-217)
+//   launch_prepare: check_cfls -> ff_implic and the CFL maxima (:113),
+//   rhos(:,:,1..nrk) (:117-152) and the implicit columns' factors per stage
+//   (:164-217), one launch
 //   per RK stage: update of every tracer, then the implicit vertical solve
-// The fused form updates all tracers of a stage in one launch on the batched
-// layout; the plain form runs the reference's passes tracer by tracer.
+// Three forms of a stage: on the batched layout either one tiled launch for
+// all tracers (transport_tile.cu) or, for few tracers and for a limited last
+// stage, the cell passes (transport_cell.cu); the plain form runs the
+// reference's passes tracer by tracer.
 // Stage outputs rotate through three buffers (scp0 stays intact), so no
 // stage writes a field another thread of the same launch still reads.
 #include <algorithm>
@@ -165,7 +167,7 @@ static void passes_stage(Context& C, CTView in, CTView scp0, CTView sct, TView o
     launch_wcol(d, C.tp, in, scp0, sct, rhos, out, nt, istage, nrk, dtr, mode, limited_stage, s);
   } else {
     OG_PROF("pass_wcol", s);
-    launch_wcell(d, C.tp, in, scp0, sct, rhos, out, nt, istage, nrk, dtr, s);
+    launch_wcell(d, C.tp, in, scp0, sct, rhos, out, istage, nrk, dtr, s);
   }
   if (limited_stage) {
     { OG_PROF("pass_vapply", s); launch_vapply(d, C.tp, nt, mode, s); }
