@@ -239,24 +239,39 @@ int launch_tile_weights(const DevGrid& d, Transport& tp, const float* rhos, cuda
 // KS chunks run by different blocks (A.ks).
 // OFF: the type of element offsets into the batched arrays -- unsigned when
 // they all fit in 32 bits (fewer address instructions), else long long.
-// LPC = 4 (16 tracers, eight columns a warp, blocks of four warps): up to 16
-// tracers in 32-column tiles, whose eight-lane form leaves half its lanes
-// idle (1.07 -> 0.63 ms a stage at NXP=100, 60 levels, 16 tracers).  There the records are staged with the 128-byte swizzle
-// (16-byte chunk c of the row at address a goes to chunk c ^ (a >> 7 & 7)), so
-// that the eight columns of a warp read theirs from different banks.
+// Up to 16 tracers (LPC = 4, eight columns a warp, four warps) and 40 or 48
+// tracers (LPC = 10, 12) run 32-column tiles with a lane group per column
+// laid over the block's threads in turn, LPC warps a block, so that no lane
+// is idle.  us a stage, before (the fastest other shape) and now:
+//   tracers       16           40           48           80
+//   NXP=100    1070 / 631   1840 / 1380  1840 / 1655  3240 / 2680
+//   NXP=47                   328 / 250    328 / 290    533 / 444
+// (60 levels order 2; 41 levels order 3 with terrain.)  24 tracers (LPC = 6)
+// took 985 against 1070 and 214 against 191, 56 (LPC = 14) 1893 against 1848:
+// left out.  There a warp's lanes read the records of several columns at
+// once, so these are staged with the 128-byte swizzle (16-byte chunk c of the
+// row at address a goes to chunk c ^ (a >> 7 & 7)): from different banks
+// (40 tracers without it 1425 and 278 us).
+#define TILE_SWIZZLED(G) ((G) == 16 || (G) == 40 || (G) == 48)
+// two blocks an SM of 10 or 12 warps: three in 64 registers 1557 us for 40 tracers at NXP=100
+constexpr int tile_blocks(int NC, int LPC, int NW) {
+  if (LPC == 4) return 6;
+  if (LPC == 10 || LPC == 12) return 2;
+  return NW > TILE_NW ? 1 : (NC == 1 ? 3 : 2);
+}
+
 template <int NC, int LPC, typename OFF, bool SPLIT, int NW = TILE_NW>
-__global__ void __launch_bounds__(NW * 32, NW > TILE_NW ? 1 : (NW < TILE_NW ? 6 : (NC == 1 ? 3 : 2)))
+__global__ void __launch_bounds__(NW * 32, tile_blocks(NC, LPC, NW))
     k_tile(TileArgs A, const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmR) {
   extern __shared__ __align__(16) unsigned char smraw[];
   // every four-row gather's shared-memory destination on a 128-byte boundary
   static_assert((4 * TILE_WR * 4) % 128 == 0 && (4 * 4 * 4 * LPC) % 128 == 0, "gather destinations");
   constexpr int NT = NW * 32;                // threads of the block
-  constexpr int CPW = 32 / LPC;              // columns a warp serves at once
-  constexpr int TW = NW * CPW;               // columns a block serves at once
+  constexpr int TW = NT / LPC;               // columns a block serves at once
   constexpr int T = TW * NC;
   constexpr int G = 4 * LPC;                 // tracers of the block's group
   constexpr int RB = 4 * G;                  // bytes of a staged row
-  constexpr bool SWZ = LPC == 4;             // the records are swizzled
+  constexpr bool SWZ = TILE_SWIZZLED(G);     // the records are swizzled
   // block order: tile, then level chunk, then tracer group (the groups of a
   // tile run side by side, so its records are read once from HBM)
   const int ngrp = A.ngrp, nks = SPLIT ? A.ks : 1;
@@ -345,9 +360,8 @@ __global__ void __launch_bounds__(NW * 32, NW > TILE_NW ? 1 : (NW < TILE_NW ? 6 
   // LPC lanes per column (columns cb, cb + TW, ...): lane hl of the group
   // holds tracers t0 + 4 hl .. + 3; the column's rows kd-2, kd-1, kd+1,
   // kd+2, kd+3 (read ahead) and its scp0 / sct rows at kd stay in registers
-  const int sub = lane / LPC, hl = lane - sub * LPC;
+  const int cb = tid / LPC, hl = tid - cb * LPC;
   const bool act = 4 * hl < seg;
-  const int cb = CPW * warp + sub;
   F4 m2[NC], m1[NC], p1[NC], p2[NC], p3[NC], s00[NC], st[NC];
   OFF cbase[NC];
   int kbc[NC];   // each column's own floor (lpw): levels below it are not prognosed
@@ -790,6 +804,8 @@ static TileKern tile_kernel_s(int T, int G, bool off32) {
   // 32-column tiles of 128 tracers: a block of 16 warps, one per SM
   if (T == 32 && G == 128) return off32 ? k_tile<2, 32, unsigned, SPLIT, 16> : k_tile<2, 32, long long, SPLIT, 16>;
   if (T == 32 && G == 64) return off32 ? k_tile<2, 16, unsigned, SPLIT> : k_tile<2, 16, long long, SPLIT>;
+  if (!SPLIT && T == 32 && G == 40) return off32 ? k_tile<1, 10, unsigned, false, 10> : k_tile<1, 10, long long, false, 10>;
+  if (!SPLIT && T == 32 && G == 48) return off32 ? k_tile<1, 12, unsigned, false, 12> : k_tile<1, 12, long long, false, 12>;
   if (T == 32 && G == 16) return off32 ? k_tile<1, 4, unsigned, SPLIT, 4> : k_tile<1, 4, long long, SPLIT, 4>;
   if (T == 32 && G == 32) return off32 ? k_tile<1, 8, unsigned, SPLIT> : k_tile<1, 8, long long, SPLIT>;
   if (T == 16 && G == 64) return off32 ? k_tile<1, 16, unsigned, SPLIT> : k_tile<1, 16, long long, SPLIT>;
@@ -799,7 +815,7 @@ static TileKern tile_kernel_s(int T, int G, bool off32) {
   return nullptr;
 }
 // threads of a shape's block
-static unsigned tile_threads(int T, int G) { return (T == 32 && G == 128) ? 512u : (G == 16 ? 128u : (unsigned)TILE_THREADS); }
+static unsigned tile_threads(int T, int G) { return T == 32 && G == 128 ? 512u : (G < 64 ? 8u * (unsigned)G : (unsigned)TILE_THREADS); }
 // the kernel of a shape; the level sweep is split (KS > 1) only in its own instance
 static TileKern tile_kernel(int T, int G, bool off32, int KS = 1) {
   return KS > 1 ? tile_kernel_s<true>(T, G, off32) : tile_kernel_s<false>(T, G, off32);
@@ -822,6 +838,20 @@ bool tile_shape_fits(const DevGrid& d, int G) {
   return tile_kernel(d.tile_T, G, true) && tile_smem_bytes(d.tile_T, d.tile_nu_max, 4 * G) <= TILE_SMEM_LIMIT;
 }
 
+// The 32-tracer shape of 32-column tiles: its group of 16 (up to 16 tracers),
+// 32, 40 or 48 tracers, whichever gives the blocks the fewest warps in all (a
+// quarter of the group's tracers each), 32 where that is among them.  The
+// wider groups have no form with split levels.
+static int tile_group(const DevGrid& d, int ntp, int KS) {
+  if (ntp <= 16) return 16;
+  int best = 32;
+  for (int G = 48; KS == 1 && G >= 40; G -= 8)
+    if (G * ((ntp + G - 1) / G) < best * ((ntp + best - 1) / best) &&
+        tile_smem_bytes(32, d.tile_nu_max, 4 * G) <= TILE_SMEM_LIMIT)
+      best = G;
+  return best;
+}
+
 int launch_tile_stage(const DevGrid& d, const Transport& tp, const float* S, const float* S0,
                       const float* SCT, float* OUT, int ntp, int istage, int nrk, float dtr, int* status,
                       cudaStream_t s, int grp0, int ngrp_run, int G_force) {
@@ -830,10 +860,8 @@ int launch_tile_stage(const DevGrid& d, const Transport& tp, const float* S, con
     return OLAMGPU_E_STATE;
   }
   int G = G_force > 0 ? G_force : d.tile_G;
-  // the 32-tracer shape with at most 16 tracers: four lanes a column
-  const bool narrow = d.tile_T == 32 && G == 32 && ntp <= 16;
-  if (narrow) G = 16;
   const int KS = std::max(1, d.tile_KS);
+  if (d.tile_T == 32 && G == 32 && (ngrp_run <= 0 || ntp <= 16)) G = tile_group(d, ntp, KS);
   TileArgs A;
   A.mza = d.mza; A.ntp = ntp; A.nrk = nrk; A.istage = istage; A.kb = 1; A.ks = KS;
   A.ntiles = d.ntiles; A.T = d.tile_T; A.nu_max = d.tile_nu_max; A.mwa = d.mwa;
@@ -879,7 +907,7 @@ int launch_tile_stage(const DevGrid& d, const Transport& tp, const float* S, con
   }
   alignas(64) CUtensorMap tmS, tmR;
   OG_CHECK(row_map(&tmS, S, ntp, (size_t)d.mwa * d.mza, G));
-  OG_CHECK(row_map(&tmR, tp.wrec.p, TILE_WR, (size_t)d.mwa * d.mza, TILE_WR, narrow));
+  OG_CHECK(row_map(&tmR, tp.wrec.p, TILE_WR, (size_t)d.mwa * d.mza, TILE_WR, TILE_SWIZZLED(G)));
   OG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<nblk, tile_threads(d.tile_T, G), smem, s>>>(A, tmS, tmR);
   OG_LAUNCHED();

@@ -30,7 +30,7 @@ def case(nlev, ntr, w_amp, terrain):
     return g, st
 
 
-def run(g, st, opts, pdef=None, coherence=abi.RESIDENT, steps=1):
+def run(g, st, opts, pdef=None, coherence=abi.RESIDENT, steps=1, shape=None):
     dev = OlamGpu(abi.FortranGrid(g), opts, HostState(vmasc=st.vmasc, wmasc=st.wmasc, rho=st.rho, wc=st.wc))
     try:
         dev.set_coherence(coherence)
@@ -39,6 +39,8 @@ def run(g, st, opts, pdef=None, coherence=abi.RESIDENT, steps=1):
         var_t = [(1e-6 * t * rng.standard_normal((t.shape[0], 1))).astype(np.float32) for t in st.tracers]
         sct = [t.copy() for t in var_t]
         dev.register_scalars(var_p, var_t, pdef=pdef)
+        if shape:
+            dev.set_tile_shape(*shape)
         for _ in range(steps):
             dev.scalar_transport_rk(st.rho_old)
         if coherence == abi.RESIDENT:
@@ -63,6 +65,19 @@ def test_stage_by_tracer_count(ntr, nlev, order, nrk, w_amp, terrain):
     g, st = case(nlev, ntr, w_amp, terrain)
     opts = abi.make_opts(1800.0, nrk_scal=nrk, scal_order=order)
     out, sct = run(g, st, opts)
+    check(out, oracle_lib.scalar_transport(abi.FortranGrid(g), opts, st.tracers, sct, st, fp64=True))
+
+
+# the 32-column tiles' groups: the counts around 32, the first and last of 40
+# and of 48 tracers a block, two blocks of 32 and of 40, and a level split
+@pytest.mark.parametrize("ntr,order,ks,w_amp,terrain", [
+    (17, 2, 1, 0.05, 0), (24, 3, 1, 3.0, 3), (25, 2, 1, 0.05, 0), (33, 3, 1, 0.05, 3), (40, 2, 1, 3.0, 0),
+    (41, 2, 1, 0.05, 3), (48, 3, 1, 0.05, 0), (49, 2, 1, 0.05, 0), (56, 3, 1, 0.05, 3), (57, 2, 1, 0.05, 0),
+    (74, 2, 1, 0.05, 3), (33, 2, 2, 0.05, 0)])
+def test_tile_groups(ntr, order, ks, w_amp, terrain):
+    g, st = case(12, ntr, w_amp, terrain)
+    opts = abi.make_opts(1800.0, scal_order=order)
+    out, sct = run(g, st, opts, shape=(32, 32, ks, 0))
     check(out, oracle_lib.scalar_transport(abi.FortranGrid(g), opts, st.tracers, sct, st, fp64=True))
 
 
