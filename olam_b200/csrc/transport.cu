@@ -287,13 +287,6 @@ static int pipelined_step(Context& C, const float* dtlr, const float* rhos_nrk) 
     OG_CUDA(cudaStreamSynchronize(s));   // the host vectors die here
   }
   if (!cells) { OG_PROF("tile_weights", s); OG_CHECK(launch_tile_weights(d, tp, rhos_nrk, s)); }
-  if (!cells && tp.autotune && tp.tuned_ntp != ntp) {
-    // the shape on this step's inputs: the tracers' device copies and the
-    // step's records (a rotation buffer as the scratch output)
-    OG_CHECK(ensure_q(s));
-    OG_CHECK(tile_autotune(C, tr.q[tr.qcur].p, tr.q[tr.qcur].p, tr.qt.p, tr.q[(tr.qcur + 1) % 3].p, dtlr[nrk - 1]));
-    tr.q_valid = false;   // the per-tracer arrays are what the pipelined step reads
-  }
   // the RK buffer sequence of the batched step
   const int a = tr.qcur;
   int bin[3], bout[3];
@@ -423,6 +416,18 @@ int transport_run(const float* rho_old_host, olamgpu_cfl_diag* diag) {
   bool anylim = false, any_pdm = false;
   OG_CHECK(tracer_modes(C, modes, pdm, anylim, any_pdm));
 
+  if (pipelined && tr.n > 64 && tp.autotune && tp.tuned_ntp != tr.ntp) {
+    // the shape on this step's inputs: the tracers' device copies and the
+    // step's records (a rotation buffer as the scratch output)
+    OG_CHECK(ensure_q(s));
+    OG_CHECK(launch_tile_weights(d, tp, rhos_nrk, s));
+    OG_CHECK(tile_autotune(C, tr.q[tr.qcur].p, tr.q[tr.qcur].p, tr.qt.p, tr.q[(tr.qcur + 1) % 3].p, dtlr[nrk - 1]));
+    tr.q_valid = false;   // the per-tracer arrays are what the pipelined step reads
+    if (!tile_shape_fits(d, 64)) {   // 8-column tiles have no group of 64
+      OG_CHECK(tracers_to_device(s));
+      pipelined = false;
+    }
+  }
   if (pipelined) {
     OG_CHECK(pipelined_step(C, dtlr, rhos_nrk));
   } else if (batched) {

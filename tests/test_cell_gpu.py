@@ -107,6 +107,18 @@ def test_per_call_groups(ntr, order, w_amp):
     check(out, oracle_lib.scalar_transport(abi.FortranGrid(g), opts, st.tracers, sct, st, fp64=True))
 
 
+# above 64 tracers on grids where the timed shapes are close, so that any of
+# them may be chosen, 8-column tiles too (which have no group of 64 tracers);
+# forced 8-column tiles take the step in one piece
+@pytest.mark.parametrize("nlev", [5, 7, 10, 14])
+@pytest.mark.parametrize("shape", [None, (8, 128, 1, 0)])
+def test_per_call_wide_groups(nlev, shape):
+    g, st = case(nlev, 70, 0.05, 0)
+    opts = abi.make_opts(1800.0)
+    out, sct = run(g, st, opts, coherence=abi.SYNC_EACH_CALL, shape=shape)
+    check(out, oracle_lib.scalar_transport(abi.FortranGrid(g), opts, st.tracers, sct, st, fp64=True))
+
+
 # mza = nlev + 1 at the sizes where the rows per lane and the warps per column
 # change, with and without the column kernel's folded set-up
 @pytest.mark.parametrize("nlev,kw", [(31, {}), (32, {}), (63, {}), (64, {}), (32, dict(ithil_monot=1))])
