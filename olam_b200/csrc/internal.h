@@ -115,6 +115,7 @@ struct DevBuf {
     n = count;
     return OLAMGPU_OK;
   }
+  int at_least(size_t count) { return n >= count ? OLAMGPU_OK : alloc(count); }
   void borrow(T* q, size_t count) {
     release();
     p = q;
@@ -560,6 +561,7 @@ int glue_mass_sums(int nsel, const int* ids, double* sums);
 int glue_timestep(unsigned flags, int nmass, const int* ids);
 int glue_timestep_diag(float* smax, double* sums);
 void glue_drop_graphs();
+int step_scratch(DevBuf<float>& b, size_t n);   // at least n floats; drops recorded steps when it grows
 void glue_release();
 int dyn_diagvel_t3d();
 // profiling off while a stream is being recorded into a graph

@@ -127,7 +127,13 @@ int tracers_to_host(cudaStream_t s) {
   return OLAMGPU_OK;
 }
 
-static int grow(DevBuf<float>& b, size_t n) { return b.n >= n ? OLAMGPU_OK : b.alloc(n); }
+// Scratch of the batched tracer step (tp.upv, tp.scale).  A recorded long
+// step holds its address, so whoever makes it larger -- the step itself or
+// the limiter's adjoint, which shares it -- drops the recorded steps first.
+int step_scratch(DevBuf<float>& b, size_t n) {
+  if (b.n < n) glue_drop_graphs();
+  return b.at_least(n);
+}
 
 // Tracers (padded) up to which a stage runs as passes over cells: the tiled
 // kernel gives 4 lanes or more to a column whatever the count, and needs the
@@ -143,12 +149,12 @@ static int ensure_pass_scratch(Context& C, int nt, int order) {
   Transport& tp = C.tp;
   const size_t wz = (size_t)d.mwa * d.mza * nt, vz = (size_t)d.mva * d.mza * nt;
   const int i2d = order == 3 ? 5 : 2;
-  OG_CHECK(grow(tp.gx, wz * i2d));
-  OG_CHECK(grow(tp.upv, vz));
-  OG_CHECK(grow(tp.hiv, vz));
-  OG_CHECK(grow(tp.sfv, vz));
-  OG_CHECK(grow(tp.scale, wz * 2));
-  OG_CHECK(grow(tp.upw, wz));
+  OG_CHECK(tp.gx.at_least(wz * i2d));
+  OG_CHECK(step_scratch(tp.upv, vz));
+  OG_CHECK(tp.hiv.at_least(vz));
+  OG_CHECK(tp.sfv.at_least(vz));
+  OG_CHECK(step_scratch(tp.scale, wz * 2));
+  OG_CHECK(tp.upw.at_least(wz));
   return OLAMGPU_OK;
 }
 
@@ -402,7 +408,7 @@ int transport_run(const float* rho_old_host, olamgpu_cfl_diag* diag) {
   } else {
     // groups of cell passes; a forced shape keeps the tiles
     pipelined = pipelined && tr.n > pipeline_group(tr.n) && tp.autotune && cell_stage_available(d, order);
-    if (pipelined && grow(tp.upv, (size_t)mva * mza * pipeline_group(tr.n)) != OLAMGPU_OK) {
+    if (pipelined && step_scratch(tp.upv, (size_t)mva * mza * pipeline_group(tr.n)) != OLAMGPU_OK) {
       cudaGetLastError();   // no room for the face values
       pipelined = false;
     }
@@ -440,7 +446,7 @@ int transport_run(const float* rho_old_host, olamgpu_cfl_diag* diag) {
     if (tp.have_turb)
       for (int n = 0; n < tr.n; ++n)
         if (tr.sgsmix[n]) launch_diffusion(d, tp, CTView{A, ntp, n}, TView{T, ntp, n}, 1, s);
-    if (cells && grow(tp.upv, (size_t)mva * mza * ntp) != OLAMGPU_OK) {
+    if (cells && step_scratch(tp.upv, (size_t)mva * mza * ntp) != OLAMGPU_OK) {
       cudaGetLastError();   // no room for the face values: the tiles need none
       cells = false;
     }
@@ -467,11 +473,12 @@ int transport_run(const float* rho_old_host, olamgpu_cfl_diag* diag) {
       if (last && anylim) {
         // limited last stage: passes over cells for tracer groups (multiples
         // of 4) sized to a scratch budget
-        const bool monot = C.opts.iscal_monot == 1;
-        const size_t vz = (size_t)mva * mza, per = 4 * ((monot ? 2 : 1) * wz + vz);
+        // (two planes of factors with either limiter: the positive-definite
+        // one's adjoint takes them in the same buffer)
+        const size_t vz = (size_t)mva * mza, per = 4 * (2 * wz + vz);
         const int grp = (int)std::max<size_t>(4, std::min<size_t>((size_t)ntp, (size_t)(8ull << 30) / per / 4 * 4));
-        OG_CHECK(grow(tp.upv, vz * grp));
-        OG_CHECK(grow(tp.scale, wz * grp * (monot ? 2 : 1)));
+        OG_CHECK(step_scratch(tp.upv, vz * grp));
+        OG_CHECK(step_scratch(tp.scale, 2 * wz * grp));
         cs.limited = C.opts.iscal_monot;
         cs.face = tp.upv.p; cs.scale = tp.scale.p;
         for (int g0 = 0; g0 < tr.n; g0 += grp) {

@@ -413,13 +413,12 @@ int pd_adjoint_stage(Context& C, const float* S, const float* S0p, const float* 
     // corrections and scale factors of the group
     const size_t wz = (size_t)d.mwa * mza * nt, vz = (size_t)d.mva * mza * nt;
     const int i2d = order == 3 ? 5 : 2;
-    auto grow = [](DevBuf<float>& b, size_t n) { return b.n >= n ? OLAMGPU_OK : b.alloc(n); };
-    OG_CHECK(grow(tp.gx, wz * i2d));
-    OG_CHECK(grow(tp.upv, vz));
-    OG_CHECK(grow(tp.hiv, vz));
-    OG_CHECK(grow(tp.sfv, vz));
-    OG_CHECK(grow(tp.scale, wz * 2));
-    OG_CHECK(grow(tp.upw, wz));
+    OG_CHECK(tp.gx.at_least(wz * i2d));
+    OG_CHECK(step_scratch(tp.upv, vz));
+    OG_CHECK(tp.hiv.at_least(vz));
+    OG_CHECK(tp.sfv.at_least(vz));
+    OG_CHECK(step_scratch(tp.scale, wz * 2));
+    OG_CHECK(tp.upw.at_least(wz));
     OG_CHECK(pda_scratch(C, nt, order, g_pda));
     float* p = g_pda.p;
     PdaArgs A;

@@ -135,3 +135,45 @@ def test_limited_window_equals_stepwise_chain():
     for n in range(NTR):
         assert relerr(g0[n][1:], l[n][1:]) < 1e-6, n
         assert relerr(gs[n][1:], ls_sum[n][1:]) < 1e-6, n
+
+
+@pytest.mark.parametrize("ntr", [3, 8])
+def test_limited_window_recorded_over_two_iterations(ntr):
+    """Two iterations of an inversion with recorded long steps: the window,
+    its adjoint (which shares scratch with the limited stage), the rewind,
+    and the window again.  Every pass equals the first pass of a run that
+    records nothing."""
+    from olam_b200.synth.state import fast_lognormal_tracers
+    from test_window_gpu import case
+    g, ds, _, _ = case(seed=12)
+    tr = fast_lognormal_tracers(g, ntr, seed=13, clip=(0.0, np.inf), zero_frac=0.0, as_list=True)
+    opts = abi.make_opts(600.0, nacoust=4, nrk_scal=2, iscal_monot=2)
+    arrays = oracle_lib.dyn_arrays(g, ds)
+    rng = np.random.default_rng(5)
+    lam = [rng.standard_normal((g.mwa, g.mza)).astype(np.float32) for _ in range(ntr)]
+    for x in lam:
+        x[0] = 0.0
+
+    def passes(flags, n):
+        dev = OlamGpu(abi.FortranGrid(g), opts, HostState(**{k: np.array(v, copy=True) for k, v in arrays.items()}))
+        out = []
+        try:
+            var_p = [t.copy() for t in tr]
+            dev.register_scalars(var_p, [np.zeros_like(t) for t in tr])
+            dev.set_coherence(abi.RESIDENT)
+            for i in range(n):
+                if i:
+                    dev.window_rewind()
+                dev.window_forward(6, 2, flags)   # three rotations recorded, then replayed
+                dev.sync_to_host(abi.F_SCALARS)
+                out.append(([t.copy() for t in var_p], *dev.window_adjoint(lam)))
+            return out
+        finally:
+            dev.close()
+
+    ref = passes(0, 1)[0]
+    for after, g0, gs in passes(abi.TS_GRAPH, 2):
+        for n in range(ntr):
+            assert np.array_equal(after[n], ref[0][n]), n
+            assert relerr(g0[n][1:], ref[1][n][1:]) < 1e-6, n
+            assert relerr(gs[n][1:], ref[2][n][1:]) < 1e-6, n
