@@ -483,10 +483,11 @@ int olamgpu_window_rewind(void);
  * in the reference: it serves callers that must not allocate device memory
  * during the call (a caller whose memory is fixed up front, or that records
  * its work into a CUDA graph).  The call allocates nothing: its scratch is
- * a fixed 64 MiB device array (gradient planes, V-face values, a zeroed
- * implicit fraction): i2d * mwa * mza + mva * mza + mwa floats must fit in
- * 16 Mi (i2d = 2 for order 2, 5 for order 3), i.e. up to NXP = 74 at order 2
- * and NXP = 58 at order 3 with mza = 61; larger grids get OLAMGPU_E_ARG.
+ * a fixed 64 MiB device array (V-face values and, in place, the result).
+ * It takes grids with i2d * mwa * mza + mva * mza + mwa <= 16 Mi (i2d = 2 for
+ * order 2, 5 for order 3), i.e. up to NXP = 74 at order 2 and NXP = 58 at
+ * order 3 with mza = 61; larger grids get OLAMGPU_E_ARG.  out may be scp,
+ * scp0 or sct itself; it must not overlap any input in another way.
  * The call must be made with the device of olamgpu_init current (else
  * OLAMGPU_E_STATE).  The first call on a device looks the scratch up (make
  * it before any stream capture; olamgpu_finalize forgets it); calls that

@@ -1117,15 +1117,15 @@ void launch_scatter_q(const float* q, float* const* dst, int n, int ntp, size_t 
 // ---------------------------------------------------------------------------
 // Stage without allocation (olamgpu_update_scalar_noalloc): one explicit,
 // unlimited RK stage of update_scalar for one tracer on device arrays the
-// caller owns, through the plain passes above.  Its scratch -- the gradient
-// planes (2 or 5 per cell), the V-face values and a zero implicit fraction
-// per column -- lives in a fixed device array, so the call itself never
-// allocates device memory.
+// caller owns, as passes over cells (transport_cell.cu).  Its scratch -- the
+// V-face values and, for a call in place, the result -- lives in a fixed
+// device array, so the call itself never allocates device memory.
 // ---------------------------------------------------------------------------
-// Scratch need in floats: i2d * mwa * mza (gradient planes, i2d = 2 for
-// order 2 and 5 for order 3) + mva * mza (V-face values) + mwa (implicit
-// fraction).  On the icosahedral grid (mwa = 10 NXP^2 + 3, mva = 30 NXP^2 + 1)
-// with mza = 61 that fits up to NXP = 74 at order 2 and NXP = 58 at order 3.
+// The grids the call takes: i2d * mwa * mza + mva * mza + mwa floats (i2d = 2
+// at order 2, 5 at order 3) must fit in the scratch, of which the faces and
+// the result use mva * mza + mwa * mza.  On the icosahedral grid (mwa = 10
+// NXP^2 + 3, mva = 30 NXP^2 + 1) with mza = 61 that is up to NXP = 74 at order
+// 2 and NXP = 58 at order 3.
 #define NOALLOC_SCRATCH_FLOATS (16u << 20)   // 64 MiB
 static __device__ __align__(256) float g_noalloc_scratch[NOALLOC_SCRATCH_FLOATS];
 
@@ -1169,8 +1169,8 @@ static int update_scalar_noalloc(const float* scp, const float* scp0, const floa
   const int order = C.opts.scal_horiz_adv_order;
   if (order != 2 && order != 3) { set_error("scal_horiz_adv_order must be 2 or 3"); return OLAMGPU_E_UNSUPPORTED; }
   const size_t i2d = order == 3 ? 5 : 2;
-  const size_t n_gx = i2d * d.mwa * d.mza, n_upv = (size_t)d.mva * d.mza, n_ff = d.mwa;
-  const size_t need = n_gx + n_upv + n_ff;
+  const size_t n_upv = (size_t)d.mva * d.mza;
+  const size_t need = i2d * d.mwa * d.mza + n_upv + d.mwa;
   if (need > NOALLOC_SCRATCH_FLOATS) {
     set_error("update_scalar_noalloc: this grid needs " + std::to_string(need) +
               " floats of scratch; the fixed scratch holds " + std::to_string(NOALLOC_SCRATCH_FLOATS));
@@ -1195,7 +1195,13 @@ static int update_scalar_noalloc(const float* scp, const float* scp0, const floa
   c.ff = nullptr;                       // every column explicit
   c.face = scr;
   c.istage = 1; c.nrk = 1; c.dtr = dtr;
+  // In place: a level's thread reads scp two levels up and down while other
+  // threads write theirs, so the result goes to the scratch (behind the face
+  // values) and then over scp.
+  const bool in_place = out == scp;
+  if (in_place) c.out = scr + n_upv;
   OG_CHECK(launch_cell_stage(d, order, c, s));
+  if (in_place) launch_copy_cols(d.jtw_prog.p, d.nw_prog, c.out, out, d.mza, s);
   OG_CUDA(cudaGetLastError());
   return OLAMGPU_OK;
 }

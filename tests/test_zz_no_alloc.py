@@ -97,3 +97,43 @@ def test_noalloc_rejects_a_grid_beyond_the_scratch():
         assert b"scratch" in dev.lib.olamgpu_strerror(rc)
     finally:
         dev.close()
+
+
+@pytest.mark.parametrize("order,terrain,alias", [(2, 0, "scp"), (3, 3, "scp"), (2, 3, "both"), (2, 0, "scp0")])
+def test_noalloc_in_place(order, terrain, alias):
+    """The result over scp (and, with "both", over scp0 at once), or over
+    scp0, equals the result in an array of its own; columns outside jtw_prog
+    stay as they were."""
+    import torch
+    g, st = small_case(nxp=6, nlev=40, ntr=1, seed=31)
+    if terrain:
+        from olam_b200.synth.grid import with_terrain
+        g = with_terrain(g, terrain)
+    dev = OlamGpu(abi.FortranGrid(g), abi.make_opts(1800.0, scal_order=order),
+                  HostState(vmasc=st.vmasc, wmasc=st.wmasc, rho=st.rho, wc=st.wc))
+    try:
+        def dv(a):
+            return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()
+        a, sct, rhos = dv(st.tracers[0]), dv(st.sct[0]), dv(st.rho)
+        vm, wm = dv(st.vmasc), dv(st.wmasc)
+        a[0] = 7.0
+        b = a if alias == "both" else a * 1.001
+
+        def stage(scp, scp0, out):
+            p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+            check(dev.lib.olamgpu_update_scalar_noalloc(p(scp), p(scp0), p(sct), p(rhos), p(vm), p(wm),
+                                                        C.c_float(900.0), p(out),
+                                                        C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+
+        ref = torch.zeros_like(a)
+        stage(a, b, ref)
+        for _ in range(3):
+            s = a.clone()
+            s0 = s if alias == "both" else b.clone()
+            out = s0 if alias == "scp0" else s
+            kept = out[0].clone()
+            stage(s, s0, out)
+            assert torch.equal(out[1:], ref[1:])
+            assert torch.equal(out[0], kept)
+    finally:
+        dev.close()
