@@ -1070,7 +1070,7 @@ __global__ void __launch_bounds__(256) k_vel_t3d(DynK g, const int* __restrict__
       z = z + c.z * u;
     };
 #pragma unroll
-    for (int n = 0; n < 6; ++n) if (n < 5 || np > 5) add(e[n], ec[n], v[r][n]);
+    for (int n = 0; n < 6; ++n) if (n < np) add(e[n], ec[n], v[r][n]);
     if (np > 6) {
       const int4 q = __ldg(E + 12);
       add(q, __ldg(ecv + iw * 7 + 6), kd >= q.z ? vc[(size_t)(q.y & 0x7fffffff) * mza + kd] : 0.f);

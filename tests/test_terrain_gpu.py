@@ -166,3 +166,51 @@ def test_terrain_timestep_matches_single_calls():
     for iw in range(1, g.mwa):
         kb = g.lpw[iw] - 1
         assert np.array_equal(scp[:, iw, :kb], np.repeat(scp[:, iw, kb:kb + 1], kb, axis=1))
+
+
+def test_terrain_velocities_of_columns_with_four_edges():
+    """Shaved columns given four edges (npoly counts from 3): edges past
+    npoly add nothing, whatever the tables hold there and at the dummy V
+    point.  diagvel_t3d against its sums in numpy (FP64)."""
+    import copy
+    from test_timestep_gpu import Dev, _case
+    g0, _, arrays, tr = _case(ntr=1)
+    g = copy.copy(terrain_grid(g0))
+    g.npoly = g.npoly.copy()
+    cols = np.flatnonzero(g.lve2 > 0)[::7]
+    g.npoly[cols] = 4
+    faces = np.arange(7)[None, :] < g.npoly[:, None]
+    g.lve2 = np.where(faces, g.lpv[g.itab_w_iv] - g.lpw[:, None], 0).max(axis=1).clip(0).astype(np.int32)
+    g.lve2[0] = 0
+    assert (g.lve2[cols] > 0).any()
+    for k in ("vnx", "vny", "vnz"):
+        setattr(g, k, getattr(g, k).copy())
+        getattr(g, k)[0] = 1.0
+    for k in ("ecvec_vx", "ecvec_vy", "ecvec_vz"):
+        setattr(g, k, np.where(faces, getattr(g, k), 10.0).astype(np.float32))
+    d = Dev(g, arrays, tr, abi.make_opts(600.0, nacoust=2), coherence=abi.SYNC_EACH_CALL)
+    try:
+        old = np.stack([d.hs[k].astype(np.float64) for k in ("vxe", "vye", "vze")])
+        d.dev.diagvel_t3d()
+        out = np.stack([d.hs[k] for k in ("vxe", "vye", "vze")])
+        wc, vc = d.hs["wc"].astype(np.float64), d.hs["vc"].astype(np.float64)
+    finally:
+        d.close()
+    vn = np.stack([g.vnx, g.vny, g.vnz]).astype(np.float64)
+    ec = np.stack([g.ecvec_vx, g.ecvec_vy, g.ecvec_vz]).astype(np.float64)
+    wn = np.stack([g.wnxo2, g.wnyo2, g.wnzo2]).astype(np.float64)
+    ref = np.zeros_like(old)
+    for iw in range(1, g.mwa):
+        kb = g.lpw[iw] - 1
+        for k in range(kb, g.mza):
+            x = wn[:, iw] * (wc[iw, k - 1] + wc[iw, k])
+            for n in range(g.npoly[iw]):
+                iv = g.itab_w_iv[iw, n]
+                if k >= g.lpv[iv] - 1:
+                    x = x + ec[:, iw, n] * vc[iv, k]
+                elif k - kb < g.lve2[iw]:
+                    x = x + ec[:, iw, n] * (vn[:, iv] @ old[:, iw, k])
+            ref[:, iw, k] = x
+        ref[:, iw, :kb] = ref[:, iw, kb:kb + 1]
+    for i in range(3):
+        assert relerr(out[i][1:], ref[i][1:]) < 1e-5, (i, relerr(out[i][1:], ref[i][1:]))
