@@ -496,7 +496,7 @@ k_grad_upv4(DynK g, const int* __restrict__ prog, int nprog, int nch, Four s, un
         w[1] = __int_as_float(b.y);
       } else {
 #pragma unroll
-        for (int m = 0; m < NPL; ++m) w[m] = xy_hu[((size_t)iw * 7 + n0 + i) * 5 + m];
+        for (int m = 0; m < NPL; ++m) w[m] = n0 + i < np ? xy_hu[((size_t)iw * 7 + n0 + i) * 5 + m] : 0.f;
       }
       // a closed edge adds nothing: q = c0
 #pragma unroll

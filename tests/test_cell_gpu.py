@@ -132,3 +132,29 @@ def test_acoustic_step_by_level_count(nlev, kw):
     o32, _ = oracle_long_steps(fg, opts, arrays, 1, False)
     hs, _ = gpu_long_steps(fg, opts, arrays, 1, abi.SYNC_EACH_CALL)
     check_fields(hs, o32, o64)
+
+
+# the tables' entries past a column's npoly are the caller's padding: NaN
+# there reaches no result
+@pytest.mark.parametrize("order", [2, 3])
+def test_padding_of_the_edge_tables_is_not_used(order):
+    import copy
+    from test_timestep_gpu import Dev, _case, _same
+    g0, _, arrays, tr = _case(ntr=3)
+    past = np.arange(7)[None, :] >= g0.npoly[:, None]
+    g1 = copy.copy(g0)
+    for k in ("gxps_coef", "gyps_coef", "xy_h", "xy_hu", "dirv", "xx_yy", "ecvec_vx", "ecvec_vy", "ecvec_vz"):
+        a = getattr(g0, k).copy()
+        a[past] = np.nan
+        setattr(g1, k, a)
+    opts = abi.make_opts(600.0, nacoust=2, scal_order=order, thil_order=order, wind_order=order)
+    out = []
+    for g in (g0, g1):
+        d = Dev(g, arrays, tr, opts)
+        try:
+            d.dev.timestep(0)
+            out.append(d.host())
+        finally:
+            d.close()
+    assert all(np.isfinite(out[0][k]).all() for k in out[0])
+    _same(out[0], out[1])
