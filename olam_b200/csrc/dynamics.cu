@@ -364,7 +364,8 @@ struct VtendArgs {
   const double* rho;
   const float* fdivh; const float* dh;             // NULL dh: no divergence damping
   const float* fvorth; const float* fvortl;        // NULL fvorth: no vorticity damping
-  const float* vl; const float* vh; int vlevel;
+  const float* vl; const float* vh;
+  int lpm;                            // the second-order plane below the M points' floors (level 3)
 };
 
 // A warp to 32 levels of a V point: here two levels a lane cost more in
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(256) k_vtend(DynK g, VtendArgs A) {
   }
   if (vor) {
     // below ka the level-3 damping takes the second-order plane
-    const int ka = A.vlevel != 3 || g.flat ? kv : max(g.lpm[im.x], g.lpm[im.y]);
+    const int ka = A.lpm ? max(g.lpm[im.x], g.lpm[im.y]) : kv;
     const float* p = kd < ka ? A.vl : A.vh;
     fv = kd < ka ? A.fvortl[iv] : A.fvorth[iv];
     v1 = p[(size_t)im.x * mza + kd];
@@ -1145,6 +1146,8 @@ int dyn_setup(const olamgpu_grid* g, const olamgpu_opts* o, cudaStream_t s) {
   }
   for (int i = 1; i < mma; ++i)
     if (g->lpm[i] < 2 || g->lpm[i] > mza) { set_error("lpm out of range [2,mza] at M point " + std::to_string(i + 1)); return OLAMGPU_E_ARG; }
+  y.lpm_flat = true;
+  for (int i = 1; i < mma; ++i) if (g->lpm[i] != 2) y.lpm_flat = false;
   // shaved cells: lve2(iw) levels from lpw up have closed V faces; every
   // closed face must lie within them (hex_grid.f90 sets lve2 to the largest
   // lpv - lpw of the column's faces)
@@ -1417,7 +1420,8 @@ static int v_tendency(Context& C, bool div, bool vor, bool setup, const float* s
   }
   if (div) { V.fdivh = y.fdivh.p; V.dh = plane(y.div2d.p, wz, ld == 1 ? 1 : (ld - 1) % 2 + 1); }
   if (vor) {
-    V.fvorth = y.fvorth.p; V.fvortl = y.fvortl.p; V.vlevel = lv;
+    V.fvorth = y.fvorth.p; V.fvortl = y.fvortl.p;
+    V.lpm = lv == 3 && !(g.flat && y.lpm_flat);
     V.vl = plane(y.vort2d.p, mz, lv == 1 ? 1 : (lv - 2) % 2 + 1);
     V.vh = plane(y.vort2d.p, mz, lv == 1 ? 1 : (lv - 1) % 2 + 1);
   }

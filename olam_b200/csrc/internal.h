@@ -364,6 +364,7 @@ struct Dyn {
   DevBuf<float> upw, upv;
   DevBuf<float> div2d, fdivh, vort2d, fvorth, fvortl, vfact;
   DevBuf<int> lpmmin;
+  bool lpm_flat = true;          // lpm = 2 at every M point
   // prognostic shaved-cell method: lve2 of every W column and the start
   // momentum of its lve2 lowest levels, (mwa, nve2_max, 3); none on grids
   // where no column has a closed face (nve2_max = 0)

@@ -158,3 +158,21 @@ def test_padding_of_the_edge_tables_is_not_used(order):
             d.close()
     assert all(np.isfinite(out[0][k]).all() for k in out[0])
     _same(out[0], out[1])
+
+
+# M-point floors of their own on a grid whose W and V floors are all level 2:
+# the level-3 vorticity damping takes its second-order plane below them
+def test_m_floors_on_a_flat_grid():
+    import copy
+    g0, ds = dyn_case()
+    g = copy.copy(g0)
+    g.lpm = g0.lpm.copy()
+    g.lpm[1::3] = 6
+    opts = abi.make_opts(600.0, nacoust=4)
+    assert opts.vort_damp_level == 3 and (g.lpw[1:] == 2).all() and (g.lpv[1:] == 2).all()
+    fg = abi.FortranGrid(g)
+    arrays = oracle_lib.dyn_arrays(g, ds)
+    o64, _ = oracle_long_steps(fg, opts, arrays, 1, True)
+    o32, _ = oracle_long_steps(fg, opts, arrays, 1, False)
+    hs, _ = gpu_long_steps(fg, opts, arrays, 1, abi.SYNC_EACH_CALL)
+    check_fields(hs, o32, o64)
