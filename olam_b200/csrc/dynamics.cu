@@ -901,6 +901,8 @@ __global__ void __launch_bounds__(32 * NW * WRT_COLS(NW), WRT_OCC / (NW * WRT_CO
     if (i > 0) ra = (double)(-arwm * (b21 + b25 + b23 * U[kd - 1]));
     rb = (double)(A.b20[kd] + arw0 * (b25 - b26 + (b23 + b24) * u[0]));
     if (i < n - 1) rc = (double)(arwp * (b22 + b26 - b24 * U[kd + 1]));
+  } else if (i == 0) {
+    A.wc[x - 1] = wcp;   // a column of one level, whose wcp is its own
   }
   column_sync<NW>();
   // phase 3: tridiffo's system across the column's lanes

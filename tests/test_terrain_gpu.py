@@ -214,3 +214,43 @@ def test_terrain_velocities_of_columns_with_four_edges():
         ref[:, iw, :kb] = ref[:, iw, kb:kb + 1]
     for i in range(3):
         assert relerr(out[i][1:], ref[i][1:]) < 1e-5, (i, relerr(out[i][1:], ref[i][1:]))
+
+
+def floors(g0, lpw):
+    """g0 with the W floors lpw and the V, M and shaved-cell floors they imply."""
+    import copy
+    g = copy.copy(g0)
+    g.lpw = lpw.astype(np.int32)
+    g.lpv = np.maximum(lpw[g.itab_v_iw[:, 0]], lpw[g.itab_v_iw[:, 1]]).astype(np.int32)
+    g.lpm = np.max(g.lpv[g.itab_m_iv], axis=1).astype(np.int32)
+    faces = np.arange(7)[None, :] < g.npoly[:, None]
+    g.lve2 = np.where(faces, g.lpv[g.itab_w_iv] - lpw[:, None], 0).max(axis=1).clip(0).astype(np.int32)
+    g.lpv[0] = g.lpm[0] = 2
+    g.lve2[0] = 0
+    return g
+
+
+def test_column_of_one_level():
+    """A column whose only level is the top one has no W face to solve for:
+    its wc below the floor is the level's own."""
+    from test_dynamics_gpu import dyn_case
+    g0, ds = dyn_case()
+    lpw = np.full(g0.mwa, 2)
+    lpw[[40, 90]] = g0.mza, g0.mza - 1
+    g = floors(g0, lpw)
+    arrays = oracle_lib.dyn_arrays(g, ds)
+    arrays["wc"] = arrays["wc"].copy()
+    arrays["wc"][1:, -1] = 0.25
+    opts = abi.make_opts(60.0, nacoust=4)
+    hs = HostState(**{k: np.array(v, copy=True) for k, v in arrays.items()})
+    dev = OlamGpu(abi.FortranGrid(g), opts, hs)
+    o = oracle_lib.DynOracle(abi.FortranGrid(g), opts, arrays, fp64=True)
+    try:
+        dev.prog_wrtv_rk(1)
+        o.prog_wrtv_rk(1)
+        for iw in (40, 90):
+            kb = g.lpw[iw] - 1
+            assert relerr(hs["wc"][iw, kb - 1:], o.a["wc"][iw, kb - 1:]) < 1e-4, iw
+            assert hs["wc"][iw, kb - 1] == hs["wc"][iw, kb], iw
+    finally:
+        dev.close()
