@@ -16,7 +16,7 @@
 //                           vmasc (:320-368); on the last stage the fields
 //                           with ithil_monot / iwind_monot > 0 take
 //                           dynamics_monot.cu's values
-//   k_vmca                  vmca / vmasc on a rank with a halo
+//   k_vmca                  vmca / vmasc on a rank with a halo, or beside border columns
 //   k_upw4                  the vertical face values where the column kernel does not
 //                           form them (eddy, Rayleigh or flux-corrected terms)
 //   k_wrt_begs              prog_wrt_begs (:494-884): lanes over levels for the explicit
@@ -1518,10 +1518,11 @@ int dyn_prog_wrtv_rk(int istp) {
     const float dts = (float)dt8;
     const int last = istage == nrk;
     // vmca = vmc arv, added to vmasc on the last stage: formed with the face
-    // values, or, on a rank with a halo, whose ring-1 columns have faces
-    // outside jtv_wadj, over that table
+    // values by the face's upwind column, or over jtv_wadj where that may be
+    // a column k_grad_upv4 does not run (a border column) and on a rank with
+    // a halo, whose ring-1 columns have faces outside the table
     FaceFlux ffx{y.arv.p, y.vmca.p, last ? tp.vmasc.p : nullptr};
-    if (C.halo.on) {
+    if (C.halo.on || !d.v_closed) {
       ffx = FaceFlux{};
       OG_PROF("vmca", s);
       k_vmca<<<nbva, 256, 0, s>>>(g, d.jtv_wadj.p, d.nv_wadj, y.vmc.p, y.arv.p, y.vmca.p, tp.vmasc.p, last);

@@ -132,6 +132,10 @@ int upload_grid(const olamgpu_grid* g, DevGrid& d, cudaStream_t s) {
       viw[(size_t)iv * 2 + k] = iv > 0 ? w - 1 : 0;
       if (g->itab_v_im) vim[(size_t)iv * 2 + k] = iv > 0 ? g->itab_v_im[(size_t)iv * 2 + k] - 1 : 0;
     }
+  d.v_closed = true;
+  for (int j = 0; j < g->nv_wadj; ++j)
+    for (int k = 0; k < 2; ++k)
+      if (!isprog[viw[(size_t)(g->jtv_wadj[j] - 1) * 2 + k]]) d.v_closed = false;
   OG_CHECK(upload(d.v_iw, viw.data(), viw.size(), s));
   OG_CHECK(upload(d.v_im, vim.data(), vim.size(), s));
   OG_CUDA(cudaStreamSynchronize(s));

@@ -369,3 +369,31 @@ def test_long_step_two_processes_over_gloo():
         covw[r["w"]] = True
         covv[r["v"]] = True
     assert covw[1:].all() and covv[1:].all()
+
+
+def test_mass_flux_of_border_faces_without_a_plan():
+    """A rank's part of the grid run without its halo plan: the time-averaged
+    mass flux takes vmc arv at the faces whose upwind cell the rank holds but
+    does not prognose too (here those whose vmc it does not update)."""
+    import oracle_lib
+    from test_dynamics_gpu import dyn_case
+    g, ds = dyn_case()
+    loc = decomp.local_grid(g, decomp.bisect(g, 2), 0)
+    lg = loc.grid
+    arrays = {k: np.ascontiguousarray(v[{g.mwa: loc.wmap, g.mva: loc.vmap}[v.shape[0]]])
+              for k, v in oracle_lib.dyn_arrays(g, ds).items()}
+    adj, prog = lg.jtv_wadj - 1, np.zeros(lg.mwa, bool)
+    prog[lg.jtw_prog - 1] = True
+    hs = HostState(**arrays)
+    vmc, start = hs["vmc"].copy(), hs["vmasc"].copy()
+    dev = OlamGpu(abi.FortranGrid(lg), abi.make_opts(600.0, nacoust=4), hs)
+    try:
+        dev.prog_wrtv_rk(1)
+    finally:
+        dev.close()
+    f = np.setdiff1d(adj, lg.jtv_prog - 1)
+    k = np.arange(lg.mza)[None, :] >= lg.lpv[f, None] - 1
+    up = np.where(vmc[f] < 0, lg.itab_v_iw[f, 1:2], lg.itab_v_iw[f, 0:1])
+    assert (k & ~prog[up]).sum() > 20
+    ref = np.where(k, start[f] + vmc[f] * lg.arv[f], start[f])
+    assert np.allclose(hs["vmasc"][f], ref, rtol=1e-6, atol=0)
