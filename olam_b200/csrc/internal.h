@@ -163,6 +163,7 @@ struct DevGrid {
   DevBuf<int> jtw_prog, jtv_wadj, jtv_prog, jtw_wadj, jtm_prog;  // 0-based
   int off_wprog = -1, off_vwadj = -1, off_vprog = -1, off_wwadj = -1, off_mprog = -1;   // contiguous tables: first entry (0-based), else -1
   bool v_closed = true;  // both cells of every face of jtv_wadj are prognosed
+  bool w_covered = true; // jtw_wadj holds every prognosed column and its neighbours
   DevBuf<int> npoly;     // (mwa)
   DevBuf<int> w_nb;      // (mwa, 8) 0-based W neighbours, padded with self
   DevBuf<int> w_ev;      // (mwa, 8) 0-based V neighbours, padded with 0

@@ -114,6 +114,14 @@ int upload_grid(const olamgpu_grid* g, DevGrid& d, cudaStream_t s) {
       if (g->itab_w_im) im[(size_t)iw * 8 + j] = g->itab_w_im[(size_t)iw * 7 + j] - 1;
     }
   }
+  {
+    std::vector<char> adj(mwa, 0);
+    for (int j = 0; j < g->nw_wadj; ++j) adj[g->jtw_wadj[j] - 1] = 1;
+    d.w_covered = true;
+    for (int iw = 1; iw < mwa; ++iw)
+      for (int j = 0; isprog[iw] && j < npoly[iw]; ++j)
+        if (!adj[iw] || !adj[nb[(size_t)iw * 8 + j]]) d.w_covered = false;
+  }
   OG_CHECK(upload(d.npoly, npoly.data(), npoly.size(), s));
   OG_CHECK(upload(d.w_nb, nb.data(), nb.size(), s));
   OG_CHECK(upload(d.w_ev, ev.data(), ev.size(), s));

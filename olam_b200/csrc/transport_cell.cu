@@ -620,7 +620,7 @@ static void over(CellArgs& A, const DevBuf<int>& cols, int n, int off) { A.cols 
 static unsigned cell_blocks(const CellArgs& A) { return cdiv((size_t)A.ncol * A.nch, 8); }
 
 bool cell_stage_available(const DevGrid& d, int order) {
-  return d.edge.p && (order == 2 || (order == 3 && d.edge3_b.p));
+  return d.w_covered && (order == 2 || order == 3);
 }
 
 template <int V, typename OFF>
@@ -634,8 +634,11 @@ static int run_stage(const DevGrid& d, int order, const CellStage& c, cudaStream
   const bool lim = c.limited != 0, monot = c.limited == 1;
   A.a_w = monot ? d.a_wu.p : d.a_w.p;
   A.edge3 = reinterpret_cast<const float4*>(monot ? d.edge3_u.p : d.edge3_b.p);
-  // every face's upwind cell is in jtw_wadj
-  over(A, d.jtw_wadj, d.nw_wadj, d.off_wwadj);
+  // Every face's upwind cell is in jtw_wadj.  A caller of the no-allocation
+  // stage may leave the table out: on a domain without borders jtw_prog holds
+  // them too.
+  if (d.w_covered || lim) over(A, d.jtw_wadj, d.nw_wadj, d.off_wwadj);
+  else over(A, d.jtw_prog, d.nw_prog, d.off_wprog);
   {
     OG_PROF(lim ? "lim_face" : "cell_face", s);
     const unsigned nb = cell_blocks(A);

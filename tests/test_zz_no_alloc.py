@@ -137,3 +137,38 @@ def test_noalloc_in_place(order, terrain, alias):
             assert torch.equal(out[0], kept)
     finally:
         dev.close()
+
+
+@pytest.mark.parametrize("order", [2, 3])
+def test_grid_without_the_jtw_wadj_table(order):
+    """On a domain without borders jtw_wadj names no column that jtw_prog
+    does not: a grid without it takes the no-allocation stage and the
+    resident step with few tracers, with the results it has with the table."""
+    import torch
+    g, st = small_case(nxp=6, nlev=12, ntr=4, seed=31)
+    out = []
+    for table in (True, False):
+        fg = abi.FortranGrid(g)
+        if not table:
+            fg.struct.nw_wadj, fg.struct.jtw_wadj = 0, None
+        dev = OlamGpu(fg, abi.make_opts(1800.0, scal_order=order),
+                      HostState(vmasc=st.vmasc, wmasc=st.wmasc, rho=st.rho, wc=st.wc))
+        try:
+            def dv(a):
+                return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()
+            arrays = [dv(a) for a in (st.tracers[0], st.tracers[0], st.sct[0], st.rho, st.vmasc, st.wmasc)]
+            res = torch.zeros_like(arrays[0])
+            p = [C.c_void_p(a.data_ptr()) for a in arrays + [res]]
+            check(dev.lib.olamgpu_update_scalar_noalloc(*p[:6], C.c_float(900.0), p[6],
+                                                        C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+            dev.set_coherence(abi.RESIDENT)
+            var_p = [t.copy() for t in st.tracers]
+            dev.register_scalars(var_p, [t.copy() for t in st.sct])
+            dev.scalar_transport_rk(st.rho_old)
+            dev.sync_to_host(abi.F_SCALARS)
+            out.append((res.cpu().numpy(), var_p))
+        finally:
+            dev.close()
+    assert np.array_equal(out[0][0], out[1][0])
+    for a, b in zip(out[0][1], out[1][1]):
+        assert relerr(b[1:], a[1:]) < 1e-6
