@@ -320,6 +320,10 @@ __global__ void __launch_bounds__(256) k_update(CellArgs A) {
   // differences from scp0: the coefficients add up to the S0 term's
   float b[5];
   zbeta(A.a_w, mza, kd, kb, wm, wp, b);
+  // The level two away on the downwind side of a face is not in the stencil:
+  // its coefficient is zero, but a NaN there times zero would reach this cell.
+  if (wm < 0.f || kd == kb) w[0] = s00;
+  if (!(wp < 0.f) || kd == mza - 1) w[4] = s00;
 #pragma unroll
   for (int m = 0; m < 5; ++m) fd = fmav<V>(fexpl * b[m], subv<V>(w[m], s00), fd);
   const Vec<V> o = fmav<V>(A.dtr / rh, fmav<V>(vt, fd, tend), s00);

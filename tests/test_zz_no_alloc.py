@@ -172,3 +172,63 @@ def test_grid_without_the_jtw_wadj_table(order):
     assert np.array_equal(out[0][0], out[1][0])
     for a, b in zip(out[0][1], out[1][1]):
         assert relerr(b[1:], a[1:]) < 1e-6
+
+
+@pytest.mark.parametrize("order,terrain", [(2, 0), (3, 3)])
+def test_noalloc_nan_and_infinity_reach_their_stencil_only(order, terrain):
+    """One stage of a tracer with NaN and infinite cells: the cells that are
+    not finite after it are those whose stencil (upwind reconstruction at the
+    six faces and the two W faces) holds one, found in numpy; all others have
+    the value that a finite tracer gives."""
+    import torch
+    g, st = small_case(nxp=6, nlev=14, ntr=1, seed=31)
+    if terrain:
+        from olam_b200.synth.grid import with_terrain
+        g = with_terrain(g, terrain)
+    rng = np.random.default_rng(2)
+    scp = st.tracers[0].copy()
+    bad = np.zeros(scp.shape, bool)
+    iw = rng.choice(np.arange(1, g.mwa), 12, replace=False)
+    kb = g.lpw[iw] - 1
+    k = rng.integers(kb, g.mza)
+    bad[iw, k] = True
+    dev = OlamGpu(abi.FortranGrid(g), abi.make_opts(1800.0, scal_order=order),
+                  HostState(vmasc=st.vmasc, wmasc=st.wmasc, rho=st.rho, wc=st.wc))
+    try:
+        def stage(q):
+            def dv(a):
+                return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()
+            arrays = [dv(a) for a in (q, st.tracers[0], st.sct[0], st.rho, st.vmasc, st.wmasc)]
+            arrays.append(torch.zeros_like(arrays[0]))
+            check(dev.lib.olamgpu_update_scalar_noalloc(*[C.c_void_p(a.data_ptr()) for a in arrays[:6]],
+                                                        C.c_float(900.0), C.c_void_p(arrays[6].data_ptr()),
+                                                        C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+            return arrays[6].cpu().numpy()
+        ref = stage(scp)
+        scp[iw, k] = np.where(np.arange(12) % 3 == 0, np.inf, np.nan)
+        out = stage(scp)
+    finally:
+        dev.close()
+    # the cells whose value a cell's gradient or its own value takes
+    grad = bad.copy()
+    for n in range(7):
+        use = (n < g.npoly)[:, None] & (np.arange(g.mza)[None, :] >= g.lpv[g.itab_w_iv[:, n]][:, None] - 1)
+        grad |= use & bad[g.itab_w_iw[:, n]]
+    hit = np.zeros_like(bad)
+    for w in range(1, g.mwa):
+        b0 = g.lpw[w] - 1
+        for lev in range(b0, g.mza):
+            for n in range(g.npoly[w]):
+                v = g.itab_w_iv[w, n]
+                if lev >= g.lpv[v] - 1:
+                    hit[w, lev] |= grad[g.itab_v_iw[v, 1 if st.vmasc[v, lev] < 0 else 0], lev]
+            for f in (lev - 1, lev):                    # the W faces below and above
+                if f < b0 or f == g.mza - 1:
+                    hit[w, lev] |= bad[w, lev]
+                    continue
+                c = f + 1 if st.wmasc[w, f] < 0 else f
+                hit[w, lev] |= bad[w, max(c - 1, b0):min(c + 2, g.mza)].any()
+    for w in range(1, g.mwa):
+        hit[w, :g.lpw[w] - 1] = hit[w, g.lpw[w] - 1]
+    assert np.array_equal(~np.isfinite(out[1:]), hit[1:])
+    assert np.array_equal(out[1:][~hit[1:]], ref[1:][~hit[1:]])
