@@ -34,6 +34,7 @@
 #include <cstring>
 #include <type_traits>
 
+#include "recip.cuh"
 #include "transport_kernels.cuh"
 
 namespace olamgpu {
@@ -632,15 +633,6 @@ template <int NW>
 __device__ __forceinline__ void column_sync() {
   if constexpr (NW == 1) __syncwarp();
   else __syncthreads();
-}
-
-// 1 / x in FP64 from the approximate reciprocal and two Newton steps (each
-// squares the error, 2^-20 at the start); x is a normal number here
-__device__ __forceinline__ double recip(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(y, fma(-x, y, 1.0), y);
-  return fma(y, fma(-x, y, 1.0), y);
 }
 
 // The W system of prog_wrt_begs, b31(k) x(k-1) + b32(k) x(k) + b33(k) x(k+1)
