@@ -343,9 +343,8 @@ static int pipelined_step(Context& C, const float* dtlr, const float* rhos_nrk) 
         launch_implicit_solve(d, tp, nrk, istage, dtr, CTView{A, ntp, tb}, TView{OUT, ntp, tb}, width, s);
       }
     }
-    // points outside jtw_prog keep their values (a later group's own are
-    // copied again when it has them)
-    launch_copy_cols(d.w_nonprog.p, d.n_nonprog, A, tr.q[fin].p, (size_t)d.mza * ntp, s);
+    // points outside jtw_prog keep their values
+    launch_copy_cols(d.w_nonprog.p, d.n_nonprog, A + tb, tr.q[fin].p + tb, d.mza, width, ntp, s);
     launch_scatter_q_range(tr.q[fin].p + tb, tp.ptab_p.p + tb, tc, width, ntp, npk, s);
     OG_CUDA(cudaEventRecord(tp.ev[2 * g + 1], s));
     OG_CUDA(cudaStreamWaitEvent(tp.s_dn, tp.ev[2 * g + 1], 0));
@@ -506,7 +505,7 @@ int transport_run(const float* rho_old_host, olamgpu_cfl_diag* diag) {
       out_b = (out_b + 1) % 3;
       if (out_b == a) out_b = (out_b + 1) % 3;
     }
-    launch_copy_cols(d.w_nonprog.p, d.n_nonprog, A, tr.q[in_b].p, (size_t)mza * ntp, s);
+    launch_copy_cols(d.w_nonprog.p, d.n_nonprog, A, tr.q[in_b].p, mza, ntp, ntp, s);
     tr.qcur = in_b;
     tr.q_valid = true;
   } else {
@@ -535,7 +534,7 @@ int transport_run(const float* rho_old_host, olamgpu_cfl_diag* diag) {
         ob ^= 1;
       }
       // the final stage output becomes the tracer's device array
-      launch_copy_cols(d.w_nonprog.p, d.n_nonprog, A, tp.plain_out[ob ^ 1].p, (size_t)mza, s);
+      launch_copy_cols(d.w_nonprog.p, d.n_nonprog, A, tp.plain_out[ob ^ 1].p, mza, 1, 1, s);
       std::swap(tr.p[n], tp.plain_out[ob ^ 1]);
     }
   }

@@ -994,21 +994,21 @@ void launch_tend(const DevGrid& d, const Transport& tp, CTView scp_in, CTView sc
 // Points outside jtw_prog (OLAM's dummy point 1, and lateral-boundary or
 // halo columns in other domains) are never updated; the reference keeps
 // their values in place.  Stage outputs live in rotating buffers, so those
-// columns are copied from the input into the final buffer.
+// columns are copied from the input into the final buffer: width floats of
+// each of a column's rows of ld floats.
 __global__ void k_copy_cols(const int* __restrict__ cols, int ncol, const float* __restrict__ src,
-                            float* __restrict__ dst, size_t colsize) {
+                            float* __restrict__ dst, size_t rows, size_t width, size_t ld) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (size_t)ncol * colsize) return;
-  size_t c = i / colsize, r = i % colsize;
-  size_t off = (size_t)cols[c] * colsize + r;
+  if (i >= (size_t)ncol * rows * width) return;
+  const size_t r = i / width, c = r / rows;
+  const size_t off = ((size_t)cols[c] * rows + (r - c * rows)) * ld + (i - r * width);
   dst[off] = src[off];
 }
 
-void launch_copy_cols(const int* cols, int ncol, const float* src, float* dst, size_t colsize,
+void launch_copy_cols(const int* cols, int ncol, const float* src, float* dst, size_t rows, size_t width, size_t ld,
                       cudaStream_t s) {
   if (ncol <= 0) return;
-  size_t n = (size_t)ncol * colsize;
-  k_copy_cols<<<cdiv(n, 256), 256, 0, s>>>(cols, ncol, src, dst, colsize);
+  k_copy_cols<<<cdiv((size_t)ncol * rows * width, 256), 256, 0, s>>>(cols, ncol, src, dst, rows, width, ld);
   OG_LAUNCHED();
 }
 
@@ -1201,7 +1201,7 @@ static int update_scalar_noalloc(const float* scp, const float* scp0, const floa
   const bool in_place = out == scp;
   if (in_place) c.out = scr + n_upv;
   OG_CHECK(launch_cell_stage(d, order, c, s));
-  if (in_place) launch_copy_cols(d.jtw_prog.p, d.nw_prog, c.out, out, d.mza, s);
+  if (in_place) launch_copy_cols(d.jtw_prog.p, d.nw_prog, c.out, out, d.mza, 1, 1, s);
   OG_CUDA(cudaGetLastError());
   return OLAMGPU_OK;
 }

@@ -132,8 +132,8 @@ int launch_cell_stage(const DevGrid& d, int order, const CellStage& c, cudaStrea
 void launch_cell_preupdate(const DevGrid& d, const Transport& tp, float* S0, const float* SCT, int ld, int nt,
                            const int* mode, float dtr, cudaStream_t s);
 
-// copy the columns outside jtw_prog (colsize floats each) from src to dst
-void launch_copy_cols(const int* cols, int ncol, const float* src, float* dst, size_t colsize,
+// copy columns of rows of ld floats, the first width floats of each row, from src to dst
+void launch_copy_cols(const int* cols, int ncol, const float* src, float* dst, size_t rows, size_t width, size_t ld,
                       cudaStream_t s);
 
 // layout transposes: per-tracer arrays <-> batched layout

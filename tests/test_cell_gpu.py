@@ -8,6 +8,8 @@ levels).
 Tolerances are the repository's: 1e-5 normwise for the transport and the
 thermodynamic fields, five times the oracle's own FP32-FP64 spread (at least
 1e-5) for the momentum fields."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -105,6 +107,39 @@ def test_per_call_groups(ntr, order, w_amp):
     opts = abi.make_opts(1800.0, scal_order=order)
     out, sct = run(g, st, opts, coherence=abi.SYNC_EACH_CALL)
     check(out, oracle_lib.scalar_transport(abi.FortranGrid(g), opts, st.tracers, sct, st, fp64=True))
+
+
+# three calls in a row (the rotation buffers change roles) equal three
+# resident steps; columns that are not prognosed -- the dummy point, and with
+# a third of the others left out of jtw_prog those -- keep their values
+@pytest.mark.parametrize("nrk", [2, 3])
+@pytest.mark.parametrize("ntr,border", [(21, False), (21, True), (70, True)])
+def test_per_call_groups_over_several_steps(ntr, border, nrk):
+    g, st = case(12, ntr, 0.05, 0)
+    opts = abi.make_opts(1800.0, nrk_scal=nrk)
+    kept = np.arange(g.mwa) % 3 == 1 if border else np.arange(g.mwa) == 0
+    out = []
+    for coherence in (abi.SYNC_EACH_CALL, abi.RESIDENT):
+        fg = abi.FortranGrid(g)
+        table = np.ascontiguousarray(np.flatnonzero(~kept)[1 if border else 0:] + 1, dtype=np.int32)
+        fg.struct.nw_prog, fg.struct.jtw_prog = table.size, abi.ptr(table, ctypes.c_int)
+        dev = OlamGpu(fg, opts, HostState(vmasc=st.vmasc, wmasc=st.wmasc, rho=st.rho, wc=st.wc))
+        try:
+            dev.set_coherence(coherence)
+            var_p = [t.copy() for t in st.tracers]
+            dev.register_scalars(var_p, [np.zeros_like(t) for t in var_p])
+            for _ in range(1 if border else 3):
+                dev.scalar_transport_rk(st.rho_old)
+            if coherence == abi.RESIDENT:
+                dev.sync_to_host(abi.F_SCALARS)
+            out.append(var_p)
+        finally:
+            dev.close()
+    for n in range(ntr):
+        if not border:
+            assert relerr(out[0][n][1:], out[1][n][1:]) < 1e-6, n
+        for o in out:
+            assert np.array_equal(o[n][kept], st.tracers[n][kept]), n
 
 
 # above 64 tracers on grids where the timed shapes are close, so that any of
