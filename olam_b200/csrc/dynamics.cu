@@ -42,6 +42,9 @@ namespace olamgpu {
 struct DynK {
   int mza, mwa, mva, mma;
   const int* __restrict__ npoly;
+  // read by no kernel here: without these three the compiler spills 28 bytes
+  // of the column kernel's registers instead of 4 (373 us a stage against 326
+  // at NXP=100, 60 levels)
   const int* __restrict__ w_nb;
   const int* __restrict__ w_ev;
   const float* __restrict__ w_dirv;
@@ -150,14 +153,10 @@ __global__ void k_div_fdivh(DynK g, const int* __restrict__ vprog, int nv, const
 
 // ---- vort_damp ----------------------------------------------------------------
 __global__ void k_vort_first_m(DynK g, const int* __restrict__ mprog, int nm, const float* __restrict__ dnv,
-                               const float* __restrict__ arm0, float* __restrict__ vfact,
-                               int* __restrict__ lpmmin) {
+                               const float* __restrict__ arm0, float* __restrict__ vfact) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nm) return;
   const int im = mprog[j];
-  int lm = 1 << 30;
-  for (int jv = 0; jv < 3; ++jv) lm = min(lm, LPV(g.m_iv[im * 3 + jv]));
-  lpmmin[im] = lm;
   for (int jv = 0; jv < 3; ++jv) {
     const int iv = g.m_iv[im * 3 + jv];
     const float v = dnv[iv] / arm0[im];
@@ -623,7 +622,7 @@ struct WrtArgs {
 };
 
 // warps per SM the column kernel is compiled for: 72 registers (at NXP=100, 60
-// levels 320 us; 24 warps and 80 registers 363, 32 warps and 64 registers 349)
+// levels 326 us; 24 warps and 80 registers 363, 32 warps and 64 registers 349)
 #define WRT_OCC 28
 // columns per block: four one-warp columns, else one
 #define WRT_COLS(NW) ((NW) == 1 ? 4 : 1)
@@ -693,7 +692,7 @@ __device__ __forceinline__ void column_solve(double* P, int n, int i, double ra,
 }
 
 // n up to 128 (four warps a column): parallel cyclic reduction of all rows,
-// each publishing a, c, d and 1 / b per step.  P: four arrays of mza doubles.
+// each publishing a, c, d and 1 / b per step.  P: four arrays of 128 doubles.
 template <>
 __device__ __forceinline__ void column_solve<4>(double* P, int n, int i, double ra, double rb, double rc, double rd,
                                                 float* x) {
@@ -1249,7 +1248,7 @@ static int ensure_dyn_buffers(Context& C) {
   OG_CHECK(A(y.div2d, 2 * wz));
   OG_CHECK(A(y.vort2d, 2 * mz));
   OG_CHECK(A(y.fvorth, C.g.mva)); OG_CHECK(A(y.fvortl, C.g.mva));
-  OG_CHECK(A(y.vfact, 3 * (size_t)C.g.mma)); OG_CHECK(A(y.lpmmin, C.g.mma));
+  OG_CHECK(A(y.vfact, 3 * (size_t)C.g.mma));
   return OLAMGPU_OK;
 }
 
@@ -1372,8 +1371,7 @@ static int v_tendency(Context& C, bool div, bool vor, bool setup, const float* s
   }
   if (vor && y.vort_first) {
     y.vort_first = false;
-    k_vort_first_m<<<cdiv(d.nm_prog, 128), 128, 0, s>>>(g, d.jtm_prog.p, d.nm_prog, y.dnv.p, y.arm0.p, y.vfact.p,
-                                                        y.lpmmin.p);
+    k_vort_first_m<<<cdiv(d.nm_prog, 128), 128, 0, s>>>(g, d.jtm_prog.p, d.nm_prog, y.dnv.p, y.arm0.p, y.vfact.p);
     k_vort_first_v<<<cdiv(d.nv_prog, 128), 128, 0, s>>>(g, d.jtv_prog.p, d.nv_prog, y.dniu.p, y.arm0.p, (float)dtm,
                                                         o.vort_damp_fact, o.vort_damp_level, y.fvorth.p, y.fvortl.p);
     OG_LAUNCHED(); OG_LAUNCHED();
@@ -1504,7 +1502,6 @@ int dyn_prog_wrtv_rk(int istp) {
   const int nrk = o.nrk_wrtv;
   const double third = 1.0 / 3.0;
   const double xstg3[3] = {third, 0.5, 1.0}, xstg2[2] = {0.5, 1.0};
-  const size_t wz = (size_t)mza * d.mwa;
   for (int istage = 1; istage <= nrk; ++istage) {
     const double dt8 = (nrk <= 2 ? xstg2[istage - 1] : xstg3[istage - 1]) * o.dtsm;
     const float dts = (float)dt8;
@@ -1630,7 +1627,6 @@ int dyn_prog_wrtv_rk(int istp) {
       OG_CHECK(halo_exchange_fields(C, HALO_W, f6, 6, s));
     }
   }
-  (void)wz;
   if (C.coherence == OLAMGPU_SYNC_EACH_CALL) {
     OG_CHECK(dyn_state_to_host(DYN_OUT_MASK, s));
     OG_CUDA(cudaStreamSynchronize(s));
@@ -1729,7 +1725,6 @@ void dyn_release() {
                         &y.th0, &y.vx0, &y.vy0, &y.vz0, &y.m_scpt, &y.m_gx, &y.m_hiw, &y.m_sfw, &y.m_hiv,
                         &y.m_sfv, &y.m_sin, &y.m_sout};
   for (auto* b : f) b->release();
-  y.lpmmin.release();
   y.lve2.release();
   y.vm0.release();
   dyn_eddy_release();

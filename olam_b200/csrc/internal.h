@@ -365,7 +365,6 @@ struct Dyn {
   // word per V point and level); upw field by field
   DevBuf<float> upw, upv;
   DevBuf<float> div2d, fdivh, vort2d, fvorth, fvortl, vfact;
-  DevBuf<int> lpmmin;
   bool lpm_flat = true;          // lpm = 2 at every M point
   // prognostic shaved-cell method: lve2 of every W column and the start
   // momentum of its lve2 lowest levels, (mwa, nve2_max, 3); none on grids

@@ -245,35 +245,35 @@ __global__ void k_implicit_solve(GridK g, const int* list, const int* count,
   const size_t all = (size_t)*count * nt;
   const int mza = g.mza;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < all; i += (size_t)gridDim.x * blockDim.x) {
-  const int slot = (int)(i / nt), t = (int)(i % nt);
-  const int iw = list[slot];
-  const int kb = g.lpw[iw];
-  const float* b1 = b + (size_t)slot * 3 * mza;
-  const float* scr1 = b1 + mza;
-  const float* cji = b1 + 2 * mza;
-  const float* wm = wmasc + (size_t)iw * mza;
-  float ffv = ff[(size_t)iw * nrk + istage - 1];
-  auto S0 = [&](int kd) { return scp0.base[((size_t)iw * mza + kd) * scp0.ld + scp0.t0 + t]; };
-  float* sp = scp.base + (size_t)iw * mza * scp.ld + scp.t0 + t;
-  // forward elimination into soln (kept in the output column), then back
-  // substitution; delex is formed on the fly from scp and scp0
-  float prev = 0.f;
-  for (int kd = kb; kd < mza; ++kd) {
-    float s0 = S0(kd);
-    float dk = (kd <= mza - 2) ? S0(kd + 1) - s0 : 0.f;
-    float dkm1 = (kd - 1 >= kb) ? s0 - S0(kd - 1) : 0.f;
-    float c1 = ffv * dtr * g.volti[(size_t)iw * mza + kd] / rhos_st[(size_t)iw * mza + kd];
-    float delex = sp[(size_t)kd * scp.ld] - s0 - c1 * (fminf(wm[kd], 0.f) * dk + fmaxf(wm[kd - 1], 0.f) * dkm1);
-    float sol = (kd == kb) ? delex * cji[kd] : cji[kd] * (delex - b1[kd] * prev);
-    sp[(size_t)kd * scp.ld] = sol;
-    prev = sol;
-  }
-  for (int kd = mza - 2; kd >= kb; --kd) {
-    float v = sp[(size_t)kd * scp.ld] - scr1[kd + 1] * sp[(size_t)(kd + 1) * scp.ld];
-    sp[(size_t)kd * scp.ld] = v;
-  }
-  for (int kd = kb; kd < mza; ++kd) sp[(size_t)kd * scp.ld] = S0(kd) + sp[(size_t)kd * scp.ld];
-  for (int kd = 1; kd < kb; ++kd) sp[(size_t)kd * scp.ld] = sp[(size_t)kb * scp.ld];
+    const int slot = (int)(i / nt), t = (int)(i % nt);
+    const int iw = list[slot];
+    const int kb = g.lpw[iw];
+    const float* b1 = b + (size_t)slot * 3 * mza;
+    const float* scr1 = b1 + mza;
+    const float* cji = b1 + 2 * mza;
+    const float* wm = wmasc + (size_t)iw * mza;
+    float ffv = ff[(size_t)iw * nrk + istage - 1];
+    auto S0 = [&](int kd) { return scp0.base[((size_t)iw * mza + kd) * scp0.ld + scp0.t0 + t]; };
+    float* sp = scp.base + (size_t)iw * mza * scp.ld + scp.t0 + t;
+    // forward elimination into soln (kept in the output column), then back
+    // substitution; delex is formed on the fly from scp and scp0
+    float prev = 0.f;
+    for (int kd = kb; kd < mza; ++kd) {
+      float s0 = S0(kd);
+      float dk = (kd <= mza - 2) ? S0(kd + 1) - s0 : 0.f;
+      float dkm1 = (kd - 1 >= kb) ? s0 - S0(kd - 1) : 0.f;
+      float c1 = ffv * dtr * g.volti[(size_t)iw * mza + kd] / rhos_st[(size_t)iw * mza + kd];
+      float delex = sp[(size_t)kd * scp.ld] - s0 - c1 * (fminf(wm[kd], 0.f) * dk + fmaxf(wm[kd - 1], 0.f) * dkm1);
+      float sol = (kd == kb) ? delex * cji[kd] : cji[kd] * (delex - b1[kd] * prev);
+      sp[(size_t)kd * scp.ld] = sol;
+      prev = sol;
+    }
+    for (int kd = mza - 2; kd >= kb; --kd) {
+      float v = sp[(size_t)kd * scp.ld] - scr1[kd + 1] * sp[(size_t)(kd + 1) * scp.ld];
+      sp[(size_t)kd * scp.ld] = v;
+    }
+    for (int kd = kb; kd < mza; ++kd) sp[(size_t)kd * scp.ld] = S0(kd) + sp[(size_t)kd * scp.ld];
+    for (int kd = 1; kd < kb; ++kd) sp[(size_t)kd * scp.ld] = sp[(size_t)kb * scp.ld];
   }
 }
 
