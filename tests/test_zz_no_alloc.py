@@ -232,3 +232,44 @@ def test_noalloc_nan_and_infinity_reach_their_stencil_only(order, terrain):
         hit[w, :g.lpw[w] - 1] = hit[w, g.lpw[w] - 1]
     assert np.array_equal(~np.isfinite(out[1:]), hit[1:])
     assert np.array_equal(out[1:][~hit[1:]], ref[1:][~hit[1:]])
+
+
+def test_noalloc_recorded_by_the_caller():
+    """Two stages and a caller's own operation between them recorded into a
+    CUDA graph, the second stage in place; the replay on new inputs equals
+    the calls made one by one."""
+    import torch
+    g, st = small_case(nxp=6, nlev=40, ntr=2, seed=31)
+    dev = OlamGpu(abi.FortranGrid(g), abi.make_opts(1800.0),
+                  HostState(vmasc=st.vmasc, wmasc=st.wmasc, rho=st.rho, wc=st.wc))
+    try:
+        def dv(a):
+            return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()
+        scp, sct, rhos, vm, wm = dv(st.tracers[0]), dv(st.sct[0]), dv(st.rho), dv(st.vmasc), dv(st.wmasc)
+        mid = torch.zeros_like(scp)
+
+        def stage(src, dst):
+            p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+            check(dev.lib.olamgpu_update_scalar_noalloc(p(src), p(scp), p(sct), p(rhos), p(vm), p(wm), C.c_float(900.0),
+                                                        p(dst), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+
+        def both():
+            stage(scp, mid)
+            mid.mul_(1.001)
+            stage(mid, mid)
+
+        both()                                         # first call: set-up
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            both()
+        for n in (1, 0):
+            scp.copy_(dv(st.tracers[n]))
+            both()
+            ref = mid.clone()
+            mid.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(mid[1:], ref[1:])
+    finally:
+        dev.close()
